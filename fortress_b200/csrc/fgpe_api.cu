@@ -22,6 +22,7 @@
 #include "fgpe_fast.cuh"
 #include "fgpe_group.cuh"
 #include "fgpe_persist.h"
+#include "fgpe_step.h"
 #include "fno_kernels.cuh"
 #include "fno_gemm_tc.cuh"
 #include "../../include/fno.h"
@@ -74,14 +75,12 @@ struct fgpe_s {
     bool bulk_off = false;
     bool fast_row = false, fast_col[3] = {false, false, false};
     bool has_fast_row = false, has_fast_col[3] = {false, false, false};
-    int fast_row_grid = 0, fast_col_grid[3] = {0, 0, 0};
-    bool col_wide[3] = {false, false, false};   // column pass uses the wide tiles
-    // column passes that transform forward and back in one launch (q2D y,
-    // 3D z) on the radix-16 plan (cplan pv 3) with its own position map
-    bool col_r16[3] = {false, false, false};
-    int col_r16_grid[3] = {0, 0, 0};
-    int* pmap16 = nullptr;
-    const int* fline16[3] = {nullptr, nullptr, nullptr};
+    int fast_row_grid = 0;
+    // column passes with register-resident transforms, by kind (fgpe_step.h);
+    // 3D y passes leave their spectra in the order of ymap (position ->
+    // frequency), which the z pass of the step reads
+    int reg_grid[4] = {0, 0, 0, 0}, reg_wide[4] = {0, 0, 0, 0};
+    int* ymap = nullptr;
     // row pass with one warp per x row (k_row_warp), where a row fits 16 KB
     bool has_warp_row = false, warp_row = false;
     int warp_row_grid = 0;
@@ -201,29 +200,9 @@ template <typename T, int MS, int N> constexpr int row_th() {
 template <typename T, int MS, int N> constexpr int col_th() {
     return FGPE_COL_TH ? FGPE_COL_TH : fast_threads(MS * col_tx<T>() * N / 8);
 }
-// Wide column tiles: FGPE_COL_WIDE_BYTES (default 128) contiguous bytes of x
-// per line element (8 complex doubles, 16 complex floats), for grids with
-// enough tiles (3D) where the 32-byte segments of the narrow tiles waste DRAM
-// bursts; FGPE_COL_NBUF_W shared buffers per block (default FGPE_COL_NBUF).
-#ifndef FGPE_COL_WIDE_BYTES
-#define FGPE_COL_WIDE_BYTES 128
-#endif
-#ifndef FGPE_COL_NBUF_W
-#define FGPE_COL_NBUF_W FGPE_COL_NBUF
-#endif
-template <typename T> constexpr int col_txw() { return FGPE_COL_WIDE_BYTES / (int)sizeof(cx<T>); }
-template <typename T, int MS, int N> constexpr size_t col_smem_w() {
-    return (size_t)FGPE_COL_NBUF_W * MS * cpad(N) * col_txw<T>() * sizeof(cx<T>);
-}
-template <typename T, int MS, int N> constexpr bool wide_ok() { return col_smem_w<T, MS, N>() <= 113 * 1024; }
-template <typename T, int MS, int N> constexpr int col_th_w() { return fast_threads(MS * col_txw<T>() * N / 8); }
 template <typename T, int MS, int N> constexpr size_t row_smem() {
     return ((size_t)FGPE_ROW_NBUF * MS * row_r(N) * cpad(N) + (FGPE_TW_SMEM ? N : 0)) * sizeof(cx<T>);
 }
-template <typename T, int MS, int N> constexpr size_t col_smem() {
-    return ((size_t)FGPE_COL_NBUF * MS * cpad(N) * col_tx<T>() + (FGPE_TW_SMEM ? N : 0)) * sizeof(cx<T>);
-}
-
 template <class K> int grid_for(K kern, int th, size_t smem, int ntiles) {
     int dev = 0, nsm = 0, per = 0;
     cudaGetDevice(&dev);
@@ -238,45 +217,6 @@ template <typename T, int MS, int N> int setup_fast_row(fgpe_t* h) {
     if (rows % row_r(N)) return 0;
     return grid_for(k_row_fast<T, MS, N, row_r(N), row_th<T, MS, N>()>, row_th<T, MS, N>(), row_smem<T, MS, N>(),
                     rows / row_r(N));
-}
-// Grid of the column kernel for one axis (0: none); *wide tells whether the
-// wide tiles were chosen: they need 128-byte rows of x and at least four
-// waves of tiles, so that their fewer, larger tiles still fill the GPU.
-template <typename T, int MS, int N> int setup_fast_col(fgpe_t* h, int n_other, bool* wide) {
-    *wide = false;
-    if constexpr (wide_ok<T, MS, N>()) {
-        if (h->p.nx % col_txw<T>() == 0) {
-            const int ntw = (h->p.nx / col_txw<T>()) * n_other;
-            const int g = grid_for(k_col_fast<T, MS, N, col_txw<T>(), col_th_w<T, MS, N>(), FGPE_COL_NBUF_W>, col_th_w<T, MS, N>(),
-                                   col_smem_w<T, MS, N>(), ntw);
-            if (g > 0 && ntw >= 4 * g) { *wide = true; return g; }
-        }
-    }
-    if (h->p.nx % col_tx<T>()) return 0;
-    return grid_for(k_col_fast<T, MS, N, col_tx<T>(), col_th<T, MS, N>()>, col_th<T, MS, N>(), col_smem<T, MS, N>(),
-                    (h->p.nx / col_tx<T>()) * n_other);
-}
-// Radix-16 plan for the column passes that transform forward and back in one
-// launch, on lengths where it saves a radix pass (128, 256, 384); build knob
-// FGPE_COL_R16 (0: every column pass on the handle's plan).
-#ifndef FGPE_COL_R16
-#define FGPE_COL_R16 1
-#endif
-constexpr bool r16_len(int n) { return FGPE_COL_R16 && cplan(n, 3).r[0] == 16; }
-// Grid of the radix-16 form of the column kernel with the same tiles as
-// setup_fast_col chose (0: not available).
-template <typename T, int MS, int N> int setup_fast_col_r16(fgpe_t* h, int n_other, bool wide) {
-    if constexpr (r16_len(N)) {
-        if constexpr (wide_ok<T, MS, N>()) {
-            if (wide)
-                return grid_for(k_col_fast<T, MS, N, col_txw<T>(), col_th_w<T, MS, N>(), FGPE_COL_NBUF_W, 3>,
-                                col_th_w<T, MS, N>(), col_smem_w<T, MS, N>(), (h->p.nx / col_txw<T>()) * n_other);
-        }
-        if (!wide)
-            return grid_for(k_col_fast<T, MS, N, col_tx<T>(), col_th<T, MS, N>(), FGPE_COL_NBUF, 3>, col_th<T, MS, N>(),
-                            col_smem<T, MS, N>(), (h->p.nx / col_tx<T>()) * n_other);
-    }
-    return 0;
 }
 // Warp-row kernel: rows of MS lines up to 16 KB (FP64 spin-1 to 256 points,
 // spin-2 to 128; FP32 spin-1 to 512, spin-2 to 256); warps per block so that
@@ -299,29 +239,15 @@ template <typename T, int MS, int N> int setup_warp_row(fgpe_t* h) {
 }
 
 // The size-specialised kernels go out as programmatic dependent launches
-// (outside stream capture): the next pass is launched while the previous one
-// drains and waits on griddepcontrol.wait before it touches the state.  Their
-// grids are one wave of resident blocks, so a waiting block never keeps the
-// previous pass from finishing.
-template <class K, class A>
-void launch_pdl(fgpe_t* h, K kern, int grid, int threads, size_t smem, const A& a) {
+// (launch_step_kernel), outside stream capture.
+bool use_pdl(fgpe_t* h) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cudaStreamIsCapturing(h->st, &cs);
-    if (cs != cudaStreamCaptureStatusNone) {
-        kern<<<grid, threads, smem, h->st>>>(h->sc, a);
-        return;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = h->st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, h->sc, a);
+    return cs == cudaStreamCaptureStatusNone;
+}
+template <class K, class A>
+void launch_pdl(fgpe_t* h, K kern, int grid, int threads, size_t smem, const A& a) {
+    launch_step_kernel(kern, grid, threads, smem, h->sc, a, h->st, use_pdl(h));
 }
 template <typename T, int MS, int N> void run_fast_row(fgpe_t* h, const RowArgs& a) {
     launch_pdl(h, k_row_fast<T, MS, N, row_r(N), row_th<T, MS, N>()>, h->fast_row_grid, row_th<T, MS, N>(),
@@ -334,34 +260,6 @@ template <typename T, int MS, int N> void run_warp_row(fgpe_t* h, const RowArgs&
                    (size_t)W * FGPE_WROW_NBUF * wrow_tile<T, MS, N>(), a);
     }
 }
-template <typename T, int MS, int N> void run_fast_col(fgpe_t* h, int axis, const ColArgs& a0, bool r16) {
-    ColArgs a = a0;
-    if constexpr (r16_len(N)) {
-        if (r16) {
-            a.fline = h->fline16[axis];
-            if constexpr (wide_ok<T, MS, N>()) {
-                if (h->col_wide[axis]) {
-                    launch_pdl(h, k_col_fast<T, MS, N, col_txw<T>(), col_th_w<T, MS, N>(), FGPE_COL_NBUF_W, 3>,
-                               h->col_r16_grid[axis], col_th_w<T, MS, N>(), col_smem_w<T, MS, N>(), a);
-                    return;
-                }
-            }
-            launch_pdl(h, k_col_fast<T, MS, N, col_tx<T>(), col_th<T, MS, N>(), FGPE_COL_NBUF, 3>, h->col_r16_grid[axis],
-                       col_th<T, MS, N>(), col_smem<T, MS, N>(), a);
-            return;
-        }
-    }
-    if constexpr (wide_ok<T, MS, N>()) {
-        if (h->col_wide[axis]) {
-            launch_pdl(h, k_col_fast<T, MS, N, col_txw<T>(), col_th_w<T, MS, N>(), FGPE_COL_NBUF_W>, h->fast_col_grid[axis],
-                       col_th_w<T, MS, N>(), col_smem_w<T, MS, N>(), a);
-            return;
-        }
-    }
-    launch_pdl(h, k_col_fast<T, MS, N, col_tx<T>(), col_th<T, MS, N>()>, h->fast_col_grid[axis], col_th<T, MS, N>(),
-               col_smem<T, MS, N>(), a);
-}
-
 #define FAST_SWITCH(n, CALL)            \
     switch (n) {                         \
         case 128: CALL(128); break;      \
@@ -435,19 +333,14 @@ void launch_col(fgpe_t* h, int axis, int flags) {
     a.flags = flags;
     a.n_other = h->p.dim == 2 ? 1 : (axis == 1 ? h->p.nz : h->p.ny);
     a.axis = axis;
-    a.fline = axis == 1 ? h->sc.fy : h->sc.fz;
-    // radix-16 lines: a pass that transforms forward and back (q2D y, 3D z),
-    // or the y passes of a 3D step when all its column passes run the
-    // size-specialised kernels (the y spectra then use that plan throughout
-    // the step: the z pass reads ky through fother)
-    const bool y16 = h->p.dim == 3 && (flags & COL_STEP) && h->col_r16[1] && h->fast_col[1] && h->fast_col[2];
-    a.fother = y16 ? h->fline16[1] : h->sc.fy;
-    const bool r16 = h->col_r16[axis] && ((axis == 1 && y16) || ((flags & COL_FWD) && (flags & COL_INV)));
+    // the y spectra of a 3D step live only between its two y passes, so those
+    // may take a radix plan of their own; the z pass reads ky through fother
+    const bool step = (flags & COL_STEP) != 0;
+    a.fother = step && h->p.dim == 3 && h->fast_col[1] ? h->ymap : h->sc.fy;
     ProfScope ps(h, axis);
-    if (h->fast_col[axis]) {
-#define RUNC(NN) run_fast_col<T, MS, NN>(h, axis, a, r16)
-        FAST_SWITCH(a.n, RUNC)
-#undef RUNC
+    if (step && h->fast_col[axis]) {
+        const int kind = h->p.dim == 2 ? 2 : axis == 2 ? 3 : (flags & COL_FWD) ? 0 : 1;
+        regcol_launch<T, MS>(a.n, kind, h->reg_wide[kind], h->reg_grid[kind], h->sc, a, h->st, use_pdl(h));
         h->launches++;
         return;
     }
@@ -820,7 +713,11 @@ int fgpe_create(const fgpe_params* pin, fgpe_t** out) {
         c.fx = h->pmap + offp[0]; c.fy = h->pmap + offp[1]; c.fz = h->pmap + offp[2];
     }
     const size_t bytes = (size_t)h->npts * h->ms * h->cs;
-    CK(cudaMalloc(&h->S, bytes));
+    // the SO-coupling table (fgpe_device.cuh, Soc4) follows S in its allocation
+    const bool soc_on = p.dim >= 2 && (c.gx != 0.0 || c.gy != 0.0);
+    const size_t nxy = (size_t)p.nx * p.ny, soc_at = (bytes + 255) / 256 * 256;
+    CK(cudaMalloc(&h->S, soc_at + (soc_on ? nxy * 2 * h->cs : 0)));
+    if (soc_on) c.soc = (char*)h->S + soc_at;
     CK(cudaMalloc(&h->psi, bytes));
     CK(cudaMalloc(&h->prev, bytes));
     CK(cudaMalloc(&h->dtab, dt_all.size() * sizeof(double)));
@@ -841,6 +738,12 @@ int fgpe_create(const fgpe_params* pin, fgpe_t** out) {
     c.twx = (char*)h->ctab + off_tw[0] * ces; c.twy = (char*)h->ctab + off_tw[1] * ces; c.twz = (char*)h->ctab + off_tw[2] * ces;
     c.kex = (char*)h->ctab + off_ke[0] * ces; c.key = (char*)h->ctab + off_ke[1] * ces; c.kez = (char*)h->ctab + off_ke[2] * ces;
     c.pvx = (char*)h->ctab + off_pv[0] * ces; c.pvy = (char*)h->ctab + off_pv[1] * ces; c.pvz = (char*)h->ctab + off_pv[2] * ces;
+    if (c.soc) {
+        const unsigned grid = (unsigned)std::min<size_t>((nxy + 255) / 256, 148 * 8);
+        if (h->fp32) k_soc_table<float><<<grid, 256, 0, h->st>>>(c, (Soc4<float>*)c.soc);
+        else k_soc_table<double><<<grid, 256, 0, h->st>>>(c, (Soc4<double>*)c.soc);
+        CK(cudaGetLastError());
+    }
     if (h->split1d) {
         h->twn = c.twx;   // W_N^j of the whole line
         h->tw1 = (char*)h->ctab + off_tw1 * ces;
@@ -940,36 +843,28 @@ int fgpe_create(const fgpe_params* pin, fgpe_t** out) {
     }
     for (int a = 1; a < p.dim; ++a) {
         if (!allow_fast_col || !fast_size(ns[a])) continue;
-        const int nob = p.dim == 2 ? 1 : (a == 1 ? p.nz : p.ny);
-        int g = 0;
-        bool wide = false;
-#define SETC(NN) g = h->fp32 ? (ms == 3 ? setup_fast_col<float, 3, NN>(h, nob, &wide) : setup_fast_col<float, 5, NN>(h, nob, &wide)) \
-                             : (ms == 3 ? setup_fast_col<double, 3, NN>(h, nob, &wide) : setup_fast_col<double, 5, NN>(h, nob, &wide))
-        FAST_SWITCH(ns[a], SETC)
-#undef SETC
-        if (g > 0) { h->fast_col[a] = h->has_fast_col[a] = true; h->fast_col_grid[a] = g; h->col_wide[a] = wide; }
-        // the pass that carries KE and SOC (q2D y, 3D z) transforms forward
-        // and back in one launch, and the 3D y spectra live only between the
-        // step's two y passes: these lines may take the radix-16 plan
-        const bool fused = (p.dim == 2 && a == 1) || p.dim == 3;
-        if (g > 0 && fused && r16_len(ns[a])) {
-            int g16 = 0;
-#define SETC16(NN) g16 = h->fp32 ? (ms == 3 ? setup_fast_col_r16<float, 3, NN>(h, nob, wide) : setup_fast_col_r16<float, 5, NN>(h, nob, wide)) \
-                                 : (ms == 3 ? setup_fast_col_r16<double, 3, NN>(h, nob, wide) : setup_fast_col_r16<double, 5, NN>(h, nob, wide))
-            FAST_SWITCH(ns[a], SETC16)
-#undef SETC16
-            if (g16 > 0) {
-                const CPlan cp = cplan(ns[a], 3);
-                FftPlan pl;
-                pl.n = ns[a]; pl.nf = cp.nf;
-                for (int f = 0; f < cp.nf; ++f) pl.r[f] = cp.r[f];
-                const std::vector<int> f = position_map(pl);
-                if (!h->pmap16) CK(cudaMalloc(&h->pmap16, 2 * 512 * sizeof(int)));
-                CK(cudaMemcpy(h->pmap16 + (a - 1) * 512, f.data(), f.size() * sizeof(int), cudaMemcpyHostToDevice));
-                h->fline16[a] = h->pmap16 + (a - 1) * 512;
-                h->col_r16[a] = true;
-                h->col_r16_grid[a] = g16;
-            }
+        const int other = p.dim == 2 ? 1 : (a == 1 ? p.nz : p.ny);
+        bool ok = true;
+        auto setup = [&](int kind) {
+            int& g = h->reg_grid[kind];
+            int& w = h->reg_wide[kind];
+            g = h->fp32 ? (ms == 3 ? regcol_grid<float, 3>(ns[a], kind, p.nx, other, &w)
+                                   : regcol_grid<float, 5>(ns[a], kind, p.nx, other, &w))
+                        : (ms == 3 ? regcol_grid<double, 3>(ns[a], kind, p.nx, other, &w)
+                                   : regcol_grid<double, 5>(ns[a], kind, p.nx, other, &w));
+            ok = ok && g > 0;
+        };
+        if (p.dim == 2) setup(2);
+        else if (a == 2) setup(3);
+        else { setup(0); setup(1); }
+        h->fast_col[a] = h->has_fast_col[a] = ok;
+        if (ok && p.dim == 3 && a == 1) {
+            FftPlan pl;
+            pl.n = p.ny;
+            pl.nf = regcol_radices(p.ny, pl.r);
+            const std::vector<int> f = position_map(pl);
+            CK(cudaMalloc(&h->ymap, f.size() * sizeof(int)));
+            CK(cudaMemcpy(h->ymap, f.data(), f.size() * sizeof(int), cudaMemcpyHostToDevice));
         }
     }
     cudaGetLastError();   // clear any attribute/occupancy probe error
@@ -1020,7 +915,7 @@ int fgpe_destroy(fgpe_t* h) {
     if (h->bulk) cudaGraphExecDestroy(h->bulk);
     cudaFree(h->S); cudaFree(h->psi); cudaFree(h->prev); cudaFree(h->stage);
     cudaFree(h->dtab); cudaFree(h->ctab); cudaFree(h->part); cudaFree(h->info);
-    cudaFree(h->counters); cudaFree(h->pmap); cudaFree(h->pmap16);
+    cudaFree(h->counters); cudaFree(h->pmap); cudaFree(h->ymap);
     if (h->h_small) cudaFreeHost(h->h_small);
     for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
     if (h->own_stream && h->st) cudaStreamDestroy(h->st);

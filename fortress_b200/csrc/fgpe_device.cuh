@@ -35,6 +35,14 @@ template <typename C> __host__ __device__ __forceinline__ C cmacc(C acc, C a, C 
 }
 template <typename C> __host__ __device__ __forceinline__ C cconj(C a) { a.y = -a.y; return a; }
 template <typename C, typename S> __host__ __device__ __forceinline__ C cscale(C a, S s) { a.x *= s; a.y *= s; return a; }
+// Single precision: both parts in one packed instruction, with the rounding
+// of the two scalar ones.  The FP32 passes are short of issue slots, and most
+// of a butterfly is complex sums.
+#if defined(__CUDA_ARCH__)
+__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 csub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.f, -1.f), a); }
+__device__ __forceinline__ float2 cscale(float2 a, float s) { return __fmul2_rn(a, make_float2(s, s)); }
+#endif
 // multiply by i (sign = +1) or -i (sign = -1)
 template <typename C> __host__ __device__ __forceinline__ C cmuli(C a, int sign) {
     C r; if (sign > 0) { r.x = -a.y; r.y = a.x; } else { r.x = a.y; r.y = -a.x; } return r;
@@ -316,6 +324,7 @@ struct StepConst {
     double* sink;                   // per-step NORMC ring (pinned host or device), or null
     unsigned* sink_ctr;             // steps appended since the ring was set
     int sink_n;                     // records of MS doubles in the ring
+    const void* soc;                // 2D/3D: Soc4<T> per (ky index, x position), or null without SO coupling
 };
 
 // Append one step's NORMC to the sink ring (called by one thread).
@@ -453,6 +462,67 @@ __device__ __forceinline__ void apply_soc(const StepConst& c, double kx, double 
         const int cc = S - r;
         cx<T> ph = cc == 0 ? mk<T>(1, 0) : cc == 1 ? e1 : cc == -1 ? cconj(e1) : cc == 2 ? e2 : cconj(e2);
         v[r] = cmulc(s, ph);
+    }
+}
+
+// The (kx, ky)-dependent numbers of the SO-coupling exponential: cos beta and
+// sin beta, and the phases exp(-+ i CDT alpha) of L = +1, -1 (real time: p, q
+// are the parts of the first, the second is its conjugate; imaginary time:
+// both are real).  They depend on the handle's parameters only, so 2D and 3D
+// handles tabulate them once per (kx, ky) (k_soc_table) in place of a
+// reciprocal square root, two series and, for large angles, exp or sincos at
+// every point of every step.
+template <typename T> struct __align__(4 * sizeof(T)) Soc4 { T cb, sb, p, q; };
+
+// v <- exp(-i CDT H_SO(k)) v from tabulated numbers; the arithmetic of apply_soc.
+template <typename T, int MS>
+__device__ __forceinline__ void soc_apply(int imag, Soc4<T> e, cx<T>* v) {
+    constexpr int S = MS / 2;
+    const cx<T> e1 = mk<T>(e.cb, e.sb);
+    const cx<T> l1 = mk<T>(e.p, imag ? (T)0 : e.q), lm1 = imag ? mk<T>(e.q, (T)0) : cconj(l1);
+    if constexpr (MS == 3) {
+        // A0 D A0 with A0 = [[1/2, -h, 1/2], [-h, 0, h], [1/2, h, 1/2]], h^2 = 1/2,
+        // between the phases e^{+-i beta} of the outer components
+        const T h = (T)0.70710678118654752440, f = (T)0.5;
+        const cx<T> w0 = cmul(v[0], e1), w2 = cmulc(v[2], e1);
+        const cx<T> s = mk<T>(f * (w0.x + w2.x), f * (w0.y + w2.y));
+        const cx<T> d = mk<T>(f * (w2.x - w0.x), f * (w2.y - w0.y));
+        const cx<T> a = fmul(imag, lm1, mk<T>(fma(-h, v[1].x, s.x), fma(-h, v[1].y, s.y)));
+        const cx<T> b = fmul(imag, l1, mk<T>(fma(h, v[1].x, s.x), fma(h, v[1].y, s.y)));
+        const cx<T> g = mk<T>(a.x + b.x, a.y + b.y);
+        v[0] = cmulc(mk<T>(fma(f, g.x, -d.x), fma(f, g.y, -d.y)), e1);
+        v[1] = mk<T>(h * (b.x - a.x), h * (b.y - a.y));
+        v[2] = cmul(mk<T>(fma(f, g.x, d.x), fma(f, g.y, d.y)), e1);
+        return;
+    }
+    const cx<T> e2 = cmul(e1, e1);
+    auto ph = [&](int cc) { return cc == 1 ? e1 : cc == -1 ? cconj(e1) : cc == 2 ? e2 : cconj(e2); };
+    cx<T> w[MS], u[MS];
+#pragma unroll
+    for (int m = 0; m < MS; ++m) w[m] = m == S ? v[m] : cmul(v[m], ph(S - m));
+#pragma unroll
+    for (int r = 0; r < MS; ++r) {
+        u[r] = mk<T>(0, 0);
+#pragma unroll
+        for (int q = 0; q < MS; ++q) {
+            const T a = (T)A0<MS>::at(q, r);
+            if (a != (T)0) { u[r].x += a * w[q].x; u[r].y += a * w[q].y; }
+        }
+        const int L = r - S;
+        if (L == 1) u[r] = fmul(imag, l1, u[r]);
+        else if (L == -1) u[r] = fmul(imag, lm1, u[r]);
+        else if (L == 2) u[r] = fmul(imag, fmul(imag, l1, l1), u[r]);
+        else if (L == -2) u[r] = fmul(imag, fmul(imag, lm1, lm1), u[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < MS; ++r) {
+        cx<T> s = mk<T>(0, 0);
+#pragma unroll
+        for (int q = 0; q < MS; ++q) {
+            const T a = (T)A0<MS>::at(r, q);
+            if (a != (T)0) { s.x += a * u[q].x; s.y += a * u[q].y; }
+        }
+        v[r] = r == S ? s : cmulc(s, ph(S - r));
     }
 }
 

@@ -10,6 +10,7 @@
 // HBM traffic overlaps the FP64/FP32 work.
 #pragma once
 #include "fgpe_device.cuh"
+#include "fgpe_async.cuh"
 #include "fgpe_kernels.h"
 
 namespace fgpe {
@@ -25,9 +26,7 @@ struct CPlan {
 // longest stride).  Only transforms whose spectra stay inside one kernel
 // (the y lines of the persistent batch kernel) use pv != 0.
 // pv = 3: a radix-16 pass first where it saves a pass: 2^7 -> 16*8,
-// 2^8 -> 16*16 (128, 256, 384 = 16*8*3); other lengths as plan 0.  Used by
-// the column passes that transform forward and back in one launch (the q2D
-// y pass, the 3D z pass), whose spectra never leave the kernel.
+// 2^8 -> 16*16 (128, 256, 384 = 16*8*3); other lengths as plan 0.
 constexpr CPlan cplan(int n, int pv = 0) {
     CPlan p{0, {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0}};
     if (pv == 3) {
@@ -154,44 +153,6 @@ __device__ __forceinline__ void ct_fft(cx<T>* s, const cx<T>* __restrict__ tw) {
     }
 }
 
-// ------------------------------------------------------------- cp.async
-#ifdef FGPE_CHECK_ALIGN
-// Diagnostic build only: record the first misaligned copy and skip it.
-static __device__ unsigned long long g_align_fault[4];
-__device__ __forceinline__ bool align_bad(const void* s, const void* g, unsigned bytes, int site) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(s);
-    if ((d % bytes) == 0 && ((unsigned long long)g % bytes) == 0) return false;
-    if (atomicCAS(&g_align_fault[0], 0ull, 1ull) == 0ull) {
-        g_align_fault[1] = (unsigned long long)site;
-        g_align_fault[2] = d;
-        g_align_fault[3] = (unsigned long long)g;
-    }
-    return true;
-}
-#define FGPE_ALIGN_GUARD(s, g, b, site) if (align_bad(s, g, b, site)) return
-#else
-#define FGPE_ALIGN_GUARD(s, g, b, site)
-#endif
-
-__device__ __forceinline__ void cp16(void* smem_dst, const void* gsrc) {
-    FGPE_ALIGN_GUARD(smem_dst, gsrc, 16, 16);
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp8(void* smem_dst, const void* gsrc) {
-    FGPE_ALIGN_GUARD(smem_dst, gsrc, 8, 8);
-    const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(gsrc) : "memory");
-}
-// One complex element: 16-byte copy for complex128, 8-byte for complex64 (the
-// padded row layout puts complex64 elements on 8-byte boundaries only).
-template <typename T> __device__ __forceinline__ void cp_elem(cx<T>* smem_dst, const cx<T>* gsrc) {
-    if constexpr (sizeof(cx<T>) == 16) cp16(smem_dst, gsrc);
-    else cp8(smem_dst, gsrc);
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
 // Blocks per SM the launch bounds target and shared buffers per block
 // (2 = double-buffered prefetch).
 // Resident blocks per SM the row kernel is compiled for: small blocks (up to
@@ -206,9 +167,6 @@ constexpr int row_minb(int th) { return FGPE_ROW_MINB ? FGPE_ROW_MINB : (th <= 1
 #endif
 #ifndef FGPE_COL_MINB
 #define FGPE_COL_MINB 2
-#endif
-#ifndef FGPE_COL_NBUF
-#define FGPE_COL_NBUF 1
 #endif
 #ifndef FGPE_TW_SMEM
 #define FGPE_TW_SMEM 0
@@ -418,166 +376,6 @@ __global__ void __launch_bounds__(WPB * 32, 2) k_row_warp(StepConst c, RowArgs a
     block_sum<MS>(acc, red, bsum);
     if (threadIdx.x < MS) a.part[(size_t)blockIdx.x * MS + threadIdx.x] = bsum[threadIdx.x];
     finish_norms<MS>(c, a.part, a.counter, a.info, red);
-}
-
-// --------------------------------------------------------- column kernel
-// Tiles of TX adjacent x positions, full lines of N along the transformed
-// axis; persistent over (x-tile, other) pairs.
-// PV: radix plan of the lines (cplan); a plan other than the handle's needs
-// a pass that transforms forward and back, with a.fline its position map.
-template <typename T, int MS, int N, int TX, int TH, int NBUF = FGPE_COL_NBUF, int PV = 0>
-__global__ void __launch_bounds__(TH, FGPE_COL_MINB) k_col_fast(StepConst c, ColArgs a) {
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
-    using CT = ColTile<N, TX>;
-    constexpr int LPN = CT::LPN;
-    constexpr int TILE = MS * LPN * TX;
-    constexpr int EPC = 16 / (int)sizeof(cx<T>);
-    // every 16-byte chunk starts at a multiple of EPC elements of a tile row
-    // of TX elements: destinations stay 16-byte aligned
-    static_assert(TX % EPC == 0, "column tile narrower than a 16-byte chunk");
-    constexpr int CPL = TX / EPC;                      // chunks per (m, e)
-    constexpr int NCH = MS * N * CPL;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    cx<T>* bufs = (cx<T>*)smraw;
-    __shared__ cx<T> usoc[TX * MS * MS];     // per-column SO-coupling matrices (z pass)
-    const long long np = c.npts;
-    const int nxt = c.nx / TX;
-    const int nother = (int)a.n_other;
-    const int ntiles = nxt * nother;
-    const cx<T>* tw = (const cx<T>*)a.tw;
-    if (FGPE_TW_SMEM) {
-        cx<T>* tws = bufs + NBUF * TILE;
-        for (int i = threadIdx.x; i < N; i += TH) tws[i] = tw[i];
-        tw = tws;
-    }
-    cx<T>* S = (cx<T>*)a.S;
-    T fac[MS];
-#pragma unroll
-    for (int m = 0; m < MS; ++m) fac[m] = (a.flags & COL_SCALE) ? (T)(a.info[INFO_SC + m] * a.cfac) : (T)1;
-
-    auto issue = [&](int tile, cx<T>* dst) {
-        const int x0 = (tile % nxt) * TX;
-        const long long off = (long long)(tile / nxt) * a.other_stride + x0;
-        for (int ch = threadIdx.x; ch < NCH; ch += TH) {
-            const int tc = (ch % CPL) * EPC;
-            const int q = ch / CPL;
-            const int e = q % N, m = q / N;
-            cp16(dst + (m * LPN + e + (e >> 3)) * TX + tc, S + (size_t)m * np + off + (size_t)e * a.axis_stride + tc);
-        }
-    };
-
-    int tile = blockIdx.x;
-    if (NBUF == 2) {
-        if (tile < ntiles) issue(tile, bufs);
-        cp_commit();
-    }
-    for (int it = 0; tile < ntiles; ++it, tile += gridDim.x) {
-        cx<T>* cur = bufs + (NBUF == 2 ? (it & 1) * TILE : 0);
-        if (NBUF == 2) {
-            const int nt = tile + gridDim.x;
-            if (nt < ntiles) issue(nt, bufs + ((it + 1) & 1) * TILE);
-            cp_commit();
-            cp_wait<1>();
-        } else {
-            issue(tile, cur);
-            cp_commit();
-            cp_wait<0>();
-        }
-        __syncthreads();
-        const int x0 = (tile % nxt) * TX;
-        const int oth = tile / nxt;
-        const long long off = (long long)oth * a.other_stride + x0;
-        // with KE/SOC in this pass the scale rides on the pointwise step
-        // (the transform is linear); otherwise it takes its own sweep
-        const bool fold = (a.flags & COL_SCALE) && (a.flags & COL_KOP);
-        if ((a.flags & COL_SCALE) && !fold) {
-            // component loop outermost and unrolled: fac[] stays in registers
-#pragma unroll
-            for (int m = 0; m < MS; ++m) {
-                for (int idx = threadIdx.x; idx < N * TX; idx += TH) {
-                    const int t = idx % TX, e = idx / TX;
-                    cx<T>& v = cur[(m * LPN + e + (e >> 3)) * TX + t];
-                    v = cscale(v, fac[m]);
-                }
-            }
-            __syncthreads();
-        }
-        if (a.flags & COL_FWD) ct_fft<T, false, N, MS * TX, TH, CT, 0, 0, PV>(cur, tw);
-        if (a.flags & COL_KOP) {
-            // z lines: (kx, ky) is fixed along each line of the tile, so the
-            // SO-coupling exponential is one MS x MS matrix per tile column,
-            // built here by applying apply_soc to the unit vectors and then
-            // applied to every point as one matrix-vector product
-            const bool zmat = a.axis == 2 && (a.flags & COL_SOC);
-            if (zmat) {
-                if (threadIdx.x < TX * MS) {
-                    const int t = threadIdx.x / MS, j = threadIdx.x - (threadIdx.x / MS) * MS;
-                    cx<T> u[MS];
-#pragma unroll
-                    for (int m = 0; m < MS; ++m) u[m] = mk<T>(m == j ? (T)1 : (T)0, (T)0);
-                    const int ixt = c.fx[x0 + t], iyt = a.fother[oth];
-                    apply_soc<T, MS>(c, c.kx[ixt], c.ky[iyt], u);
-                    // the kx, ky part of KE, exp(-i CDT (kx^2 + ky^2)), is a
-                    // scalar along the line: folded into the matrix
-                    const cx<T> f = (a.flags & COL_KE) ? fmul(c.imag, ((const cx<T>*)c.kex)[ixt], ((const cx<T>*)c.key)[iyt])
-                                                        : mk<T>((T)1, (T)0);
-#pragma unroll
-                    for (int r = 0; r < MS; ++r) usoc[(t * MS + r) * MS + j] = cmul(u[r], f);
-                }
-                __syncthreads();
-            }
-            for (int p = threadIdx.x; p < N * TX; p += TH) {
-                const int t = p % TX, e = p / TX;
-                const int ix = c.fx[x0 + t];
-                // y lines: ky at the line position; z lines: ky at the tile's y
-                int iy, iz;
-                if (a.axis == 1) { iy = a.fline[e]; iz = 0; } else { iy = a.fother[oth]; iz = a.fline[e]; }
-                cx<T> v[MS];
-#pragma unroll
-                for (int m = 0; m < MS; ++m) v[m] = cur[(m * LPN + e + (e >> 3)) * TX + t];
-                if (fold) {
-#pragma unroll
-                    for (int m = 0; m < MS; ++m) v[m] = cscale(v[m], fac[m]);
-                }
-                if (zmat) {
-                    if (a.flags & COL_KE) {
-                        // the kz part, exp(-i CDT (kz^2 - 2 L GAMMAZ kz)) per component
-                        const cx<T>* kez = (const cx<T>*)c.kez;
-#pragma unroll
-                        for (int m = 0; m < MS; ++m) v[m] = fmul(c.imag, kez[m * c.nz + iz], v[m]);
-                    }
-                } else if (a.flags & COL_KE) {
-                    apply_ke<T, MS>(c, ix, iy, iz, v);
-                }
-                if (zmat) {
-                    const cx<T>* U = usoc + t * MS * MS;
-                    cx<T> w[MS];
-#pragma unroll
-                    for (int r = 0; r < MS; ++r) {
-                        cx<T> acc = cmul(U[r * MS], v[0]);
-#pragma unroll
-                        for (int q = 1; q < MS; ++q) acc = cmac(acc, U[r * MS + q], v[q]);
-                        w[r] = acc;
-                    }
-#pragma unroll
-                    for (int m = 0; m < MS; ++m) v[m] = w[m];
-                } else if (a.flags & COL_SOC) {
-                    apply_soc<T, MS>(c, c.kx[ix], c.ky[iy], v);
-                }
-#pragma unroll
-                for (int m = 0; m < MS; ++m) cur[(m * LPN + e + (e >> 3)) * TX + t] = v[m];
-            }
-            __syncthreads();
-        }
-        if (a.flags & COL_INV) ct_fft<T, true, N, MS * TX, TH, CT, 0, 0, PV>(cur, tw);
-        for (int idx = threadIdx.x; idx < MS * N * TX; idx += TH) {
-            const int t = idx % TX, q = idx / TX, e = q % N, m = q / N;
-            S[(size_t)m * np + off + (size_t)e * a.axis_stride + t] = cur[(m * LPN + e + (e >> 3)) * TX + t];
-        }
-        __syncthreads();
-    }
-    cp_wait<0>();
-    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
 }  // namespace fgpe

@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(TH, FGPE_COL_MINB) k_col_group(GroupArgs g) {
 #pragma unroll
             for (int m = 0; m < MS; ++m) v[m] = cscale(cur[(m * LPN + e + (e >> 3)) * TX + tt], fac[m]);
             apply_ke<T, MS>(c, ix, iy, 0, v);
-            apply_soc<T, MS>(c, c.kx[ix], c.ky[iy], v);
+            if (c.soc) soc_apply<T, MS>(c.imag, ((const Soc4<T>*)c.soc)[(size_t)iy * c.nx + x0 + tt], v);
 #pragma unroll
             for (int m = 0; m < MS; ++m) cur[(m * LPN + e + (e >> 3)) * TX + tt] = v[m];
         }

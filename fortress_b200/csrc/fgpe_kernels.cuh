@@ -175,8 +175,11 @@ k_row(StepConst c, RowArgs a) {
 // ----------------------------------------------------------- column pass
 // A tile of TX adjacent x positions, full lines of length n along the
 // transformed axis (stride a.axis_stride), all MS components.
+// Three blocks per SM (FP32 four): the pass waits on its loads and barriers,
+// and left alone would take registers for one block fewer (96 x 80 x 120
+// spin-2 FP64: y pass 131 against 100 us).
 template <typename T, int MS>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4)
 k_col(StepConst c, ColArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T>* sm = (cx<T>*)smraw;
@@ -207,12 +210,12 @@ k_col(StepConst c, ColArgs a) {
             const int ix = c.fx[x0 + t];
             // y lines: ky at the line position; z lines: ky at the block's y
             int iy, iz;
-            if (a.axis == 1) { iy = c.fy[e]; iz = 0; } else { iy = c.fy[blockIdx.y]; iz = c.fz[e]; }
+            if (a.axis == 1) { iy = c.fy[e]; iz = 0; } else { iy = a.fother[blockIdx.y]; iz = c.fz[e]; }
             cx<T> v[MS];
 #pragma unroll
             for (int m = 0; m < MS; ++m) v[m] = sm[(m * lpn + pad_idx(e)) * TX + t];
             if (a.flags & COL_KE) apply_ke<T, MS>(c, ix, iy, iz, v);
-            if (a.flags & COL_SOC) apply_soc<T, MS>(c, c.kx[ix], c.ky[iy], v);
+            if ((a.flags & COL_SOC) && c.soc) soc_apply<T, MS>(c.imag, ((const Soc4<T>*)c.soc)[(size_t)iy * c.nx + x0 + t], v);
 #pragma unroll
             for (int m = 0; m < MS; ++m) sm[(m * lpn + pad_idx(e)) * TX + t] = v[m];
         }
@@ -860,6 +863,23 @@ __global__ void k_apply_scale(T* psi, long long n2, long long per2, double* info
 static __global__ void k_norms_out(const double* __restrict__ info, double* __restrict__ dst, int ms) {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     if ((int)threadIdx.x < ms) dst[threadIdx.x] = info[INFO_NORM + threadIdx.x];
+}
+
+// Fills the SO-coupling table of a 2D/3D handle, in FP64 arithmetic whatever T.
+template <typename T>
+__global__ void k_soc_table(StepConst c, Soc4<T>* soc) {
+    const long long n = (long long)c.nx * c.ny;
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+        const int x = (int)(t % c.nx), iy = (int)(t / c.nx);
+        const double kx = c.kx[c.fx[x]], ky = c.ky[iy];
+        const double ax = c.gx * kx, ay = c.gy * ky, r2 = ax * ax + ay * ay;
+        const double r = sqrt(r2), alpha = 2.0 * r;
+        Soc4<double> e = {1.0, 0.0, 1.0, c.imag ? 1.0 : 0.0};
+        if (alpha > 1.0e-40) { e.cb = ax / r; e.sb = ay / r; }
+        if (c.imag) { e.p = exp(-c.dt * alpha); e.q = exp(c.dt * alpha); }
+        else { sincos(c.dt * alpha, &e.q, &e.p); e.q = -e.q; }
+        soc[t] = {(T)e.cb, (T)e.sb, (T)e.p, (T)e.q};
+    }
 }
 
 // Unfused single operators on a full real/Fourier-space buffer (parity

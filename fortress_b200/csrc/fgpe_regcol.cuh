@@ -1,0 +1,359 @@
+// fgpe_regcol.cuh -- column passes with their transforms in registers.
+//
+// A tile is TX adjacent x positions by a whole line of N along y or z.  A
+// line is transformed by two or three radix passes (LPlan), and each thread
+// keeps whole butterflies in registers: the first pass reads its elements
+// straight from global memory (with the operators: from slots of its own that
+// an asynchronous copy has filled), the last one of an inverse transform
+// writes them straight back, and in the pass that carries KE and SOC the last
+// forward pass, the k-space operators and the first inverse pass are one
+// visit to registers that hold all MS components of the same spectral
+// positions.  Shared memory carries only the exchanges between radix passes:
+// two to four trips where passes over a shared tile take up to eight.
+//
+// Measured on one B200, 256^3 spin-1, against the shared-tile passes:
+//   y pass   FP64 0.33 -> 0.30 ms (5.3 TB/s, 0.81 of the measured copy
+//            rate), FP32 0.19 -> 0.14 ms (5.7 TB/s): bound by HBM;
+//   z pass   FP64 0.65 -> 0.41 ms, FP32 0.37 -> 0.25 ms: bound by latency at
+//            8 or 12 warps per SM, the FP64 pipe about half busy.  A thread
+//            holds 48 complex values there; (8,4,8) and (32,8) lines with
+//            twice the warps took 10 to 40 % longer.
+#pragma once
+#include "fgpe_async.cuh"
+#include "fgpe_dft.cuh"
+#include "fgpe_kernels.h"
+
+namespace fgpe {
+
+// Radix plan of a column line: two passes (R2 = 1) or three.
+template <int R0_, int R1_, int R2_ = 1> struct LPlan {
+    static constexpr int R0 = R0_, R1 = R1_, R2 = R2_;
+    static constexpr int N = R0 * R1 * R2;
+    static constexpr bool three = R2 > 1;
+    static constexpr int RL = three ? R2 : R1;      // radix of the last pass (contiguous positions)
+    // frequency of position q*RL is krev(q); position q*RL + r adds r*N/RL
+    static __host__ __device__ __forceinline__ int krev(int q) { return three ? q / R1 + R0 * (q % R1) : q; }
+};
+
+// COLK_FWD / COLK_INV: one transform of one component's lines (3D y passes);
+// COLK_Y2D: F_y, pending scale + KE + SOC, F_y^-1 (the q2D pass);
+// COLK_Z3D: F_z, KE and SOC as one matrix per tile column, F_z^-1.
+enum { COLK_FWD = 0, COLK_INV = 1, COLK_Y2D = 2, COLK_Z3D = 3 };
+
+template <typename T, int TX, int RL> struct RegTile {
+    // tile rows narrower than 128 bytes are padded by one row every RL, so
+    // that the strided butterflies of the last pass fall on distinct banks
+    static constexpr bool padded = TX * (int)sizeof(cx<T>) < 128;
+    static constexpr __host__ __device__ int rows(int n) { return padded ? n + n / RL : n; }
+    static __device__ __forceinline__ int at(int e, int t) { return (padded ? e + e / RL : e) * TX + t; }
+};
+
+template <typename T, int MS, int N, int TX, class PL, int KIND> constexpr size_t regcol_smem() {
+    return ((size_t)(KIND >= COLK_Y2D ? MS : 1) * RegTile<T, TX, PL::RL>::rows(N) * TX + (KIND == COLK_Z3D ? MS * N : 0)) * sizeof(cx<T>);
+}
+
+template <typename T> __device__ __forceinline__ cx<T> ld_stream(const cx<T>* p) { return __ldcg(p); }
+
+template <typename T, int MS, int N, int TX, int TH, int MINB, class PL, int KIND>
+__global__ void __launch_bounds__(TH, MINB) k_regcol(StepConst c, ColArgs a) {
+    static_assert(PL::N == N, "plan length");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    constexpr bool KOP = KIND >= COLK_Y2D;
+    constexpr int R0 = PL::R0, RL = PL::RL, S0 = N / R0, NQ = N / RL;
+    using TL = RegTile<T, TX, RL>;
+    constexpr int LINE = TL::rows(N) * TX;           // one component's tile
+    constexpr int T0 = S0 * TX, TF = NQ * TX;        // butterflies of the first / last pass per component
+    // components one thread takes through the outer passes together: all of
+    // them, on one set of twiddles, where that still occupies every thread
+    constexpr int CNT = KOP && T0 % TH == 0 && R0 <= 16 && MS * R0 <= 48 ? MS : 1;
+    constexpr int TOT0 = KOP ? MS / CNT * T0 : T0;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cx<T>* sm = (cx<T>*)smraw;
+    cx<T>* kez = sm + MS * LINE;                     // z pass: exp(-i CDT (kz^2 - 2 L GAMMAZ kz)) per component
+    const long long np = c.npts;
+    const int nxt = (c.nx + TX - 1) / TX;
+    const cx<T>* tw = (const cx<T>*)a.tw;
+    const long long st = a.axis_stride;
+    const int ncomp = KOP ? 1 : MS;
+    const int per = nxt * a.n_other;
+    const int ntiles = per * ncomp;
+    T fac[MS];
+#pragma unroll
+    for (int m = 0; m < MS; ++m)
+        fac[m] = (KIND == COLK_FWD || KIND == COLK_Y2D) ? (T)(a.info[INFO_SC + m] * a.cfac) : (T)1;
+
+    // where a thread's butterfly is the same in every tile, its twiddles stay
+    // in registers
+    constexpr bool KEEPW = T0 == TH;
+    Twiddles<T, R0> wq;
+    if constexpr (KEEPW) wq.load(tw, (threadIdx.x / TX) % S0, 1);
+    if constexpr (KIND == COLK_Z3D) {
+        for (int i = threadIdx.x; i < MS * N; i += TH) kez[i] = ((const cx<T>*)c.kez)[i];
+    }
+    // passes with the operators: a butterfly's slots of the first forward and
+    // of the last inverse pass belong to one thread, which refills them with
+    // the next tile's elements as soon as it has read the last pass's, so the
+    // copies overlap that pass's arithmetic and stores
+    auto fetch = [&](int tile, int m, int q, int t) {
+        const int oth = tile / nxt, x0 = (tile - oth * nxt) * TX;
+        if (t > c.nx - 1 - x0) return;
+        const cx<T>* g = (const cx<T>*)a.S + (size_t)m * np + (long long)oth * a.other_stride + x0 + t + (long long)q * st;
+#pragma unroll
+        for (int r = 0; r < R0; ++r) cp_elem<T>(sm + m * LINE + TL::at(q + r * S0, t), g + (long long)(r * S0) * st);
+    };
+    if constexpr (KOP) {
+        if (blockIdx.x < ntiles) {
+#pragma unroll 1
+            for (int b = threadIdx.x; b < MS * T0; b += TH) fetch(blockIdx.x, b / T0, (b / TX) % S0, b % TX);
+        }
+        cp_commit();
+    }
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+        const int comp = KOP ? 0 : tile / per;
+        const int rest = KOP ? tile : tile - comp * per;
+        const int oth = rest / nxt, x0 = (rest - oth * nxt) * TX;
+        cx<T>* S = (cx<T>*)a.S + (size_t)comp * np + (long long)oth * a.other_stride + x0;
+        const int last = c.nx - 1 - x0;            // tile columns past it are absent (nx not a multiple of TX)
+        T fc = (T)1;
+        if constexpr (KIND == COLK_FWD) {
+#pragma unroll
+            for (int m = 0; m < MS; ++m) fc = comp == m ? fac[m] : fc;
+        }
+        // z lines: (kx, ky) is fixed along a line, so its SO-coupling numbers and
+        // its part of KE come once per tile, ahead of their use (TH is a
+        // multiple of TX, so a thread keeps its line)
+        static_assert(TH % TX == 0, "threads per tile row");
+        cx<T> ke;
+        Soc4<T> so;
+        if constexpr (KIND == COLK_Z3D) {
+            const int x = x0 + min((int)threadIdx.x % TX, last), ix = c.fx[x], iy = a.fother[oth];
+            ke = fmul(c.imag, ((const cx<T>*)c.kex)[ix], ((const cx<T>*)c.key)[iy]);
+            if (c.soc) so = ((const Soc4<T>*)c.soc)[(size_t)iy * c.nx + x];
+        }
+        if constexpr (KIND != COLK_INV) {
+            // first forward pass; without the operators from global memory
+            if constexpr (KOP) cp_wait<0>();
+#pragma unroll 1
+            for (int b = threadIdx.x; b < TOT0; b += TH) {
+                const int t = b % TX, w = b / TX, q = w % S0, m0 = w / S0;
+                cx<T>* d = sm + m0 * LINE;
+                cx<T> v[CNT][R0];
+#pragma unroll
+                for (int m = 0; m < CNT; ++m) {
+                    if constexpr (KOP) {
+#pragma unroll
+                        for (int r = 0; r < R0; ++r) v[m][r] = d[m * LINE + TL::at(q + r * S0, t)];
+                    } else {
+                        const cx<T>* g = S + (long long)q * st + t;
+#pragma unroll
+                        for (int r = 0; r < R0; ++r) v[0][r] = t <= last ? ld_stream<T>(g + (long long)(r * S0) * st) : mk<T>(0, 0);
+#pragma unroll
+                        for (int r = 0; r < R0; ++r) v[0][r] = cscale(v[0][r], fc);
+                    }
+                    Dft<T, false, R0>::run(v[m]);
+                }
+                if constexpr (!KEEPW) wq.load(tw, q, 1);
+                if (q) wq.template apply<false, CNT>(v);
+#pragma unroll
+                for (int m = 0; m < CNT; ++m)
+#pragma unroll
+                    for (int r = 0; r < R0; ++r) d[m * LINE + TL::at(q + r * S0, t)] = v[m][r];
+            }
+            __syncthreads();
+            if constexpr (PL::three) {
+                constexpr int R1 = PL::R1, S1 = S0 / R1, NB = N / R1;
+                constexpr int TOT1 = (KOP ? MS : 1) * NB * TX;
+#pragma unroll 1
+                for (int b = threadIdx.x; b < TOT1; b += TH) {
+                    const int t = b % TX, w = b / TX, q = w % NB, m = w / NB;
+                    const int blk = q / S1, n2 = q - blk * S1, e0 = blk * S0 + n2;
+                    cx<T>* d = sm + m * LINE;
+                    cx<T> v[1][R1];
+#pragma unroll
+                    for (int r = 0; r < R1; ++r) v[0][r] = d[TL::at(e0 + r * S1, t)];
+                    Dft<T, false, R1>::run(v[0]);
+                    Twiddles<T, R1> w1;
+                    w1.load(tw, n2, R0);
+                    if (n2) w1.template apply<false, 1>(v);
+#pragma unroll
+                    for (int r = 0; r < R1; ++r) d[TL::at(e0 + r * S1, t)] = v[0][r];
+                }
+                __syncthreads();
+            }
+        }
+        if constexpr (KOP) {
+            // last forward pass, k-space operators, first inverse pass
+#pragma unroll 1
+            for (int b = threadIdx.x; b < TF; b += TH) {
+                const int t = b % TX, q = b / TX;
+                cx<T> v[MS][RL];
+#pragma unroll
+                for (int m = 0; m < MS; ++m) {
+#pragma unroll
+                    for (int r = 0; r < RL; ++r) v[m][r] = sm[m * LINE + TL::at(q * RL + r, t)];
+                    Dft<T, false, RL>::run(v[m]);
+                }
+                const int kq = PL::krev(q);
+                if constexpr (KIND == COLK_Z3D) {
+#pragma unroll
+                    for (int r = 0; r < RL; ++r) {
+                        cx<T> u[MS];
+#pragma unroll
+                        for (int m = 0; m < MS; ++m) u[m] = fmul(c.imag, fmul(c.imag, ke, kez[m * N + kq + r * NQ]), v[m][r]);
+                        if (c.soc) soc_apply<T, MS>(c.imag, so, u);
+#pragma unroll
+                        for (int m = 0; m < MS; ++m) v[m][r] = u[m];
+                    }
+                } else {
+                    const int ix = c.fx[x0 + min(t, last)];
+                    const Soc4<T>* soc = (const Soc4<T>*)c.soc + x0 + min(t, last);
+#pragma unroll
+                    for (int r = 0; r < RL; ++r) {
+                        const int iy = kq + r * NQ;
+                        cx<T> u[MS];
+#pragma unroll
+                        for (int m = 0; m < MS; ++m) u[m] = cscale(v[m][r], fac[m]);
+                        apply_ke<T, MS>(c, ix, iy, 0, u);
+                        if (c.soc) soc_apply<T, MS>(c.imag, soc[(size_t)iy * c.nx], u);
+#pragma unroll
+                        for (int m = 0; m < MS; ++m) v[m][r] = u[m];
+                    }
+                }
+#pragma unroll
+                for (int m = 0; m < MS; ++m) {
+                    Dft<T, true, RL>::run(v[m]);
+#pragma unroll
+                    for (int r = 0; r < RL; ++r) sm[m * LINE + TL::at(q * RL + r, t)] = v[m][r];
+                }
+            }
+            __syncthreads();
+        } else if constexpr (KIND == COLK_FWD) {
+            // last forward pass, to global memory in position order
+#pragma unroll 1
+            for (int b = threadIdx.x; b < TF; b += TH) {
+                const int t = b % TX, q = b / TX;
+                cx<T> v[RL];
+#pragma unroll
+                for (int r = 0; r < RL; ++r) v[r] = sm[TL::at(q * RL + r, t)];
+                Dft<T, false, RL>::run(v);
+                cx<T>* g = S + (long long)(q * RL) * st + t;
+                if (t <= last) {
+#pragma unroll
+                    for (int r = 0; r < RL; ++r) g[(long long)r * st] = v[r];
+                }
+            }
+            __syncthreads();
+        } else {
+            // first inverse pass, from global memory
+#pragma unroll 1
+            for (int b = threadIdx.x; b < TF; b += TH) {
+                const int t = b % TX, q = b / TX;
+                const cx<T>* g = S + (long long)(q * RL) * st + t;
+                cx<T> v[RL];
+#pragma unroll
+                for (int r = 0; r < RL; ++r) v[r] = t <= last ? ld_stream<T>(g + (long long)r * st) : mk<T>(0, 0);
+                Dft<T, true, RL>::run(v);
+#pragma unroll
+                for (int r = 0; r < RL; ++r) sm[TL::at(q * RL + r, t)] = v[r];
+            }
+            __syncthreads();
+        }
+        if constexpr (KIND != COLK_FWD) {
+            if constexpr (PL::three) {
+                constexpr int R1 = PL::R1, S1 = S0 / R1, NB = N / R1;
+                constexpr int TOT1 = (KOP ? MS : 1) * NB * TX;
+#pragma unroll 1
+                for (int b = threadIdx.x; b < TOT1; b += TH) {
+                    const int t = b % TX, w = b / TX, q = w % NB, m = w / NB;
+                    const int blk = q / S1, n2 = q - blk * S1, e0 = blk * S0 + n2;
+                    cx<T>* d = sm + m * LINE;
+                    cx<T> v[1][R1];
+#pragma unroll
+                    for (int r = 0; r < R1; ++r) v[0][r] = d[TL::at(e0 + r * S1, t)];
+                    Twiddles<T, R1> w1;
+                    w1.load(tw, n2, R0);
+                    if (n2) w1.template apply<true, 1>(v);
+                    Dft<T, true, R1>::run(v[0]);
+#pragma unroll
+                    for (int r = 0; r < R1; ++r) d[TL::at(e0 + r * S1, t)] = v[0][r];
+                }
+                __syncthreads();
+            }
+            // last inverse pass, to global memory
+#pragma unroll 1
+            for (int b = threadIdx.x; b < TOT0; b += TH) {
+                const int t = b % TX, w = b / TX, q = w % S0, m0 = w / S0;
+                const cx<T>* d = sm + m0 * LINE;
+                cx<T> v[CNT][R0];
+#pragma unroll
+                for (int m = 0; m < CNT; ++m)
+#pragma unroll
+                    for (int r = 0; r < R0; ++r) v[m][r] = d[m * LINE + TL::at(q + r * S0, t)];
+                if constexpr (KOP) {
+                    if (tile + (int)gridDim.x < ntiles)
+#pragma unroll
+                        for (int m = 0; m < CNT; ++m) fetch(tile + gridDim.x, m0 + m, q, t);
+                }
+                if constexpr (!KEEPW) wq.load(tw, q, 1);
+                if (q) wq.template apply<true, CNT>(v);
+#pragma unroll
+                for (int m = 0; m < CNT; ++m) {
+                    Dft<T, true, R0>::run(v[m]);
+                    cx<T>* g = S + (size_t)(m0 + m) * np + (long long)q * st + t;
+                    if (t <= last) {
+#pragma unroll
+                        for (int r = 0; r < R0; ++r) g[(long long)(r * S0) * st] = v[m][r];
+                    }
+                }
+            }
+            if constexpr (KOP) cp_commit();
+            else __syncthreads();
+        }
+    }
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+// ------------------------------------------------------- launch shapes
+// Radix plans.  Single-component passes take (N/16, 16): one exchange.  The z
+// pass of a grid that fills the GPU holds MS * RL complex values per thread
+// between its transforms, so RL = 16 with three components and 8 with five.
+// The q2D pass, and the z pass of a small grid, have few tiles and are bound
+// by one tile's latency: short last radices and more threads per tile
+// (512^2 spin-1 FP32: 16 us with (8, 16, 4) and 256 threads, 27 us with
+// (32, 16) and 128).
+template <int MS, int N, int KIND, bool BIG> struct ColPlan { using P = LPlan<N / 16, 16>; };
+template <int N> struct ColPlan<5, N, COLK_Z3D, true> { using P = LPlan<N / 8, 8>; };
+template <> struct ColPlan<5, 384, COLK_Z3D, true> { using P = LPlan<8, 6, 8>; };
+template <> struct ColPlan<5, 512, COLK_Z3D, true> { using P = LPlan<8, 8, 8>; };
+template <int N> struct SmallPlan { using P = LPlan<8, N / 32, 4>; };
+template <> struct SmallPlan<128> { using P = LPlan<8, 8, 2>; };
+template <int MS, int N> struct ColPlan<MS, N, COLK_Z3D, false> : SmallPlan<N> {};
+template <int N> struct ColPlan<5, N, COLK_Z3D, false> : SmallPlan<N> {};
+template <int MS, int N, bool BIG> struct ColPlan<MS, N, COLK_Y2D, BIG> : SmallPlan<N> {};
+
+template <typename T, int MS, int N, int KIND, bool BIG> struct ColShape {
+    using P = typename ColPlan<MS, N, KIND, BIG>::P;
+    static constexpr bool KOP = KIND >= COLK_Y2D, F64 = sizeof(T) == 8;
+    static constexpr bool SMALL = KIND == COLK_Y2D || (KIND == COLK_Z3D && !BIG);
+    // x positions per tile.  Single-component passes: 128 bytes.  Big z
+    // tiles: the widest that leaves room for two (FP64) or three (FP32)
+    // blocks per SM.  Small tiles: 2 positions, 4 where FP32 lines are long.
+    static constexpr int ROOM = F64 ? 108 * 1024 : 74 * 1024;
+    static constexpr int TXB = !KOP || MS * N * 128 <= ROOM ? 128 : MS * N * 64 <= ROOM ? 64 : 32;
+    static constexpr int TX = SMALL ? (!F64 && N >= 384 ? 4 : 2) : TXB / (int)sizeof(cx<T>);
+    // threads: one butterfly of the operator pass (or of the wider pass of a
+    // single-component kernel) each
+    static constexpr int TASKS = TX * (KOP ? N / P::RL : 16);
+    static constexpr int TH = SMALL ? (N == 128 || (F64 && N >= 384) ? 128 : 256) : TASKS < 64 ? 64 : (TASKS + 31) / 32 * 32;
+    // threads per SM that share the register file
+    static constexpr int PER_SM = SMALL ? (F64 || MS == 5 ? 256 : 512)
+                                  : KOP ? (F64 ? 256 : 384)
+                                        : (F64 ? (P::R0 > 16 ? 256 : 512) : (P::R0 > 16 ? 512 : 768));
+    static constexpr size_t SMEM = regcol_smem<T, MS, N, TX, P, KIND>();
+    static constexpr int FIT = (int)((226 * 1024) / (SMEM + 1024));
+    static constexpr int MINB0 = PER_SM / TH < 1 ? 1 : PER_SM / TH;
+    static constexpr int MINB = MINB0 < FIT ? MINB0 : (FIT < 1 ? 1 : FIT);
+    static constexpr auto kernel() { return k_regcol<T, MS, N, TX, TH, MINB, P, KIND>; }
+};
+
+}  // namespace fgpe

@@ -1,0 +1,6 @@
+// Register-resident step passes, double complex, spin 1 (fgpe_step.h).
+#include "fgpe_step_impl.cuh"
+
+namespace fgpe {
+FGPE_STEP_INSTANTIATE(double, 3)
+}  // namespace fgpe
