@@ -84,6 +84,9 @@ struct fgpe_s {
     // row pass with one warp per x row (k_row_warp), where a row fits 16 KB
     bool has_warp_row = false, warp_row = false;
     int warp_row_grid = 0;
+    // spin-1 row pass with its transforms in registers (fgpe_regrow.cuh)
+    bool reg_row = false;
+    int reg_row_grid = 0;
     bool psi_valid = false, S_valid = false, prev_valid = false, norms_valid = false, has_state = false;
     long long launches = 0;
     std::string msg;
@@ -270,6 +273,12 @@ template <typename T, int MS, int N> void run_warp_row(fgpe_t* h, const RowArgs&
         default: break;                  \
     }
 
+// Rows from which AUTO takes the one-warp-per-row passes.  Below, a warp per
+// row leaves schedulers empty and the block pass is faster (us, warp / block,
+// 256-point spin-1 rows: FP64 512 rows 19.7 / 16.8, 2048 31.1 / 35.3, 16384
+// 156 / 195; FP32 512 rows 16.8 / 15.4, 1024 18.9 / 20.9, 16384 95 / 149).
+constexpr long long many_rows(bool fp32) { return fp32 ? 1024 : 2048; }
+
 bool fast_size(int n) {
     for (int v : kFastN) if (v == n) return true;
     return false;
@@ -293,6 +302,15 @@ struct ProfScope {
     }
 };
 
+// Row pass of a kernel family.  AUTO: k_regrow (spin-1) or k_row_warp (spin-2
+// FP64) from many_rows() rows, below that the block pass.
+void choose_row_pass(fgpe_t* h, int kernels) {
+    const long long rows = (long long)h->p.ny * h->p.nz;
+    const bool autom = kernels == FGPE_KERNELS_AUTO, many = rows >= many_rows(h->fp32);
+    h->reg_row = h->reg_row_grid > 0 && autom && many;
+    h->warp_row = h->has_warp_row && (kernels == FGPE_KERNELS_WARP_ROW || (autom && many && !h->fp32 && !h->reg_row));
+}
+
 // ---------------------------------------------------------------- launches
 template <typename T, int MS>
 void launch_row(fgpe_t* h, int mode, void* snap) {
@@ -300,6 +318,13 @@ void launch_row(fgpe_t* h, int mode, void* snap) {
     a.S = h->S; a.psi = h->psi; a.snap = snap; a.part = h->part; a.counter = h->counters;
     a.info = h->info; a.rows = h->row.tile; a.mode = mode;
     ProfScope ps(h, 0);
+    if constexpr (MS == 3) {
+        if (h->reg_row && mode == ROW_FULL) {
+            regrow_launch<T>(h->p.nx, h->reg_row_grid, h->sc, a, h->st, use_pdl(h));
+            h->launches++;
+            return;
+        }
+    }
     if (h->warp_row && mode == ROW_FULL) {
 #define RUNW(NN) run_warp_row<T, MS, NN>(h, a)
         FAST_SWITCH(h->p.nx, RUNW)
@@ -713,21 +738,20 @@ int fgpe_create(const fgpe_params* pin, fgpe_t** out) {
         c.fx = h->pmap + offp[0]; c.fy = h->pmap + offp[1]; c.fz = h->pmap + offp[2];
     }
     const size_t bytes = (size_t)h->npts * h->ms * h->cs;
-    // the SO-coupling table (fgpe_device.cuh, Soc4) follows S in its allocation
-    const bool soc_on = p.dim >= 2 && (c.gx != 0.0 || c.gy != 0.0);
-    const size_t nxy = (size_t)p.nx * p.ny, soc_at = (bytes + 255) / 256 * 256;
-    CK(cudaMalloc(&h->S, soc_at + (soc_on ? nxy * 2 * h->cs : 0)));
-    if (soc_on) c.soc = (char*)h->S + soc_at;
+    CK(cudaMalloc(&h->S, bytes));
     CK(cudaMalloc(&h->psi, bytes));
     CK(cudaMalloc(&h->prev, bytes));
     CK(cudaMalloc(&h->dtab, dt_all.size() * sizeof(double)));
     CK(cudaMemcpy(h->dtab, dt_all.data(), dt_all.size() * sizeof(double), cudaMemcpyHostToDevice));
+    // the SO-coupling table (fgpe_device.cuh, Soc4) follows the complex tables
+    const bool soc_on = p.dim >= 2 && (c.gx != 0.0 || c.gy != 0.0);
+    const size_t nxy = (size_t)p.nx * p.ny, soc_at = (ct.size() / 2 * h->cs + 255) / 256 * 256;
+    CK(cudaMalloc(&h->ctab, soc_at + (soc_on ? nxy * 2 * h->cs : 0)));
+    if (soc_on) c.soc = (char*)h->ctab + soc_at;
     if (h->fp32) {
         std::vector<float> f(ct.begin(), ct.end());
-        CK(cudaMalloc(&h->ctab, f.size() * sizeof(float)));
         CK(cudaMemcpy(h->ctab, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice));
     } else {
-        CK(cudaMalloc(&h->ctab, ct.size() * sizeof(double)));
         CK(cudaMemcpy(h->ctab, ct.data(), ct.size() * sizeof(double), cudaMemcpyHostToDevice));
     }
     const size_t ces = h->cs;  // bytes per complex table entry
@@ -838,8 +862,9 @@ int fgpe_create(const fgpe_params* pin, fgpe_t** out) {
         if (gw > 0) {
             h->has_warp_row = true;
             h->warp_row_grid = gw;
-            h->warp_row = p.kernels == FGPE_KERNELS_WARP_ROW || (p.kernels == FGPE_KERNELS_AUTO && !h->fp32);
         }
+        if (ms == 3) h->reg_row_grid = h->fp32 ? regrow_grid<float>(p.nx, p.ny * p.nz) : regrow_grid<double>(p.nx, p.ny * p.nz);
+        choose_row_pass(h, p.kernels);
     }
     for (int a = 1; a < p.dim; ++a) {
         if (!allow_fast_col || !fast_size(ns[a])) continue;
@@ -872,7 +897,7 @@ int fgpe_create(const fgpe_params* pin, fgpe_t** out) {
     const size_t nq = 3 * ms + 3;
     const size_t npart = std::max<size_t>(std::max<size_t>((size_t)h->obsl.grid.x * nq,
                                                            (size_t)std::max<int>(std::max<int>(h->row.grid.x, h->fast_row_grid),
-                                                                                 h->warp_row_grid) * ms),
+                                                                                 std::max(h->warp_row_grid, h->reg_row_grid)) * ms),
                                           (size_t)h->c1d.grid.x * ms) + 64;
     CK(cudaMalloc(&h->part, npart * sizeof(double)));
     CK(cudaMalloc(&h->info, 4 * INFO_LEN * sizeof(double)));
@@ -1261,7 +1286,7 @@ int fgpe_set_kernels(fgpe_t* h, int kernels) {
     if (h->bulk) { CK(cudaStreamSynchronize(h->st)); cudaGraphExecDestroy(h->bulk); h->bulk = nullptr; }
     const bool fast = kernels != FGPE_KERNELS_GENERIC;
     h->fast_row = fast && h->has_fast_row && kernels != FGPE_KERNELS_FAST_COL_ONLY;
-    h->warp_row = h->has_warp_row && (kernels == FGPE_KERNELS_WARP_ROW || (kernels == FGPE_KERNELS_AUTO && !h->fp32));
+    choose_row_pass(h, kernels);
     for (int a = 0; a < 3; ++a) h->fast_col[a] = fast && h->has_fast_col[a] && kernels != FGPE_KERNELS_FAST_ROW_ONLY;
     return FGPE_OK;
 }

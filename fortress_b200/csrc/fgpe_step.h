@@ -20,6 +20,12 @@ cudaError_t regcol_launch(int n, int kind, int wide, int grid, const StepConst& 
 // pass reads.
 inline int regcol_radices(int n, int* r) { r[0] = n / 16; r[1] = 16; return 2; }
 
+// Row pass of spin-1 lines of the same lengths (fgpe_regrow.cuh): resident
+// grid for the given number of rows (0: not available).
+template <typename T> int regrow_grid(int n, int rows);
+template <typename T>
+cudaError_t regrow_launch(int n, int grid, const StepConst& c, const RowArgs& a, cudaStream_t st, bool pdl);
+
 // Launch as a programmatic dependent (pdl): the pass is launched while the
 // previous one drains and waits on griddepcontrol.wait before it touches the
 // state.  Grids are one wave of resident blocks, so a waiting block never
@@ -55,6 +61,12 @@ template <class K> inline int resident_grid(K kern, int th, size_t smem, long lo
     extern template int regcol_grid<T, MS>(int, int, int, int, int*);                                        \
     extern template cudaError_t regcol_launch<T, MS>(int, int, int, int, const StepConst&, const ColArgs&,   \
                                                      cudaStream_t, bool);
+#define FGPE_STEP_ROW_EXTERN(T)                                                                              \
+    extern template int regrow_grid<T>(int, int);                                                            \
+    extern template cudaError_t regrow_launch<T>(int, int, const StepConst&, const RowArgs&, cudaStream_t, bool);
+FGPE_STEP_ROW_EXTERN(float)
+FGPE_STEP_ROW_EXTERN(double)
+#undef FGPE_STEP_ROW_EXTERN
 FGPE_STEP_EXTERN(float, 3)
 FGPE_STEP_EXTERN(float, 5)
 FGPE_STEP_EXTERN(double, 3)

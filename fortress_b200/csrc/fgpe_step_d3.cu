@@ -3,4 +3,5 @@
 
 namespace fgpe {
 FGPE_STEP_INSTANTIATE(double, 3)
+FGPE_STEP_ROW_INSTANTIATE(double)
 }  // namespace fgpe

@@ -3,4 +3,5 @@
 
 namespace fgpe {
 FGPE_STEP_INSTANTIATE(float, 3)
+FGPE_STEP_ROW_INSTANTIATE(float)
 }  // namespace fgpe

@@ -2,6 +2,7 @@
 // included by one translation unit per (precision, spin).
 #pragma once
 #include "fgpe_regcol.cuh"
+#include "fgpe_regrow.cuh"
 #include "fgpe_step.h"
 
 namespace fgpe {
@@ -67,6 +68,44 @@ cudaError_t regcol_launch(int n, int kind, int wide, int grid, const StepConst& 
         default: return cudaErrorInvalidValue;
     }
 }
+
+template <typename T> int regrow_grid(int n, int rows) {
+    switch (n) {
+#define G(NN)                                                                                                       \
+    case NN:                                                                                                        \
+        if constexpr (RowShape<T, NN>::RW > 0) {                                                                    \
+            using H = RowShape<T, NN>;                                                                              \
+            constexpr int per = H::RW * H::WPB;                                                                     \
+            return resident_grid(k_regrow<T, 3, NN, H::RW, H::WPB, H::MINB>, H::WPB * 32,                           \
+                                 H::WPB * regrow_warp_smem<T, 3, NN, H::RW>(), (rows + per - 1) / per);             \
+        }                                                                                                           \
+        return 0;
+        FGPE_STEP_SIZES(G)
+#undef G
+        default: return 0;
+    }
+}
+
+template <typename T>
+cudaError_t regrow_launch(int n, int grid, const StepConst& c, const RowArgs& a, cudaStream_t st, bool pdl) {
+    switch (n) {
+#define L(NN)                                                                                                       \
+    case NN:                                                                                                        \
+        if constexpr (RowShape<T, NN>::RW > 0) {                                                                    \
+            using H = RowShape<T, NN>;                                                                              \
+            return launch_step_kernel(k_regrow<T, 3, NN, H::RW, H::WPB, H::MINB>, grid, H::WPB * 32,                \
+                                      H::WPB * regrow_warp_smem<T, 3, NN, H::RW>(), c, a, st, pdl);                 \
+        }                                                                                                           \
+        return cudaErrorInvalidValue;
+        FGPE_STEP_SIZES(L)
+#undef L
+        default: return cudaErrorInvalidValue;
+    }
+}
+
+#define FGPE_STEP_ROW_INSTANTIATE(T)            \
+    template int regrow_grid<T>(int, int);      \
+    template cudaError_t regrow_launch<T>(int, int, const StepConst&, const RowArgs&, cudaStream_t, bool);
 
 #define FGPE_STEP_INSTANTIATE(T, MS)                                                                  \
     template int regcol_grid<T, MS>(int, int, int, int, int*);                                        \
