@@ -155,9 +155,6 @@ template <class K> cudaError_t allow_smem(K kern) {
     return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
 }
 
-template <class K> cudaError_t allow_smem_exact(K kern, size_t bytes) {
-    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
 
 template <typename T, int MS> cudaError_t set_smem_attrs() {
     cudaError_t e = allow_smem(k_row<T, MS>);
@@ -174,73 +171,6 @@ template <typename T, int MS> cudaError_t set_smem_attrs() {
 // kernels (same layout and results).
 constexpr int kFastN[] = {128, 192, 256, 384, 512};
 
-#ifndef FGPE_COL_TX32
-#define FGPE_COL_TX32 2
-#endif
-template <typename T> constexpr int col_tx() { return sizeof(T) == 8 ? 2 : FGPE_COL_TX32; }
-// Rows per row-kernel tile (FGPE_ROW_R256 fixes it for 256-point rows at
-// build time).
-#ifndef FGPE_ROW_R256
-#define FGPE_ROW_R256 0
-#endif
-constexpr int row_r(int n) { return n >= 384 ? 1 : (n == 256 && FGPE_ROW_R256 ? FGPE_ROW_R256 : 512 / n); }
-constexpr int fast_threads(int tot) {
-    const int iter = (tot + 511) / 512;
-    const int per = (tot + iter - 1) / iter;
-    return (per + 31) / 32 * 32;
-}
-// Thread counts of the size-specialised kernels: one radix-8 butterfly per
-// thread and pass unless FGPE_ROW_TH / FGPE_COL_TH fix them at build time.
-#ifndef FGPE_ROW_TH
-#define FGPE_ROW_TH 0
-#endif
-#ifndef FGPE_COL_TH
-#define FGPE_COL_TH 0
-#endif
-template <typename T, int MS, int N> constexpr int row_th() {
-    return FGPE_ROW_TH ? FGPE_ROW_TH : fast_threads(MS * row_r(N) * N / 8);
-}
-template <typename T, int MS, int N> constexpr int col_th() {
-    return FGPE_COL_TH ? FGPE_COL_TH : fast_threads(MS * col_tx<T>() * N / 8);
-}
-template <typename T, int MS, int N> constexpr size_t row_smem() {
-    return ((size_t)FGPE_ROW_NBUF * MS * row_r(N) * cpad(N) + (FGPE_TW_SMEM ? N : 0)) * sizeof(cx<T>);
-}
-template <class K> int grid_for(K kern, int th, size_t smem, int ntiles) {
-    int dev = 0, nsm = 0, per = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (allow_smem_exact(kern, smem) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, th, smem) != cudaSuccess || per < 1) return 0;
-    return std::min(ntiles, per * nsm);
-}
-
-template <typename T, int MS, int N> int setup_fast_row(fgpe_t* h) {
-    const int rows = h->p.ny * h->p.nz;
-    if (rows % row_r(N)) return 0;
-    return grid_for(k_row_fast<T, MS, N, row_r(N), row_th<T, MS, N>()>, row_th<T, MS, N>(), row_smem<T, MS, N>(),
-                    rows / row_r(N));
-}
-// Warp-row kernel: rows of MS lines up to 16 KB (FP64 spin-1 to 256 points,
-// spin-2 to 128; FP32 spin-1 to 512, spin-2 to 256); warps per block so that
-// two blocks of NBUF rows per warp fit the shared memory.
-template <typename T, int MS, int N> constexpr size_t wrow_tile() { return (size_t)MS * cpad(N) * sizeof(cx<T>); }
-template <typename T, int MS, int N> constexpr bool wrow_ok() { return wrow_tile<T, MS, N>() <= 16 * 1024; }
-template <typename T, int MS, int N> constexpr int wrow_wpb() {
-    const int w = (int)((110 * 1024) / (wrow_tile<T, MS, N>() * FGPE_WROW_NBUF));
-    return w < 1 ? 1 : (w > 8 ? 8 : w);
-}
-template <typename T, int MS, int N> int setup_warp_row(fgpe_t* h) {
-    if constexpr (!wrow_ok<T, MS, N>()) {
-        return 0;
-    } else {
-        constexpr int W = wrow_wpb<T, MS, N>();
-        const int rows = h->p.ny * h->p.nz;
-        return grid_for(k_row_warp<T, MS, N, W, FGPE_WROW_NBUF>, W * 32,
-                        (size_t)W * FGPE_WROW_NBUF * wrow_tile<T, MS, N>(), (rows + W - 1) / W);
-    }
-}
-
 // The size-specialised kernels go out as programmatic dependent launches
 // (launch_step_kernel), outside stream capture.
 bool use_pdl(fgpe_t* h) {
@@ -248,31 +178,6 @@ bool use_pdl(fgpe_t* h) {
     cudaStreamIsCapturing(h->st, &cs);
     return cs == cudaStreamCaptureStatusNone;
 }
-template <class K, class A>
-void launch_pdl(fgpe_t* h, K kern, int grid, int threads, size_t smem, const A& a) {
-    launch_step_kernel(kern, grid, threads, smem, h->sc, a, h->st, use_pdl(h));
-}
-template <typename T, int MS, int N> void run_fast_row(fgpe_t* h, const RowArgs& a) {
-    launch_pdl(h, k_row_fast<T, MS, N, row_r(N), row_th<T, MS, N>()>, h->fast_row_grid, row_th<T, MS, N>(),
-               row_smem<T, MS, N>(), a);
-}
-template <typename T, int MS, int N> void run_warp_row(fgpe_t* h, const RowArgs& a) {
-    if constexpr (wrow_ok<T, MS, N>()) {
-        constexpr int W = wrow_wpb<T, MS, N>();
-        launch_pdl(h, k_row_warp<T, MS, N, W, FGPE_WROW_NBUF>, h->warp_row_grid, W * 32,
-                   (size_t)W * FGPE_WROW_NBUF * wrow_tile<T, MS, N>(), a);
-    }
-}
-#define FAST_SWITCH(n, CALL)            \
-    switch (n) {                         \
-        case 128: CALL(128); break;      \
-        case 192: CALL(192); break;      \
-        case 256: CALL(256); break;      \
-        case 384: CALL(384); break;      \
-        case 512: CALL(512); break;      \
-        default: break;                  \
-    }
-
 // Rows from which AUTO takes the one-warp-per-row passes.  Below, a warp per
 // row leaves schedulers empty and the block pass is faster (us, warp / block,
 // 256-point spin-1 rows: FP64 512 rows 19.7 / 16.8, 2048 31.1 / 35.3, 16384
@@ -326,16 +231,12 @@ void launch_row(fgpe_t* h, int mode, void* snap) {
         }
     }
     if (h->warp_row && mode == ROW_FULL) {
-#define RUNW(NN) run_warp_row<T, MS, NN>(h, a)
-        FAST_SWITCH(h->p.nx, RUNW)
-#undef RUNW
+        row_launch<T, MS>(h->p.nx, true, h->warp_row_grid, h->sc, a, h->st, use_pdl(h));
         h->launches++;
         return;
     }
     if (h->fast_row) {
-#define RUNR(NN) run_fast_row<T, MS, NN>(h, a)
-        FAST_SWITCH(h->p.nx, RUNR)
-#undef RUNR
+        row_launch<T, MS>(h->p.nx, false, h->fast_row_grid, h->sc, a, h->st, use_pdl(h));
         h->launches++;
         return;
     }
@@ -848,22 +749,16 @@ int fgpe_create(const fgpe_params* pin, fgpe_t** out) {
     const bool allow_fast_row = allow_fast && p.kernels != FGPE_KERNELS_FAST_COL_ONLY;
     const bool allow_fast_col = allow_fast && p.kernels != FGPE_KERNELS_FAST_ROW_ONLY;
     if (allow_fast_row && p.dim >= 2 && fast_size(p.nx)) {
-        int g = 0;
-#define SETR(NN) g = h->fp32 ? (ms == 3 ? setup_fast_row<float, 3, NN>(h) : setup_fast_row<float, 5, NN>(h)) \
-                             : (ms == 3 ? setup_fast_row<double, 3, NN>(h) : setup_fast_row<double, 5, NN>(h))
-        FAST_SWITCH(p.nx, SETR)
-#undef SETR
-        if (g > 0) { h->fast_row = h->has_fast_row = true; h->fast_row_grid = g; }
-        int gw = 0;
-#define SETW(NN) gw = h->fp32 ? (ms == 3 ? setup_warp_row<float, 3, NN>(h) : setup_warp_row<float, 5, NN>(h)) \
-                              : (ms == 3 ? setup_warp_row<double, 3, NN>(h) : setup_warp_row<double, 5, NN>(h))
-        FAST_SWITCH(p.nx, SETW)
-#undef SETW
-        if (gw > 0) {
-            h->has_warp_row = true;
-            h->warp_row_grid = gw;
-        }
-        if (ms == 3) h->reg_row_grid = h->fp32 ? regrow_grid<float>(p.nx, p.ny * p.nz) : regrow_grid<double>(p.nx, p.ny * p.nz);
+        const int rows = p.ny * p.nz;
+        auto grid = [&](bool warp) {
+            return h->fp32 ? (ms == 3 ? row_grid<float, 3>(p.nx, warp, rows) : row_grid<float, 5>(p.nx, warp, rows))
+                           : (ms == 3 ? row_grid<double, 3>(p.nx, warp, rows) : row_grid<double, 5>(p.nx, warp, rows));
+        };
+        h->fast_row_grid = grid(false);
+        h->fast_row = h->has_fast_row = h->fast_row_grid > 0;
+        h->warp_row_grid = grid(true);
+        h->has_warp_row = h->warp_row_grid > 0;
+        if (ms == 3) h->reg_row_grid = h->fp32 ? regrow_grid<float>(p.nx, rows) : regrow_grid<double>(p.nx, rows);
         choose_row_pass(h, p.kernels);
     }
     for (int a = 1; a < p.dim; ++a) {
@@ -1395,7 +1290,7 @@ struct BatchGroup {
     InstDesc* h_desc = nullptr;      // pinned staging of the descriptors
     double* part = nullptr;          // NORMC chunk partials [members][chunks][MS]
     unsigned* counter = nullptr;     // per-instance chunk counters
-    int row_tiles = 0, chunk = 0, col_tiles = 0, row_grid = 0, col_grid = 0;
+    GroupShape shape;
 };
 
 // Persistent mode: the instances of one spin and precision that the
@@ -1510,68 +1405,21 @@ int capture(fgpe_batch_t* b, int nsteps) {
     return FGPE_OK;
 }
 // ----------------------------------------------------------- grouped mode
-constexpr int group_chunk(int tiles) {
-    int c = 1;
-    for (int d = 1; d <= 16; ++d) if (tiles % d == 0) c = d;
-    return c;
-}
-template <typename T, int MS, int NX> int setup_group_row(BatchGroup& g) {
-    constexpr int R = row_r(NX), TH = row_th<T, MS, NX>();
-    if (g.ny % R) return FGPE_E_ARG;
-    g.row_tiles = g.ny / R;
-    g.chunk = group_chunk(g.row_tiles);
-    const size_t smem = (size_t)FGPE_ROW_NBUF * MS * R * cpad(NX) * sizeof(cx<T>);
-    g.row_grid = grid_for(k_row_group<T, MS, NX, R, TH>, TH, smem, (int)g.members.size() * (g.row_tiles / g.chunk));
-    return g.row_grid > 0 ? FGPE_OK : FGPE_E_CUDA;
-}
-template <typename T, int MS, int NY> int setup_group_col(BatchGroup& g) {
-    constexpr int TX = col_tx<T>(), TH = col_th<T, MS, NY>();
-    if (g.nx % TX) return FGPE_E_ARG;
-    g.col_tiles = g.nx / TX;
-    const size_t smem = (size_t)MS * cpad(NY) * TX * sizeof(cx<T>);
-    g.col_grid = grid_for(k_col_group<T, MS, NY, TX, TH>, TH, smem, (int)g.members.size() * g.col_tiles);
-    return g.col_grid > 0 ? FGPE_OK : FGPE_E_CUDA;
-}
-template <typename T, int MS, int NX> void launch_group_row(const BatchGroup& g, int snap, cudaStream_t st) {
-    constexpr int R = row_r(NX), TH = row_th<T, MS, NX>();
-    const size_t smem = (size_t)FGPE_ROW_NBUF * MS * R * cpad(NX) * sizeof(cx<T>);
-    GroupArgs a{g.d_desc, (int)g.members.size(), g.row_tiles, g.chunk, snap};
-    k_row_group<T, MS, NX, R, TH><<<g.row_grid, TH, smem, st>>>(a);
-}
-template <typename T, int MS, int NY> void launch_group_col(const BatchGroup& g, cudaStream_t st) {
-    constexpr int TX = col_tx<T>(), TH = col_th<T, MS, NY>();
-    const size_t smem = (size_t)MS * cpad(NY) * TX * sizeof(cx<T>);
-    GroupArgs a{g.d_desc, (int)g.members.size(), g.col_tiles, 1, 0};
-    k_col_group<T, MS, NY, TX, TH><<<g.col_grid, TH, smem, st>>>(a);
-}
-template <typename T, int MS> int group_setup_tm(BatchGroup& g) {
-    int r = FGPE_E_ARG;
-#define GR(NN) r = setup_group_row<T, MS, NN>(g)
-    FAST_SWITCH(g.nx, GR)
-#undef GR
-    if (r) return r;
-    r = FGPE_E_ARG;
-#define GC(NN) r = setup_group_col<T, MS, NN>(g)
-    FAST_SWITCH(g.ny, GC)
-#undef GC
-    return r;
-}
-template <typename T, int MS> void group_launch_tm(const BatchGroup& g, int snap, cudaStream_t st) {
-#define GC(NN) launch_group_col<T, MS, NN>(g, st)
-    FAST_SWITCH(g.ny, GC)
-#undef GC
-#define GR(NN) launch_group_row<T, MS, NN>(g, snap, st)
-    FAST_SWITCH(g.nx, GR)
-#undef GR
-}
-int group_setup(BatchGroup& g) {
-    if (g.fp32) return g.ms == 3 ? group_setup_tm<float, 3>(g) : group_setup_tm<float, 5>(g);
-    return g.ms == 3 ? group_setup_tm<double, 3>(g) : group_setup_tm<double, 5>(g);
+bool group_setup(BatchGroup& g) {
+    const int n = (int)g.members.size();
+    if (g.fp32) return g.ms == 3 ? group_shape<float, 3>(g.nx, g.ny, n, &g.shape) : group_shape<float, 5>(g.nx, g.ny, n, &g.shape);
+    return g.ms == 3 ? group_shape<double, 3>(g.nx, g.ny, n, &g.shape) : group_shape<double, 5>(g.nx, g.ny, n, &g.shape);
 }
 // One whole step of every instance of g: the column pass, then the row pass.
 void group_step(const BatchGroup& g, int snap, cudaStream_t st) {
-    if (g.fp32) { if (g.ms == 3) group_launch_tm<float, 3>(g, snap, st); else group_launch_tm<float, 5>(g, snap, st); }
-    else { if (g.ms == 3) group_launch_tm<double, 3>(g, snap, st); else group_launch_tm<double, 5>(g, snap, st); }
+    const int n = (int)g.members.size();
+    if (g.fp32) {
+        if (g.ms == 3) group_launch<float, 3>(g.nx, g.ny, g.shape, g.d_desc, n, snap, st);
+        else group_launch<float, 5>(g.nx, g.ny, g.shape, g.d_desc, n, snap, st);
+    } else {
+        if (g.ms == 3) group_launch<double, 3>(g.nx, g.ny, g.shape, g.d_desc, n, snap, st);
+        else group_launch<double, 5>(g.nx, g.ny, g.shape, g.d_desc, n, snap, st);
+    }
 }
 
 void free_groups(fgpe_batch_t* b) {
@@ -1605,10 +1453,9 @@ int build_groups(fgpe_batch_t* b) {
         g->members.push_back(i);
     }
     for (BatchGroup& g : b->groups) {
-        int r = group_setup(g);
-        if (r) { free_groups(b); return bfail(b, r, "grouped batch: no launch shape for a group"); }
+        if (!group_setup(g)) { free_groups(b); return bfail(b, FGPE_E_CUDA, "grouped batch: no launch shape for a group"); }
         const size_t n = g.members.size();
-        const size_t slots = n * (size_t)(g.row_tiles / g.chunk) * g.ms;
+        const size_t slots = n * (size_t)(g.shape.row_tiles / g.shape.chunk) * g.ms;
         BCK(cudaMalloc(&g.d_desc, n * sizeof(InstDesc)));
         BCK(cudaMallocHost(&g.h_desc, n * sizeof(InstDesc)));
         BCK(cudaMalloc(&g.part, slots * sizeof(double)));
@@ -1623,7 +1470,7 @@ int build_groups(fgpe_batch_t* b) {
 // of the graph launch on the batch's launch stream.
 int refresh_descs(fgpe_batch_t* b) {
     for (BatchGroup& g : b->groups) {
-        const int nci = g.row_tiles / g.chunk;
+        const int nci = g.shape.row_tiles / g.shape.chunk;
         for (size_t k = 0; k < g.members.size(); ++k) {
             fgpe_t* h = b->inst[g.members[k]];
             InstDesc& d = g.h_desc[k];

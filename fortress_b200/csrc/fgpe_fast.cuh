@@ -11,7 +11,7 @@
 #pragma once
 #include "fgpe_device.cuh"
 #include "fgpe_async.cuh"
-#include "fgpe_kernels.h"
+#include "fgpe_kernels.cuh"
 
 namespace fgpe {
 
@@ -165,14 +165,34 @@ constexpr int row_minb(int th) { return FGPE_ROW_MINB ? FGPE_ROW_MINB : (th <= 1
 #ifndef FGPE_ROW_NBUF
 #define FGPE_ROW_NBUF 2
 #endif
-#ifndef FGPE_COL_MINB
-#define FGPE_COL_MINB 2
-#endif
 #ifndef FGPE_TW_SMEM
 #define FGPE_TW_SMEM 0
 #endif
 
 // ------------------------------------------------------------ row kernel
+// Rows per row-kernel tile (FGPE_ROW_R256 fixes it for 256-point rows at
+// build time).
+#ifndef FGPE_ROW_R256
+#define FGPE_ROW_R256 0
+#endif
+constexpr int row_r(int n) { return n >= 384 ? 1 : (n == 256 && FGPE_ROW_R256 ? FGPE_ROW_R256 : 512 / n); }
+constexpr int fast_threads(int tot) {
+    const int iter = (tot + 511) / 512;
+    const int per = (tot + iter - 1) / iter;
+    return (per + 31) / 32 * 32;
+}
+// Threads of the block row pass: one radix-8 butterfly per thread and pass
+// unless FGPE_ROW_TH fixes them at build time.
+#ifndef FGPE_ROW_TH
+#define FGPE_ROW_TH 0
+#endif
+template <typename T, int MS, int N> constexpr int row_th() {
+    return FGPE_ROW_TH ? FGPE_ROW_TH : fast_threads(MS * row_r(N) * N / 8);
+}
+template <typename T, int MS, int N> constexpr size_t row_smem() {
+    return ((size_t)FGPE_ROW_NBUF * MS * row_r(N) * cpad(N) + (FGPE_TW_SMEM ? N : 0)) * sizeof(cx<T>);
+}
+
 // Tiles of R x-lines (all MS components); see k_row for the three modes.
 template <typename T, int MS, int N, int R, int TH, int NBUF = FGPE_ROW_NBUF>
 __global__ void __launch_bounds__(TH, row_minb(TH)) k_row_fast(StepConst c, RowArgs a) {

@@ -4,13 +4,13 @@
 //
 // A group's instances differ in their physics (TAU, GAMMA, ALPHA, DT) and
 // state buffers, described per instance by an InstDesc in device memory.  A
-// launch walks the tiles of all of them: column tiles are independent; row
-// tiles are taken in chunks of consecutive tiles of one instance, each chunk
-// adds its NORMC partial to the instance's slot for that chunk, and the
-// block that completes an instance's last chunk reduces the slots in a
-// fixed order and publishes the norms and next scales (as the last block of
-// the single-instance row pass does), so results do not depend on timing.
-// The per-tile arithmetic is that of k_row_fast / k_col_fast.
+// launch walks the tiles of all of them: column tiles are independent
+// (k_regcol_group); rows are taken in chunks of consecutive tiles (the block
+// pass below) or batches (k_regrow_group) of one instance, each chunk adds
+// its NORMC partial to the instance's slot for that chunk, and whoever
+// completes an instance's last chunk reduces the slots in a fixed order and
+// publishes the norms and next scales (as the last block of the
+// single-instance row pass does), so results do not depend on timing.
 #pragma once
 #include "fgpe_fast.cuh"
 
@@ -80,6 +80,55 @@ __device__ void finish_group_norms(const InstDesc& D, const StepConst& c, int nc
         *D.counter = 0u;
     }
     __syncthreads();
+}
+
+// The same by one warp, whose NORMC terms (one value per lane and component)
+// are those of the instance's chunk `slot`; acc starts again from zero.
+template <int MS>
+__device__ __forceinline__ void warp_finish_norms(const InstDesc& D, int slot, int nslots, bool keep_prev, double (&acc)[MS]) {
+    const int lane = threadIdx.x & 31;
+    auto warp_sum = [&](double (&v)[MS]) {
+#pragma unroll
+        for (int m = 0; m < MS; ++m)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[m] += __shfl_xor_sync(0xffffffffu, v[m], o);
+    };
+    warp_sum(acc);
+    int last = 0;
+    if (lane == 0) {
+#pragma unroll
+        for (int m = 0; m < MS; ++m) D.part[(size_t)slot * MS + m] = acc[m];
+        __threadfence();
+        last = atomicAdd(D.counter, 1u) == (unsigned)nslots - 1u;
+    }
+#pragma unroll
+    for (int m = 0; m < MS; ++m) acc[m] = 0.0;
+    last = __shfl_sync(0xffffffffu, last, 0);
+    if (!last) return;
+    __threadfence();
+    for (int b = lane; b < nslots; b += 32) {
+#pragma unroll
+        for (int m = 0; m < MS; ++m) acc[m] += __ldcg(D.part + (size_t)b * MS + m);
+    }
+    warp_sum(acc);
+    if (lane == 0) {
+        double tot = 0, n[MS], sc[MS];
+        double* info = D.info;
+        for (int m = 0; m < MS; ++m) { n[m] = acc[m]; tot += n[m]; info[INFO_NORM + m] = n[m]; }
+        info[INFO_TOTAL] = tot;
+        sink_norms<MS>(D.c, n);
+        const int rc = compute_scales<MS>(D.c, n, info + INFO_SIG, sc);
+        bool bad = !(tot == tot) || !(tot < 1e300);
+        for (int m = 0; m < MS; ++m) { info[INFO_SC + m] = sc[m]; bad = bad || !(sc[m] == sc[m]); }
+        if (bad) info[INFO_ERR] = 1.0;
+        if (rc) info[INFO_ERR] = (double)rc;
+        if (keep_prev)
+            for (int i = 0; i < INFO_LEN; ++i) D.info_prev[i] = info[i];
+        *D.counter = 0u;
+    }
+#pragma unroll
+    for (int m = 0; m < MS; ++m) acc[m] = 0.0;
+    __syncwarp();
 }
 
 // ------------------------------------------------------------ row pass
@@ -193,69 +242,6 @@ __global__ void __launch_bounds__(TH, row_minb(TH)) k_row_group(GroupArgs g) {
         inst = ninst; lt = nlt; have = nxt;
     }
     cp_wait<0>();
-}
-
-// --------------------------------------------------------- column pass
-// The 2D column pass (F_y, scale + KE + SOC, F_y^-1) of every instance:
-// tiles of TX adjacent x positions, full y lines.
-template <typename T, int MS, int N, int TX, int TH>
-__global__ void __launch_bounds__(TH, FGPE_COL_MINB) k_col_group(GroupArgs g) {
-    using CT = ColTile<N, TX>;
-    constexpr int LPN = CT::LPN;
-    constexpr int EPC = 16 / (int)sizeof(cx<T>);
-    static_assert(TX % EPC == 0, "column tile narrower than a 16-byte chunk");
-    constexpr int CPL = TX / EPC;
-    constexpr int NCH = MS * N * CPL;
-    extern __shared__ __align__(16) unsigned char smraw[];
-    cx<T>* cur = (cx<T>*)smraw;
-    __shared__ StepConst c;
-    const int ntiles = g.ninst * g.tiles;
-    int cur_inst = -1;
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int inst = t / g.tiles;
-        const int x0 = (t - inst * g.tiles) * TX;
-        const InstDesc& D = g.d[inst];
-        if (inst != cur_inst) {
-            load_const(c, D.c);
-            cur_inst = inst;
-        }
-        const long long np = D.c.npts;
-        const long long stride = D.c.nx;
-        cx<T>* S = (cx<T>*)D.S;
-        for (int ch = threadIdx.x; ch < NCH; ch += TH) {
-            const int tc = (ch % CPL) * EPC;
-            const int q = ch / CPL;
-            const int e = q % N, m = q / N;
-            cp16(cur + (m * LPN + e + (e >> 3)) * TX + tc, S + (size_t)m * np + x0 + (size_t)e * stride + tc);
-        }
-        cp_commit();
-        cp_wait<0>();
-        __syncthreads();
-        const double cfac = 1.0 / (double)c.npts;
-        T fac[MS];
-#pragma unroll
-        for (int m = 0; m < MS; ++m) fac[m] = (T)(D.info[INFO_SC + m] * cfac);
-        const cx<T>* tw = (const cx<T>*)c.twy;
-        ct_fft<T, false, N, MS * TX, TH, CT>(cur, tw);
-        for (int p = threadIdx.x; p < N * TX; p += TH) {
-            const int tt = p % TX, e = p / TX;
-            const int ix = c.fx[x0 + tt], iy = c.fy[e];
-            cx<T> v[MS];
-#pragma unroll
-            for (int m = 0; m < MS; ++m) v[m] = cscale(cur[(m * LPN + e + (e >> 3)) * TX + tt], fac[m]);
-            apply_ke<T, MS>(c, ix, iy, 0, v);
-            if (c.soc) soc_apply<T, MS>(c.imag, ((const Soc4<T>*)c.soc)[(size_t)iy * c.nx + x0 + tt], v);
-#pragma unroll
-            for (int m = 0; m < MS; ++m) cur[(m * LPN + e + (e >> 3)) * TX + tt] = v[m];
-        }
-        __syncthreads();
-        ct_fft<T, true, N, MS * TX, TH, CT>(cur, tw);
-        for (int idx = threadIdx.x; idx < MS * N * TX; idx += TH) {
-            const int tt = idx % TX, q = idx / TX, e = q % N, m = q / N;
-            S[(size_t)m * np + x0 + (size_t)e * stride + tt] = cur[(m * LPN + e + (e >> 3)) * TX + tt];
-        }
-        __syncthreads();
-    }
 }
 
 }  // namespace fgpe

@@ -21,6 +21,7 @@
 #pragma once
 #include "fgpe_async.cuh"
 #include "fgpe_dft.cuh"
+#include "fgpe_group.cuh"
 #include "fgpe_kernels.h"
 
 namespace fgpe {
@@ -54,10 +55,53 @@ template <typename T, int MS, int N, int TX, class PL, int KIND> constexpr size_
 
 template <typename T> __device__ __forceinline__ cx<T> ld_stream(const cx<T>* p) { return __ldcg(p); }
 
-template <typename T, int MS, int N, int TX, int TH, int MINB, class PL, int KIND>
-__global__ void __launch_bounds__(TH, MINB) k_regcol(StepConst c, ColArgs a) {
+// Where the tiles of a pass come from.  OneGrid: the x tiles of one handle's
+// lines, the components one after the other in single-component passes.
+template <typename T, int MS, int TX, int KIND> struct OneGrid {
+    static constexpr bool many = false, KOP = KIND >= COLK_Y2D;
+    const StepConst& k;
+    const ColArgs& a;
+    int nxt, per;
+    __device__ __forceinline__ OneGrid(const StepConst& c, const ColArgs& args) : k(c), a(args) {
+        nxt = (c.nx + TX - 1) / TX;
+        per = nxt * a.n_other;
+    }
+    __device__ __forceinline__ int tiles() const { return KOP ? per : per * MS; }
+    __device__ __forceinline__ const StepConst& c(int) const { return k; }
+    __device__ __forceinline__ const void* tw() const { return a.tw; }
+    __device__ __forceinline__ long long stride() const { return a.axis_stride; }
+    __device__ __forceinline__ int comp(int tile) const { return KOP ? 0 : tile / per; }
+    __device__ __forceinline__ int other(int tile) const { return (KOP ? tile : tile % per) / nxt; }
+    __device__ __forceinline__ int x0(int tile) const { return (KOP ? tile : tile % per) % nxt * TX; }
+    __device__ __forceinline__ int ky(int tile) const { return a.fother[other(tile)]; }
+    __device__ __forceinline__ cx<T>* S(int tile) const {
+        return (cx<T>*)a.S + (size_t)comp(tile) * k.npts + (long long)other(tile) * a.other_stride + x0(tile);
+    }
+    __device__ __forceinline__ T scale(int, int m) const { return (T)(a.info[INFO_SC + m] * a.cfac); }
+};
+// ManyGrids: the x tiles of every instance of a group of q2D instances of one
+// shape (fgpe_group.cuh), one instance after the other.
+template <typename T, int TX> struct ManyGrids {
+    static constexpr bool many = true;
+    const InstDesc* d;
+    int ninst, per, nx;
+    __device__ __forceinline__ ManyGrids(const GroupArgs& g) : d(g.d), ninst(g.ninst), per(g.tiles), nx(g.d[0].c.nx) {}
+    __device__ __forceinline__ int tiles() const { return ninst * per; }
+    __device__ __forceinline__ const StepConst& c(int tile) const { return d[tile / per].c; }
+    __device__ __forceinline__ const void* tw() const { return d[0].c.twy; }     // one line length: one table
+    __device__ __forceinline__ long long stride() const { return nx; }
+    __device__ __forceinline__ int comp(int) const { return 0; }
+    __device__ __forceinline__ int x0(int tile) const { return tile % per * TX; }
+    __device__ __forceinline__ int ky(int) const { return 0; }
+    __device__ __forceinline__ cx<T>* S(int tile) const { return (cx<T>*)d[tile / per].S + x0(tile); }
+    __device__ __forceinline__ T scale(int tile, int m) const {
+        return (T)(d[tile / per].info[INFO_SC + m] * (1.0 / (double)d[0].c.npts));
+    }
+};
+
+template <typename T, int MS, int N, int TX, int TH, class PL, int KIND, class Src>
+__device__ __forceinline__ void regcol_tiles(const Src& src) {
     static_assert(PL::N == N, "plan length");
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
     constexpr bool KOP = KIND >= COLK_Y2D;
     constexpr int R0 = PL::R0, RL = PL::RL, S0 = N / R0, NQ = N / RL;
     using TL = RegTile<T, TX, RL>;
@@ -70,17 +114,16 @@ __global__ void __launch_bounds__(TH, MINB) k_regcol(StepConst c, ColArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T>* sm = (cx<T>*)smraw;
     cx<T>* kez = sm + MS * LINE;                     // z pass: exp(-i CDT (kz^2 - 2 L GAMMAZ kz)) per component
-    const long long np = c.npts;
-    const int nxt = (c.nx + TX - 1) / TX;
-    const cx<T>* tw = (const cx<T>*)a.tw;
-    const long long st = a.axis_stride;
-    const int ncomp = KOP ? 1 : MS;
-    const int per = nxt * a.n_other;
-    const int ntiles = per * ncomp;
+    const StepConst& c0 = src.c(0);
+    const long long np = c0.npts;
+    const int nx = c0.nx;
+    const cx<T>* tw = (const cx<T>*)src.tw();
+    const long long st = src.stride();
+    const int ntiles = src.tiles();
+    constexpr bool SCALED = KIND == COLK_FWD || KIND == COLK_Y2D;
     T fac[MS];
 #pragma unroll
-    for (int m = 0; m < MS; ++m)
-        fac[m] = (KIND == COLK_FWD || KIND == COLK_Y2D) ? (T)(a.info[INFO_SC + m] * a.cfac) : (T)1;
+    for (int m = 0; m < MS; ++m) fac[m] = SCALED && !Src::many ? src.scale(0, m) : (T)1;
 
     // where a thread's butterfly is the same in every tile, its twiddles stay
     // in registers
@@ -88,16 +131,15 @@ __global__ void __launch_bounds__(TH, MINB) k_regcol(StepConst c, ColArgs a) {
     Twiddles<T, R0> wq;
     if constexpr (KEEPW) wq.load(tw, (threadIdx.x / TX) % S0, 1);
     if constexpr (KIND == COLK_Z3D) {
-        for (int i = threadIdx.x; i < MS * N; i += TH) kez[i] = ((const cx<T>*)c.kez)[i];
+        for (int i = threadIdx.x; i < MS * N; i += TH) kez[i] = ((const cx<T>*)c0.kez)[i];
     }
     // passes with the operators: a butterfly's slots of the first forward and
     // of the last inverse pass belong to one thread, which refills them with
     // the next tile's elements as soon as it has read the last pass's, so the
     // copies overlap that pass's arithmetic and stores
     auto fetch = [&](int tile, int m, int q, int t) {
-        const int oth = tile / nxt, x0 = (tile - oth * nxt) * TX;
-        if (t > c.nx - 1 - x0) return;
-        const cx<T>* g = (const cx<T>*)a.S + (size_t)m * np + (long long)oth * a.other_stride + x0 + t + (long long)q * st;
+        if (t > nx - 1 - src.x0(tile)) return;
+        const cx<T>* g = src.S(tile) + (size_t)m * np + t + (long long)q * st;
 #pragma unroll
         for (int r = 0; r < R0; ++r) cp_elem<T>(sm + m * LINE + TL::at(q + r * S0, t), g + (long long)(r * S0) * st);
     };
@@ -109,26 +151,33 @@ __global__ void __launch_bounds__(TH, MINB) k_regcol(StepConst c, ColArgs a) {
         cp_commit();
     }
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int comp = KOP ? 0 : tile / per;
-        const int rest = KOP ? tile : tile - comp * per;
-        const int oth = rest / nxt, x0 = (rest - oth * nxt) * TX;
-        cx<T>* S = (cx<T>*)a.S + (size_t)comp * np + (long long)oth * a.other_stride + x0;
-        const int last = c.nx - 1 - x0;            // tile columns past it are absent (nx not a multiple of TX)
+        const StepConst& c = src.c(tile);
+        const int imag = c.imag;
+        const int x0 = src.x0(tile);
+        cx<T>* S = src.S(tile);
+        const int last = nx - 1 - x0;              // tile columns past it are absent (nx not a multiple of TX)
+        if constexpr (SCALED && Src::many) {
+#pragma unroll
+            for (int m = 0; m < MS; ++m) fac[m] = src.scale(tile, m);
+        }
         T fc = (T)1;
         if constexpr (KIND == COLK_FWD) {
 #pragma unroll
-            for (int m = 0; m < MS; ++m) fc = comp == m ? fac[m] : fc;
+            for (int m = 0; m < MS; ++m) fc = src.comp(tile) == m ? fac[m] : fc;
         }
-        // z lines: (kx, ky) is fixed along a line, so its SO-coupling numbers and
-        // its part of KE come once per tile, ahead of their use (TH is a
-        // multiple of TX, so a thread keeps its line)
+        // a thread keeps its line (TH is a multiple of TX), so the line's kx part
+        // of KE, and on z lines, where (kx, ky) is fixed, its ky part and its
+        // SO-coupling numbers come once per tile, ahead of their use
         static_assert(TH % TX == 0, "threads per tile row");
+        const int xt = x0 + min((int)threadIdx.x % TX, last);
+        const Soc4<T>* soc = (const Soc4<T>*)c.soc;
         cx<T> ke;
         Soc4<T> so;
+        if constexpr (KOP) ke = ((const cx<T>*)c.kex)[c.fx[xt]];
         if constexpr (KIND == COLK_Z3D) {
-            const int x = x0 + min((int)threadIdx.x % TX, last), ix = c.fx[x], iy = a.fother[oth];
-            ke = fmul(c.imag, ((const cx<T>*)c.kex)[ix], ((const cx<T>*)c.key)[iy]);
-            if (c.soc) so = ((const Soc4<T>*)c.soc)[(size_t)iy * c.nx + x];
+            const int iy = src.ky(tile);
+            ke = fmul(imag, ke, ((const cx<T>*)c.key)[iy]);
+            if (soc) so = soc[(size_t)iy * nx + xt];
         }
         if constexpr (KIND != COLK_INV) {
             // first forward pass; without the operators from global memory
@@ -199,22 +248,21 @@ __global__ void __launch_bounds__(TH, MINB) k_regcol(StepConst c, ColArgs a) {
                     for (int r = 0; r < RL; ++r) {
                         cx<T> u[MS];
 #pragma unroll
-                        for (int m = 0; m < MS; ++m) u[m] = fmul(c.imag, fmul(c.imag, ke, kez[m * N + kq + r * NQ]), v[m][r]);
-                        if (c.soc) soc_apply<T, MS>(c.imag, so, u);
+                        for (int m = 0; m < MS; ++m) u[m] = fmul(imag, fmul(imag, ke, kez[m * N + kq + r * NQ]), v[m][r]);
+                        if (soc) soc_apply<T, MS>(imag, so, u);
 #pragma unroll
                         for (int m = 0; m < MS; ++m) v[m][r] = u[m];
                     }
                 } else {
-                    const int ix = c.fx[x0 + min(t, last)];
-                    const Soc4<T>* soc = (const Soc4<T>*)c.soc + x0 + min(t, last);
+                    const cx<T>* key = (const cx<T>*)c.key;
 #pragma unroll
                     for (int r = 0; r < RL; ++r) {
                         const int iy = kq + r * NQ;
+                        const cx<T> f = fmul(imag, ke, key[iy]);
                         cx<T> u[MS];
 #pragma unroll
-                        for (int m = 0; m < MS; ++m) u[m] = cscale(v[m][r], fac[m]);
-                        apply_ke<T, MS>(c, ix, iy, 0, u);
-                        if (c.soc) soc_apply<T, MS>(c.imag, soc[(size_t)iy * c.nx], u);
+                        for (int m = 0; m < MS; ++m) u[m] = fmul(imag, f, cscale(v[m][r], fac[m]));
+                        if (soc) soc_apply<T, MS>(imag, soc[(size_t)iy * nx + xt], u);
 #pragma unroll
                         for (int m = 0; m < MS; ++m) v[m][r] = u[m];
                     }
@@ -310,7 +358,21 @@ __global__ void __launch_bounds__(TH, MINB) k_regcol(StepConst c, ColArgs a) {
             else __syncthreads();
         }
     }
+}
+
+template <typename T, int MS, int N, int TX, int TH, int MINB, class PL, int KIND>
+__global__ void __launch_bounds__(TH, MINB) k_regcol(const __grid_constant__ StepConst c, const __grid_constant__ ColArgs a) {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    const OneGrid<T, MS, TX, KIND> src(c, a);
+    regcol_tiles<T, MS, N, TX, TH, PL, KIND>(src);
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+
+// The q2D pass of every instance of a group.
+template <typename T, int MS, int N, int TX, int TH, int MINB, class PL>
+__global__ void __launch_bounds__(TH, MINB) k_regcol_group(const __grid_constant__ GroupArgs g) {
+    const ManyGrids<T, TX> src(g);
+    regcol_tiles<T, MS, N, TX, TH, PL, COLK_Y2D>(src);
 }
 
 // ------------------------------------------------------- launch shapes

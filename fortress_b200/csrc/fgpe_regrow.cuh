@@ -22,6 +22,7 @@
 #pragma once
 #include "fgpe_async.cuh"
 #include "fgpe_dft.cuh"
+#include "fgpe_group.cuh"
 #include "fgpe_kernels.cuh"
 
 namespace fgpe {
@@ -97,9 +98,51 @@ template <int M> __device__ __forceinline__ void st_points(const float2 (&v)[M],
     for (int i = 0; i < M; i += 2) *(float4*)(s + i) = make_float4(v[i].x, v[i].y, v[i + 1].x, v[i + 1].y);
 }
 
-template <typename T, int MS, int N, int RW, int WPB, int MINB>
-__global__ void __launch_bounds__(WPB * 32, MINB) k_regrow(StepConst c, RowArgs a) {
-    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+// Where a pass's rows come from: batches of RW rows.  OneSpinor: the rows of
+// one handle; its NORMC terms are summed over the grid at the end.
+template <typename T> struct OneSpinor {
+    static constexpr bool many = false;
+    const StepConst& k;
+    const RowArgs& a;
+    int nrows;
+    __device__ __forceinline__ OneSpinor(const StepConst& c, const RowArgs& args) : k(c), a(args), nrows(c.ny * c.nz) {}
+    __device__ __forceinline__ int batches(int rw) const { return (nrows + rw - 1) / rw; }
+    __device__ __forceinline__ int next(int batch, int nw) const { return batch + nw; }
+    __device__ __forceinline__ int first(int warp) const { return warp; }
+    __device__ __forceinline__ const StepConst& c(int) const { return k; }
+    __device__ __forceinline__ cx<T>* S(int) const { return (cx<T>*)a.S; }
+    __device__ __forceinline__ cx<T>* snap(int) const { return (cx<T>*)a.snap; }
+    __device__ __forceinline__ int row0(int batch, int rw) const { return batch * rw; }
+};
+// ManySpinors: the rows of every instance of a group, in chunks of
+// consecutive batches of one instance; the warp that ends a chunk leaves its
+// NORMC terms in the instance's slot for it.
+template <typename T> struct ManySpinors {
+    static constexpr bool many = true;
+    const GroupArgs& g;
+    int nrows, per;             // rows and batches of an instance
+    __device__ __forceinline__ ManySpinors(const GroupArgs& a) : g(a), nrows(a.d[0].c.ny), per(a.tiles) {}
+    __device__ __forceinline__ int batches(int) const { return g.ninst * per; }
+    __device__ __forceinline__ int next(int batch, int nw) const {
+        return (batch + 1) % g.chunk ? batch + 1 : batch + 1 + (nw - 1) * g.chunk;
+    }
+    __device__ __forceinline__ int first(int warp) const { return warp * g.chunk; }
+    __device__ __forceinline__ const InstDesc& inst(int batch) const { return g.d[batch / per]; }
+    __device__ __forceinline__ const StepConst& c(int batch) const { return inst(batch).c; }
+    __device__ __forceinline__ cx<T>* S(int batch) const { return (cx<T>*)inst(batch).S; }
+    __device__ __forceinline__ cx<T>* snap(int batch) const {
+        return g.snap == 1 ? (cx<T>*)inst(batch).psi : g.snap == 2 ? (cx<T>*)inst(batch).prev : nullptr;
+    }
+    __device__ __forceinline__ int row0(int batch, int rw) const { return batch % per * rw; }
+    // the chunk that ends with this batch is done
+    template <int MS> __device__ __forceinline__ void flush(int batch, double (&acc)[MS]) const {
+        if ((batch + 1) % g.chunk) return;
+        warp_finish_norms<MS>(inst(batch), batch % per / g.chunk, per / g.chunk, g.snap == 2, acc);
+    }
+};
+
+template <typename T, int MS, int N, int RW, int WPB, class Src>
+__device__ __forceinline__ void regrow_rows(const Src& src, double (&acc)[MS]) {
     constexpr int M = RegRow<T, N>::M, SL = RegRow<T, N>::SL;
     using L = RegRow<T, N>;
     constexpr int NSUB = RW * MS * 8, NPT = RW * M;   // block transforms, radix-8 butterflies (of MS components)
@@ -108,25 +151,21 @@ __global__ void __launch_bounds__(WPB * 32, MINB) k_regrow(StepConst c, RowArgs 
     extern __shared__ __align__(16) unsigned char smraw[];
     const int warp = (int)(threadIdx.x >> 5), lane = (int)(threadIdx.x & 31);
     cx<T>* s = (cx<T>*)smraw + (size_t)warp * RW * MS * 8 * SL;
-    __shared__ double red[32 * (MS + 1)];
-    __shared__ double bsum[MS];
-    const long long np = c.npts;
-    const int nrows = c.ny * c.nz, nw = (int)gridDim.x * WPB;
-    const int nb = (nrows + RW - 1) / RW;
-    const cx<T>* tw = (const cx<T>*)c.twx;
-    cx<T>* S = (cx<T>*)a.S;
-    cx<T>* snap = (cx<T>*)a.snap;
+    const StepConst& c0 = src.c(0);
+    const long long np = c0.npts;
+    const int nrows = src.nrows, nw = (int)gridDim.x * WPB, nb = src.batches(RW);
+    const cx<T>* tw = (const cx<T>*)c0.twx;
 
-    // rows batch * RW ... into this warp's blocks, 16 bytes per copy
+    // a batch's rows into this warp's blocks
     auto fetch = [&](int batch) {
         constexpr int E = L::two ? 1 : 16 / (int)sizeof(cx<T>), PER = N / E;
         static_assert(M % E == 0, "16-byte chunks stay inside a block");
 #pragma unroll
         for (int q = 0; q < RW * MS; ++q) {
             const int rr = q / MS, m = q - rr * MS;
-            const int row = batch * RW + rr;
+            const int row = src.row0(batch, RW) + rr;
             if (RW > 1 && row >= nrows) break;
-            const cx<T>* g = S + (size_t)m * np + (size_t)row * N;
+            const cx<T>* g = src.S(batch) + (size_t)m * np + (size_t)row * N;
 #pragma unroll
             for (int i = 0; i < (PER + 31) / 32; ++i) {
                 const int x = (lane + 32 * i) * E;
@@ -138,18 +177,21 @@ __global__ void __launch_bounds__(WPB * 32, MINB) k_regrow(StepConst c, RowArgs 
             }
         }
     };
-    double acc[MS];
-#pragma unroll
-    for (int m = 0; m < MS; ++m) acc[m] = 0.0;
     // a thread keeps its points from row to row, and their twiddles
     constexpr bool KEEPW = NPT <= 32;
     Twiddles<T, 8> wq;
     if constexpr (KEEPW) wq.load(tw, lane % M, 1);
 
-    int batch = (int)blockIdx.x * WPB + warp;
+    int batch = src.first((int)blockIdx.x * WPB + warp);
     if (batch < nb) fetch(batch);
     cp_commit();
-    for (; batch < nb; batch += nw) {
+    while (batch < nb) {
+        // a group's constants come from memory once per batch, one handle's are
+        // the kernel's parameters
+        std::conditional_t<Src::many, const StepConst, const StepConst&> c = src.c(batch);
+        cx<T>* S = src.S(batch);
+        cx<T>* snap = src.snap(batch);
+        const int row0 = src.row0(batch, RW), nxt = src.next(batch, nw);
         cp_wait<0>();
         __syncwarp();
         if constexpr (!L::two) {
@@ -192,7 +234,7 @@ __global__ void __launch_bounds__(WPB * 32, MINB) k_regrow(StepConst c, RowArgs 
 #pragma unroll 1
         for (int b = lane; b < NPT; b += 32) {
             const int rr = RW == 1 ? 0 : b / M, x0 = RW == 1 ? b : b - rr * M;
-            const int row = batch * RW + rr;
+            const int row = row0 + rr;
             if (RW > 1 && row >= nrows) break;
             cx<T>* d = s + rr * MS * 8 * SL + L::at(x0);
             if constexpr (!KEEPW) wq.load(tw, x0, 1);
@@ -276,13 +318,13 @@ __global__ void __launch_bounds__(WPB * 32, MINB) k_regrow(StepConst c, RowArgs 
                 if (i0 + STEP >= IT) {
                     // every block has been read: the next rows may come in
                     __syncwarp();
-                    if (batch + nw < nb) fetch(batch + nw);
+                    if (nxt < nb) fetch(nxt);
                     cp_commit();
                 }
 #pragma unroll
                 for (int k = 0; k < STEP; ++k) {
                     const int b = lane + (i0 + k) * 32;
-                    const int q = b / 64, rr = q / MS, m = q - rr * MS, row = batch * RW + rr;
+                    const int q = b / 64, rr = q / MS, m = q - rr * MS, row = row0 + rr;
                     Dft<T, false, RB>::run(v[k]);
                     if (RW == 1 || row < nrows) {
                         cx<T>* g = S + (size_t)m * np + (size_t)row * N + (b % 64) * RB;
@@ -310,12 +352,12 @@ __global__ void __launch_bounds__(WPB * 32, MINB) k_regrow(StepConst c, RowArgs 
                 if (b0 + 32 >= NSUB) {
                     // every block has been read: the next rows may come in
                     __syncwarp();
-                    if (batch + nw < nb) fetch(batch + nw);
+                    if (nxt < nb) fetch(nxt);
                     cp_commit();
                 }
                 if (on) {
                     Dft<T, false, M>::run(v);
-                    const int q = b / 8, rr = q / MS, m = q - rr * MS, row = batch * RW + rr;
+                    const int q = b / 8, rr = q / MS, m = q - rr * MS, row = row0 + rr;
                     if (RW == 1 || row < nrows) {
                         cx<T>* g = S + (size_t)m * np + (size_t)row * N + (b % 8) * M;
                         static_for<0, M / V>([&](auto i) {
@@ -328,12 +370,36 @@ __global__ void __launch_bounds__(WPB * 32, MINB) k_regrow(StepConst c, RowArgs 
                 }
             }
         }
+        if constexpr (Src::many) src.template flush<MS>(batch, acc);
+        batch = nxt;
     }
     cp_wait<0>();
+}
+
+template <typename T, int MS, int N, int RW, int WPB, int MINB>
+__global__ void __launch_bounds__(WPB * 32, MINB) k_regrow(const __grid_constant__ StepConst c, const __grid_constant__ RowArgs a) {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    __shared__ double red[32 * (MS + 1)];
+    __shared__ double bsum[MS];
+    double acc[MS];
+#pragma unroll
+    for (int m = 0; m < MS; ++m) acc[m] = 0.0;
+    const OneSpinor<T> src(c, a);
+    regrow_rows<T, MS, N, RW, WPB>(src, acc);
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     block_sum<MS>(acc, red, bsum);
     if (threadIdx.x < MS) a.part[(size_t)blockIdx.x * MS + threadIdx.x] = bsum[threadIdx.x];
     finish_norms<MS>(c, a.part, a.counter, a.info, red);
+}
+
+// The row pass of every instance of a group (g.tiles batches of RW rows each).
+template <typename T, int MS, int N, int RW, int WPB, int MINB>
+__global__ void __launch_bounds__(WPB * 32, MINB) k_regrow_group(const __grid_constant__ GroupArgs g) {
+    double acc[MS];
+#pragma unroll
+    for (int m = 0; m < MS; ++m) acc[m] = 0.0;
+    const ManySpinors<T> src(g);
+    regrow_rows<T, MS, N, RW, WPB>(src, acc);
 }
 
 // ------------------------------------------------------- launch shapes

@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "fgpe_group.cuh"
 #include "fgpe_kernels.h"
 
 namespace fgpe {
@@ -20,11 +21,27 @@ cudaError_t regcol_launch(int n, int kind, int wide, int grid, const StepConst& 
 // pass reads.
 inline int regcol_radices(int n, int* r) { r[0] = n / 16; r[1] = 16; return 2; }
 
+// Row pass over shared tiles of the same lengths, one block per tile of rows or
+// (warp) one warp per row (fgpe_fast.cuh): resident grid for the given number
+// of rows (0: not available).
+template <typename T, int MS> int row_grid(int n, bool warp, int rows);
+template <typename T, int MS>
+cudaError_t row_launch(int n, bool warp, int grid, const StepConst& c, const RowArgs& a, cudaStream_t st, bool pdl);
+
 // Row pass of spin-1 lines of the same lengths (fgpe_regrow.cuh): resident
 // grid for the given number of rows (0: not available).
 template <typename T> int regrow_grid(int n, int rows);
 template <typename T>
 cudaError_t regrow_launch(int n, int grid, const StepConst& c, const RowArgs& a, cudaStream_t st, bool pdl);
+
+// Grouped passes of q2D instances of one nx x ny shape (fgpe_group.cuh): tiles
+// per instance, row tiles or batches per chunk, resident grids.
+struct GroupShape { int col_tiles = 0, col_grid = 0, row_tiles = 0, chunk = 1, row_grid = 0; };
+template <typename T, int MS> bool group_shape(int nx, int ny, int members, GroupShape* g);
+// One whole step of every instance: the column pass, then the row pass
+// (snap: see GroupArgs).
+template <typename T, int MS>
+cudaError_t group_launch(int nx, int ny, const GroupShape& g, const InstDesc* d, int members, int snap, cudaStream_t st);
 
 // Launch as a programmatic dependent (pdl): the pass is launched while the
 // previous one drains and waits on griddepcontrol.wait before it touches the
@@ -60,7 +77,13 @@ template <class K> inline int resident_grid(K kern, int th, size_t smem, long lo
 #define FGPE_STEP_EXTERN(T, MS)                                                                              \
     extern template int regcol_grid<T, MS>(int, int, int, int, int*);                                        \
     extern template cudaError_t regcol_launch<T, MS>(int, int, int, int, const StepConst&, const ColArgs&,   \
-                                                     cudaStream_t, bool);
+                                                     cudaStream_t, bool);                                    \
+    extern template int row_grid<T, MS>(int, bool, int);                                                     \
+    extern template cudaError_t row_launch<T, MS>(int, bool, int, const StepConst&, const RowArgs&,          \
+                                                  cudaStream_t, bool);                                       \
+    extern template bool group_shape<T, MS>(int, int, int, GroupShape*);                                     \
+    extern template cudaError_t group_launch<T, MS>(int, int, const GroupShape&, const InstDesc*, int, int,  \
+                                                    cudaStream_t);
 #define FGPE_STEP_ROW_EXTERN(T)                                                                              \
     extern template int regrow_grid<T>(int, int);                                                            \
     extern template cudaError_t regrow_launch<T>(int, int, const StepConst&, const RowArgs&, cudaStream_t, bool);

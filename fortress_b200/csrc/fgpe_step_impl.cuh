@@ -1,6 +1,7 @@
 // fgpe_step_impl.cuh -- definitions of the pass launchers of fgpe_step.h,
 // included by one translation unit per (precision, spin).
 #pragma once
+#include "fgpe_fast.cuh"
 #include "fgpe_regcol.cuh"
 #include "fgpe_regrow.cuh"
 #include "fgpe_step.h"
@@ -69,6 +70,55 @@ cudaError_t regcol_launch(int n, int kind, int wide, int grid, const StepConst& 
     }
 }
 
+// Warp-row kernel: rows of MS lines up to 16 KB (FP64 spin-1 to 256 points,
+// spin-2 to 128; FP32 spin-1 to 512, spin-2 to 256); warps per block so that
+// two blocks of NBUF rows per warp fit the shared memory.
+template <typename T, int MS, int N> constexpr size_t wrow_tile() { return (size_t)MS * cpad(N) * sizeof(cx<T>); }
+template <typename T, int MS, int N> constexpr bool wrow_ok() { return wrow_tile<T, MS, N>() <= 16 * 1024; }
+template <typename T, int MS, int N> constexpr int wrow_wpb() {
+    const int w = (int)((110 * 1024) / (wrow_tile<T, MS, N>() * FGPE_WROW_NBUF));
+    return w < 1 ? 1 : (w > 8 ? 8 : w);
+}
+
+template <typename T, int MS> int row_grid(int n, bool warp, int rows) {
+    switch (n) {
+#define G(NN)                                                                                                       \
+    case NN: {                                                                                                      \
+        constexpr int R = row_r(NN), TH = row_th<T, MS, NN>();                                                      \
+        if (!warp) return rows % R ? 0 : resident_grid(k_row_fast<T, MS, NN, R, TH>, TH, row_smem<T, MS, NN>(), rows / R); \
+        if constexpr (wrow_ok<T, MS, NN>()) {                                                                       \
+            constexpr int W = wrow_wpb<T, MS, NN>();                                                                \
+            return resident_grid(k_row_warp<T, MS, NN, W, FGPE_WROW_NBUF>, W * 32,                                  \
+                                 (size_t)W * FGPE_WROW_NBUF * wrow_tile<T, MS, NN>(), (rows + W - 1) / W);          \
+        }                                                                                                           \
+        return 0;                                                                                                   \
+    }
+        FGPE_STEP_SIZES(G)
+#undef G
+        default: return 0;
+    }
+}
+
+template <typename T, int MS>
+cudaError_t row_launch(int n, bool warp, int grid, const StepConst& c, const RowArgs& a, cudaStream_t st, bool pdl) {
+    switch (n) {
+#define L(NN)                                                                                                       \
+    case NN: {                                                                                                      \
+        constexpr int R = row_r(NN), TH = row_th<T, MS, NN>();                                                      \
+        if (!warp) return launch_step_kernel(k_row_fast<T, MS, NN, R, TH>, grid, TH, row_smem<T, MS, NN>(), c, a, st, pdl); \
+        if constexpr (wrow_ok<T, MS, NN>()) {                                                                       \
+            constexpr int W = wrow_wpb<T, MS, NN>();                                                                \
+            return launch_step_kernel(k_row_warp<T, MS, NN, W, FGPE_WROW_NBUF>, grid, W * 32,                       \
+                                      (size_t)W * FGPE_WROW_NBUF * wrow_tile<T, MS, NN>(), c, a, st, pdl);          \
+        }                                                                                                           \
+        return cudaErrorInvalidValue;                                                                               \
+    }
+        FGPE_STEP_SIZES(L)
+#undef L
+        default: return cudaErrorInvalidValue;
+    }
+}
+
 template <typename T> int regrow_grid(int n, int rows) {
     switch (n) {
 #define G(NN)                                                                                                       \
@@ -103,6 +153,95 @@ cudaError_t regrow_launch(int n, int grid, const StepConst& c, const RowArgs& a,
     }
 }
 
+// ---------------------------------------------------------- grouped passes
+// Column tiles take the big z pass's plan and shape: with many instances there
+// is a tile for every resident block, and wide rows of x keep whole sectors.
+template <typename T, int MS, int N> struct GroupCol {
+    using B = ColShape<T, MS, N, COLK_Z3D, true>;
+    using P = typename B::P;
+    static constexpr int TX = B::TX, TH = B::TH;
+    static constexpr size_t SMEM = regcol_smem<T, MS, N, TX, P, COLK_Y2D>();
+    static constexpr auto kernel() { return k_regcol_group<T, MS, N, TX, TH, B::MINB, P>; }
+};
+// Rows: k_regrow_group where k_regrow is available, else the block pass.
+template <typename T, int MS, int N> struct GroupRow {
+    using H = RowShape<T, N>;
+    static constexpr bool reg = MS == 3 && H::RW > 0;
+    static constexpr int R = row_r(N), TH = row_th<T, MS, N>();
+};
+constexpr int most_dividing(int tiles, int most) {
+    int c = 1;
+    for (int d = 1; d <= most; ++d) if (tiles % d == 0) c = d;
+    return c;
+}
+
+template <typename T, int MS> bool group_shape(int nx, int ny, int members, GroupShape* g) {
+    g->col_grid = g->row_grid = 0;
+    switch (ny) {
+#define C(NN)                                                                                                     \
+    case NN: {                                                                                                    \
+        using G = GroupCol<T, MS, NN>;                                                                            \
+        g->col_tiles = (nx + G::TX - 1) / G::TX;                                                                  \
+        g->col_grid = resident_grid(G::kernel(), G::TH, G::SMEM, (long long)members * g->col_tiles);              \
+    } break;
+        FGPE_STEP_SIZES(C)
+#undef C
+    }
+    switch (nx) {
+#define R(NN)                                                                                                     \
+    case NN: {                                                                                                    \
+        using G = GroupRow<T, MS, NN>;                                                                            \
+        if constexpr (G::reg) {                                                                                   \
+            using H = typename G::H;                                                                              \
+            g->row_tiles = (ny + H::RW - 1) / H::RW;                                                              \
+            g->chunk = most_dividing(g->row_tiles, 2);                                                            \
+            const long long chunks = (long long)members * (g->row_tiles / g->chunk);                              \
+            g->row_grid = resident_grid(k_regrow_group<T, MS, NN, H::RW, H::WPB, H::MINB>, H::WPB * 32,           \
+                                        H::WPB * regrow_warp_smem<T, MS, NN, H::RW>(), (chunks + H::WPB - 1) / H::WPB); \
+        } else {                                                                                                  \
+            if (ny % G::R) return false;                                                                          \
+            g->row_tiles = ny / G::R;                                                                             \
+            g->chunk = most_dividing(g->row_tiles, 16);                                                           \
+            g->row_grid = resident_grid(k_row_group<T, MS, NN, G::R, G::TH>, G::TH, row_smem<T, MS, NN>(),        \
+                                        (long long)members * (g->row_tiles / g->chunk));                          \
+        }                                                                                                         \
+    } break;
+        FGPE_STEP_SIZES(R)
+#undef R
+    }
+    return g->col_grid > 0 && g->row_grid > 0;
+}
+
+template <typename T, int MS>
+cudaError_t group_launch(int nx, int ny, const GroupShape& g, const InstDesc* d, int members, int snap, cudaStream_t st) {
+    const GroupArgs ca{d, members, g.col_tiles, 1, 0}, ra{d, members, g.row_tiles, g.chunk, snap};
+    switch (ny) {
+#define C(NN)                                                                                                     \
+    case NN: {                                                                                                    \
+        using G = GroupCol<T, MS, NN>;                                                                            \
+        G::kernel()<<<g.col_grid, G::TH, G::SMEM, st>>>(ca);                                                      \
+    } break;
+        FGPE_STEP_SIZES(C)
+#undef C
+    }
+    switch (nx) {
+#define R(NN)                                                                                                     \
+    case NN: {                                                                                                    \
+        using G = GroupRow<T, MS, NN>;                                                                            \
+        if constexpr (G::reg) {                                                                                   \
+            using H = typename G::H;                                                                              \
+            k_regrow_group<T, MS, NN, H::RW, H::WPB, H::MINB>                                                     \
+                <<<g.row_grid, H::WPB * 32, H::WPB * regrow_warp_smem<T, MS, NN, H::RW>(), st>>>(ra);             \
+        } else {                                                                                                  \
+            k_row_group<T, MS, NN, G::R, G::TH><<<g.row_grid, G::TH, row_smem<T, MS, NN>(), st>>>(ra);            \
+        }                                                                                                         \
+    } break;
+        FGPE_STEP_SIZES(R)
+#undef R
+    }
+    return cudaGetLastError();
+}
+
 #define FGPE_STEP_ROW_INSTANTIATE(T)            \
     template int regrow_grid<T>(int, int);      \
     template cudaError_t regrow_launch<T>(int, int, const StepConst&, const RowArgs&, cudaStream_t, bool);
@@ -110,6 +249,10 @@ cudaError_t regrow_launch(int n, int grid, const StepConst& c, const RowArgs& a,
 #define FGPE_STEP_INSTANTIATE(T, MS)                                                                  \
     template int regcol_grid<T, MS>(int, int, int, int, int*);                                        \
     template cudaError_t regcol_launch<T, MS>(int, int, int, int, const StepConst&, const ColArgs&,   \
-                                              cudaStream_t, bool);
+                                              cudaStream_t, bool);                                    \
+    template int row_grid<T, MS>(int, bool, int);                                                     \
+    template cudaError_t row_launch<T, MS>(int, bool, int, const StepConst&, const RowArgs&, cudaStream_t, bool); \
+    template bool group_shape<T, MS>(int, int, int, GroupShape*);                                     \
+    template cudaError_t group_launch<T, MS>(int, int, const GroupShape&, const InstDesc*, int, int, cudaStream_t);
 
 }  // namespace fgpe
