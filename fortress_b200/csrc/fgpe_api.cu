@@ -114,6 +114,16 @@ int fail(fgpe_t* h, int code, const std::string& m) {
             return fail(h, FGPE_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
+// FastDiv factors of a plan's passes.
+void plan_divisors(FftPlan* pl) {
+    int block = pl->n;
+    for (int p = 0; p < pl->nf; ++p) {
+        block /= pl->r[p];
+        pl->mnb[p] = FastDiv(pl->n / pl->r[p]).m;
+        pl->msi[p] = FastDiv(block).m;
+    }
+}
+
 bool plan_fft(int n, FftPlan* pl) {
     pl->n = n; pl->nf = 0;
     int m = n;
@@ -126,6 +136,7 @@ bool plan_fft(int n, FftPlan* pl) {
     if (m != 1 || f.size() > 16) return false;
     for (size_t i = 0; i < f.size(); ++i) pl->r[i] = f[i];
     pl->nf = (int)f.size();
+    plan_divisors(pl);
     return true;
 }
 

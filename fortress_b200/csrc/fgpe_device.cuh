@@ -87,9 +87,25 @@ template <typename C> __device__ __forceinline__ C fmul(int imag, C a, C b) {
 // reordering pass is ever needed.  Every butterfly reads and writes only its
 // own r slots: a thread holds r values, and passes are separated by one
 // barrier.
+// Division of 0 <= a by a run-time d as the high word of a product, exact for
+// a * d < 2^32 (tile-local indices; both stay below 2^15): the passes of
+// run-time lengths divide several times per butterfly and per element, and a
+// hardware-emulated division costs as much as a radix-4 butterfly (320 x 240
+// spin-1 FP64 step 43 -> 37 us, 2048-point spin-2 line 16.6 -> 13.8 us).
+struct FastDiv {
+    unsigned d, m;      // divisor, ceil(2^32 / d) (0 for d = 1)
+    __host__ __device__ __forceinline__ FastDiv(unsigned dd, unsigned mm) : d(dd), m(mm) {}
+    __host__ __device__ __forceinline__ explicit FastDiv(int dd) : d((unsigned)dd), m(0xffffffffu / (unsigned)dd + 1u) {}
+    __device__ __forceinline__ int div(int a) const { return m ? (int)__umulhi((unsigned)a, m) : a; }
+    __device__ __forceinline__ int mod(int a) const { return a - div(a) * (int)d; }
+    friend __device__ __forceinline__ int operator/(int a, const FastDiv& f) { return f.div(a); }
+    friend __device__ __forceinline__ int operator%(int a, const FastDiv& f) { return f.mod(a); }
+};
+
 struct FftPlan {
     int n, nf;
     int r[16];
+    unsigned mnb[16], msi[16];   // FastDiv factors of pass p: butterflies per line n/r, and their stride
 };
 
 __host__ __device__ __forceinline__ int padded_len(int n) { return n + (n + 7) / 8; }
@@ -100,19 +116,26 @@ __device__ __forceinline__ int pad_idx(int e) { return e + (e >> 3); }
 // conflicts).
 struct RowMap {
     int lp;
-    __device__ __forceinline__ void split(int b, int nb, int& l, int& q) const { l = b / nb; q = b - l * nb; }
-    __device__ __forceinline__ int base(int l) const { return l * lp; }
+    // task b of a pass with nb butterflies per line -> start of its line, butterfly
+    __device__ __forceinline__ void split(int b, const FastDiv& nb, int& base, int& q) const {
+        const int l = b / nb;
+        q = b - l * (int)nb.d;
+        base = l * lp;
+    }
     __device__ __forceinline__ int at(int base, int e) const { return base + pad_idx(e); }
 };
 
 // Column tile [m][e][t], t < tx fastest (consecutive threads walk t first).
 struct ColMap {
-    int tx, lpn;  // tile width, padded line length
-    __device__ __forceinline__ void split(int b, int nb, int& l, int& q) const {
-        const int t = b % tx; const int w = b / tx; q = w % nb; const int m = w / nb; l = m * tx + t;
+    FastDiv tx;    // tile width
+    int lpn;       // padded line length
+    __device__ __forceinline__ void split(int b, const FastDiv& nb, int& base, int& q) const {
+        const int w = b / tx, t = b - w * (int)tx.d;
+        const int m = w / nb;
+        q = w - m * (int)nb.d;
+        base = m * lpn * (int)tx.d + t;
     }
-    __device__ __forceinline__ int base(int l) const { return (l / tx) * lpn * tx + (l % tx); }
-    __device__ __forceinline__ int at(int base, int e) const { return base + pad_idx(e) * tx; }
+    __device__ __forceinline__ int at(int base, int e) const { return base + pad_idx(e) * (int)tx.d; }
 };
 
 template <typename T, bool INV, int R> struct Dft;
@@ -235,17 +258,18 @@ __device__ __forceinline__ void tw_powers(const cx<T>* __restrict__ tw, int j, i
 }
 
 template <typename T, bool INV, int R, class Map>
-__device__ __forceinline__ void fft_pass(cx<T>* s, const Map& mp, int nlines, int n, int Bp,
+__device__ __forceinline__ void fft_pass(cx<T>* s, const Map& mp, int nlines, const FftPlan& pl, int p, int Bp,
                                          const cx<T>* __restrict__ tw) {
-    const int si = Bp / R;
-    const int nb = n / R;
+    const int si = Bp / R;           // R is a constant here
+    const int n = pl.n, nb = n / R;
     const int total = nlines * nb;
-    const int tstep = n / Bp;
+    const FastDiv dnb((unsigned)nb, pl.mnb[p]), dsi((unsigned)si, pl.msi[p]);
+    int tstep = 1;
+    for (int i = 0; i < p; ++i) tstep *= pl.r[i];
     for (int b = threadIdx.x; b < total; b += blockDim.x) {
-        int l, q; mp.split(b, nb, l, q);
-        const int blk = q / si, n2 = q - blk * si;
+        int bs, q; mp.split(b, dnb, bs, q);
+        const int blk = q / dsi, n2 = q - blk * si;
         const int e0 = blk * Bp + n2;
-        const int bs = mp.base(l);
         cx<T> v[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) v[r] = s[mp.at(bs, e0 + r * si)];
@@ -273,14 +297,14 @@ __device__ __forceinline__ void fft_pass(cx<T>* s, const Map& mp, int nlines, in
 }
 
 template <typename T, bool INV, class Map>
-__device__ __forceinline__ void fft_dispatch(int R, cx<T>* s, const Map& mp, int nlines, int n, int Bp,
+__device__ __forceinline__ void fft_dispatch(cx<T>* s, const Map& mp, int nlines, const FftPlan& pl, int p, int Bp,
                                              const cx<T>* __restrict__ tw) {
-    switch (R) {
-        case 8: fft_pass<T, INV, 8>(s, mp, nlines, n, Bp, tw); break;
-        case 4: fft_pass<T, INV, 4>(s, mp, nlines, n, Bp, tw); break;
-        case 2: fft_pass<T, INV, 2>(s, mp, nlines, n, Bp, tw); break;
-        case 3: fft_pass<T, INV, 3>(s, mp, nlines, n, Bp, tw); break;
-        default: fft_pass<T, INV, 5>(s, mp, nlines, n, Bp, tw); break;
+    switch (pl.r[p]) {
+        case 8: fft_pass<T, INV, 8>(s, mp, nlines, pl, p, Bp, tw); break;
+        case 4: fft_pass<T, INV, 4>(s, mp, nlines, pl, p, Bp, tw); break;
+        case 2: fft_pass<T, INV, 2>(s, mp, nlines, pl, p, Bp, tw); break;
+        case 3: fft_pass<T, INV, 3>(s, mp, nlines, pl, p, Bp, tw); break;
+        default: fft_pass<T, INV, 5>(s, mp, nlines, pl, p, Bp, tw); break;
     }
 }
 
@@ -289,11 +313,14 @@ template <typename T, bool INV, class Map>
 __device__ void block_fft(cx<T>* s, const Map& mp, int nlines, const FftPlan& pl, const cx<T>* __restrict__ tw) {
     if (!INV) {
         int Bp = pl.n;
-        for (int p = 0; p < pl.nf; ++p) { fft_dispatch<T, false>(pl.r[p], s, mp, nlines, pl.n, Bp, tw); Bp /= pl.r[p]; }
+        for (int p = 0; p < pl.nf; ++p) {
+            fft_dispatch<T, false>(s, mp, nlines, pl, p, Bp, tw);
+            Bp /= pl.r[p];
+        }
     } else if (pl.nf > 0) {
         int Bp = pl.r[pl.nf - 1];
         for (int p = pl.nf - 1; p >= 0; --p) {
-            fft_dispatch<T, true>(pl.r[p], s, mp, nlines, pl.n, Bp, tw);
+            fft_dispatch<T, true>(s, mp, nlines, pl, p, Bp, tw);
             if (p > 0) Bp *= pl.r[p - 1];
         }
     }

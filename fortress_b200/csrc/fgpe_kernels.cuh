@@ -105,6 +105,7 @@ k_row(StepConst c, RowArgs a) {
     __shared__ double red[32 * (MS + 1)];
     __shared__ double bsum[MS];
     const int nx = c.nx, R = a.rows;
+    const FastDiv dnx(nx), dr(R);
     const int lp = padded_len(nx);
     const RowMap mp{lp};
     const int row0 = blockIdx.x * R;
@@ -113,7 +114,7 @@ k_row(StepConst c, RowArgs a) {
     const int nel = MS * R * nx;
     const cx<T>* src = (a.mode == ROW_FWD) ? (const cx<T>*)a.psi : (const cx<T>*)a.S;
     for (int idx = threadIdx.x; idx < nel; idx += blockDim.x) {
-        const int x = idx % nx, q = idx / nx, r = q % R, m = q / R;
+        const int x = idx % dnx, q = idx / dnx, r = q % dr, m = q / dr;
         sm[(m * R + r) * lp + pad_idx(x)] = src[(size_t)m * np + (size_t)(row0 + r) * nx + x];
     }
     __syncthreads();
@@ -125,7 +126,7 @@ k_row(StepConst c, RowArgs a) {
             const T inv = (T)(1.0 / nx);
             cx<T>* dst = (cx<T>*)a.psi;
             for (int idx = threadIdx.x; idx < nel; idx += blockDim.x) {
-                const int x = idx % nx, q = idx / nx, r = q % R, m = q / R;
+                const int x = idx % dnx, q = idx / dnx, r = q % dr, m = q / dr;
                 dst[(size_t)m * np + (size_t)(row0 + r) * nx + x] = cscale(sm[(m * R + r) * lp + pad_idx(x)], inv);
             }
             return;
@@ -136,7 +137,7 @@ k_row(StepConst c, RowArgs a) {
         for (int m = 0; m < MS; ++m) acc[m] = 0.0;
         cx<T>* snap = (cx<T>*)a.snap;
         for (int p = threadIdx.x; p < R * nx; p += blockDim.x) {
-            const int x = p % nx, r = p / nx;
+            const int x = p % dnx, r = p / dnx;
             const int row = row0 + r;
             const int j = row % c.ny, k = row / c.ny;
             cx<T> v[MS];
@@ -167,7 +168,7 @@ k_row(StepConst c, RowArgs a) {
     }
     cx<T>* dst = (cx<T>*)a.S;
     for (int idx = threadIdx.x; idx < nel; idx += blockDim.x) {
-        const int x = idx % nx, q = idx / nx, r = q % R, m = q / R;
+        const int x = idx % dnx, q = idx / dnx, r = q % dr, m = q / dr;
         dst[(size_t)m * np + (size_t)(row0 + r) * nx + x] = sm[(m * R + r) * lp + pad_idx(x)];
     }
 }
@@ -184,8 +185,9 @@ k_col(StepConst c, ColArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T>* sm = (cx<T>*)smraw;
     const int TX = a.tx, n = a.n;
+    const FastDiv dtx(TX), dn(n);
     const int lpn = padded_len(n);
-    const ColMap mp{TX, lpn};
+    const ColMap mp{dtx, lpn};
     const int x0 = blockIdx.x * TX;
     const long long off = (long long)blockIdx.y * a.other_stride + x0;
     const long long np = c.npts;
@@ -196,7 +198,7 @@ k_col(StepConst c, ColArgs a) {
 #pragma unroll
     for (int m = 0; m < MS; ++m) fac[m] = (a.flags & COL_SCALE) ? (T)(a.info[INFO_SC + m] * a.cfac) : (T)1;
     for (int idx = threadIdx.x; idx < nel; idx += blockDim.x) {
-        const int t = idx % TX, q = idx / TX, e = q % n, m = q / n;
+        const int t = idx % dtx, q = idx / dtx, e = q % dn, m = q / dn;
         cx<T> v = S[(size_t)m * np + off + (size_t)e * a.axis_stride + t];
         if (a.flags & COL_SCALE) v = cscale(v, fac[m]);
         sm[(m * lpn + pad_idx(e)) * TX + t] = v;
@@ -206,7 +208,7 @@ k_col(StepConst c, ColArgs a) {
     if (a.flags & COL_KOP) {
         // spectral positions -> frequency indices (digit-reversed order)
         for (int p = threadIdx.x; p < n * TX; p += blockDim.x) {
-            const int t = p % TX, e = p / TX;
+            const int t = p % dtx, e = p / dtx;
             const int ix = c.fx[x0 + t];
             // y lines: ky at the line position; z lines: ky at the block's y
             int iy, iz;
@@ -223,7 +225,7 @@ k_col(StepConst c, ColArgs a) {
     }
     if (a.flags & COL_INV) block_fft<T, true>(sm, mp, MS * TX, a.plan, tw);
     for (int idx = threadIdx.x; idx < nel; idx += blockDim.x) {
-        const int t = idx % TX, q = idx / TX, e = q % n, m = q / n;
+        const int t = idx % dtx, q = idx / dtx, e = q % dn, m = q / dn;
         S[(size_t)m * np + off + (size_t)e * a.axis_stride + t] = sm[(m * lpn + pad_idx(e)) * TX + t];
     }
 }
@@ -238,6 +240,7 @@ k_r1d(StepConst c, Split1dArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T>* sm = (cx<T>*)smraw;
     const int n1 = a.n1, R = a.tile;
+    const FastDiv dn1(n1), dr(R);
     const int lp = padded_len(n1);
     const RowMap mp{lp};
     const int row0 = blockIdx.x * R;
@@ -248,13 +251,13 @@ k_r1d(StepConst c, Split1dArgs a) {
     for (int m = 0; m < MS; ++m) fac[m] = (T)(a.info[INFO_SC + m] / (double)np);
     const int nel = MS * R * n1;
     for (int idx = threadIdx.x; idx < nel; idx += blockDim.x) {
-        const int x = idx % n1, q = idx / n1, r = q % R, m = q / R;
+        const int x = idx % dn1, q = idx / dn1, r = q % dr, m = q / dr;
         sm[(m * R + r) * lp + pad_idx(x)] = cscale(S[(size_t)m * np + (size_t)(row0 + r) * n1 + x], fac[m]);
     }
     __syncthreads();
     block_fft<T, false>(sm, mp, MS * R, c.px, (const cx<T>*)a.tw1);
     for (int p = threadIdx.x; p < R * n1; p += blockDim.x) {
-        const int x = p % n1, r = p / n1;
+        const int x = p % dn1, r = p / dn1;
         const int k = c.fy[row0 + r] + a.n2 * c.fx[x];
         cx<T> v[MS];
 #pragma unroll
@@ -267,7 +270,7 @@ k_r1d(StepConst c, Split1dArgs a) {
     __syncthreads();
     block_fft<T, true>(sm, mp, MS * R, c.px, (const cx<T>*)a.tw1);
     for (int idx = threadIdx.x; idx < nel; idx += blockDim.x) {
-        const int x = idx % n1, q = idx / n1, r = q % R, m = q / R;
+        const int x = idx % dn1, q = idx / dn1, r = q % dr, m = q / dr;
         S[(size_t)m * np + (size_t)(row0 + r) * n1 + x] = sm[(m * R + r) * lp + pad_idx(x)];
     }
 }
@@ -286,8 +289,9 @@ k_c1d(StepConst c, Split1dArgs a) {
     __shared__ double red[32 * (MS + 1)];
     __shared__ double bsum[MS];
     const int n1 = a.n1, n2 = a.n2, TX = a.tile;
+    const FastDiv dtx(TX), dn2(n2);
     const int lpn = padded_len(n2);
-    const ColMap mp{TX, lpn};
+    const ColMap mp{dtx, lpn};
     const int x0 = blockIdx.x * TX;
     const long long np = c.npts;
     const cx<T>* twn = (const cx<T>*)a.twn;
@@ -296,7 +300,7 @@ k_c1d(StepConst c, Split1dArgs a) {
     const int nel = MS * n2 * TX;
     const cx<T>* src = a.mode == C1D_FWD ? (const cx<T>*)a.psi : S;
     for (int idx = threadIdx.x; idx < nel; idx += blockDim.x) {
-        const int t = idx % TX, q = idx / TX, e = q % n2, m = q / n2;
+        const int t = idx % dtx, q = idx / dtx, e = q % dn2, m = q / dn2;
         cx<T> v = src[(size_t)m * np + (size_t)e * n1 + x0 + t];
         if (a.mode != C1D_FWD) v = cmulc(v, twn[(size_t)(x0 + t) * c.fy[e]]);   // conj twiddle
         sm[(m * lpn + pad_idx(e)) * TX + t] = v;
@@ -307,7 +311,7 @@ k_c1d(StepConst c, Split1dArgs a) {
         const T inv = (T)(1.0 / n2);
         cx<T>* dst = (cx<T>*)a.psi;
         for (int idx = threadIdx.x; idx < nel; idx += blockDim.x) {
-            const int t = idx % TX, q = idx / TX, e = q % n2, m = q / n2;
+            const int t = idx % dtx, q = idx / dtx, e = q % dn2, m = q / dn2;
             dst[(size_t)m * np + (size_t)e * n1 + x0 + t] = cscale(sm[(m * lpn + pad_idx(e)) * TX + t], inv);
         }
         return;
@@ -318,7 +322,7 @@ k_c1d(StepConst c, Split1dArgs a) {
         for (int m = 0; m < MS; ++m) acc[m] = 0.0;
         cx<T>* snap = (cx<T>*)a.snap;
         for (int p = threadIdx.x; p < n2 * TX; p += blockDim.x) {
-            const int t = p % TX, e = p / TX;
+            const int t = p % dtx, e = p / dtx;
             const int x = x0 + t + n1 * e;             // 1D grid index
             cx<T> v[MS];
 #pragma unroll
@@ -344,7 +348,7 @@ k_c1d(StepConst c, Split1dArgs a) {
     }
     block_fft<T, false>(sm, mp, MS * TX, c.py, tw2);
     for (int idx = threadIdx.x; idx < nel; idx += blockDim.x) {
-        const int t = idx % TX, q = idx / TX, e = q % n2, m = q / n2;
+        const int t = idx % dtx, q = idx / dtx, e = q % dn2, m = q / dn2;
         S[(size_t)m * np + (size_t)e * n1 + x0 + t] = cmul(sm[(m * lpn + pad_idx(e)) * TX + t], twn[(size_t)(x0 + t) * c.fy[e]]);
     }
 }
@@ -381,13 +385,14 @@ k_cl1d(StepConst c, Cluster1dArgs a) {
     __shared__ double s_sig[2];
     const int n1 = a.n1, n2 = a.n2;
     const int RR = n2 / CL1D, CC = n1 / CL1D;
+    const FastDiv dn1(n1), dn2(n2), drr(RR), dcc(CC);
     const int lp1 = padded_len(n1), lpn = padded_len(n2);
     const int nrow = MS * RR * n1;
     const int rtile = MS * RR * lp1;               // one row buffer, [m][r][pad(x)]
     cx<T>* rowbuf = (cx<T>*)smraw;                 // two row buffers
     cx<T>* cols = rowbuf + 2 * rtile;              // [m][pad(e)][t], t < CC
     const RowMap rmp{lp1};
-    const ColMap cmp{CC, lpn};
+    const ColMap cmp{dcc, lpn};
     const int rank = (int)cl.block_rank();
     const int row0 = rank * RR, x0 = rank * CC;
     const long long np = c.npts;
@@ -400,7 +405,7 @@ k_cl1d(StepConst c, Cluster1dArgs a) {
     __syncthreads();
     // this CTA's rows, scaled by sc_m/N as the row pass loads them
     for (int idx = threadIdx.x; idx < nrow; idx += blockDim.x) {
-        const int x = idx % n1, q = idx / n1, r = q % RR, m = q / RR;
+        const int x = idx % dn1, q = idx / dn1, r = q % drr, m = q / drr;
         rowbuf[(m * RR + r) * lp1 + pad_idx(x)] =
             cscale(S[(size_t)m * np + (size_t)(row0 + r) * n1 + x], (T)(s_sc[m] / (double)np));
     }
@@ -412,7 +417,7 @@ k_cl1d(StepConst c, Cluster1dArgs a) {
         // ---- row phase: F_N1, KE and SOC at k = k2 + N2*k1, F_N1^-1
         block_fft<T, false>(rows, rmp, MS * RR, c.px, tw1);
         for (int p = threadIdx.x; p < RR * n1; p += blockDim.x) {
-            const int x = p % n1, r = p / n1;
+            const int x = p % dn1, r = p / dn1;
             const int k = c.fy[row0 + r] + n2 * c.fx[x];
             cx<T> v[MS];
 #pragma unroll
@@ -428,9 +433,9 @@ k_cl1d(StepConst c, Cluster1dArgs a) {
         // ---- column phase: gather with the conjugate twiddle, F_N2^-1,
         // SE, SP, NORMC (+ snapshot), F_N2
         for (int idx = threadIdx.x; idx < ncol; idx += blockDim.x) {
-            const int t = idx % CC, q = idx / CC, e = q % n2, m = q / n2;
-            const cx<T>* src = cl.map_shared_rank(rows, e / RR);
-            const cx<T> v = src[(m * RR + e % RR) * lp1 + pad_idx(x0 + t)];
+            const int t = idx % dcc, q = idx / dcc, e = q % dn2, m = q / dn2;
+            const cx<T>* src = cl.map_shared_rank(rows, e / drr);
+            const cx<T> v = src[(m * RR + e % drr) * lp1 + pad_idx(x0 + t)];
             cols[(m * lpn + pad_idx(e)) * CC + t] = cmulc(v, twn[(size_t)(x0 + t) * c.fy[e]]);
         }
         __syncthreads();
@@ -441,7 +446,7 @@ k_cl1d(StepConst c, Cluster1dArgs a) {
 #pragma unroll
         for (int m = 0; m < MS; ++m) acc[m] = 0.0;
         for (int p = threadIdx.x; p < n2 * CC; p += blockDim.x) {
-            const int t = p % CC, e = p / CC;
+            const int t = p % dcc, e = p / dcc;
             const int x = x0 + t + n1 * e;             // 1D grid index
             cx<T> v[MS];
 #pragma unroll
@@ -467,9 +472,9 @@ k_cl1d(StepConst c, Cluster1dArgs a) {
         block_fft<T, false>(cols, cmp, MS * CC, c.py, tw2);
         // ---- scatter with the twiddle into the owners' next rows
         for (int idx = threadIdx.x; idx < ncol; idx += blockDim.x) {
-            const int t = idx % CC, q = idx / CC, e = q % n2, m = q / n2;
-            cx<T>* dst = cl.map_shared_rank(next, e / RR);
-            dst[(m * RR + e % RR) * lp1 + pad_idx(x0 + t)] =
+            const int t = idx % dcc, q = idx / dcc, e = q % dn2, m = q / dn2;
+            cx<T>* dst = cl.map_shared_rank(next, e / drr);
+            dst[(m * RR + e % drr) * lp1 + pad_idx(x0 + t)] =
                 cmul(cols[(m * lpn + pad_idx(e)) * CC + t], twn[(size_t)(x0 + t) * c.fy[e]]);
         }
         cl.sync();                               // (2) next rows complete, block sums in place
@@ -503,7 +508,7 @@ k_cl1d(StepConst c, Cluster1dArgs a) {
         // leaves the scales pending in info)
         if (step + 1 < a.nsteps) {
             for (int idx = threadIdx.x; idx < nrow; idx += blockDim.x) {
-                const int x = idx % n1, q = idx / n1, r = q % RR, m = q / RR;
+                const int x = idx % dn1, q = idx / dn1, r = q % drr, m = q / drr;
                 cx<T>& v = next[(m * RR + r) * lp1 + pad_idx(x)];
                 v = cscale(v, (T)(s_sc[m] / (double)np));
             }
@@ -513,7 +518,7 @@ k_cl1d(StepConst c, Cluster1dArgs a) {
     // Q back to global memory; the scales stay pending in info
     const cx<T>* fin = rowbuf + (a.nsteps & 1) * rtile;
     for (int idx = threadIdx.x; idx < nrow; idx += blockDim.x) {
-        const int x = idx % n1, q = idx / n1, r = q % RR, m = q / RR;
+        const int x = idx % dn1, q = idx / dn1, r = q % drr, m = q / drr;
         S[(size_t)m * np + (size_t)(row0 + r) * n1 + x] = fin[(m * RR + r) * lp1 + pad_idx(x)];
     }
 }
@@ -531,12 +536,13 @@ k_1d(StepConst c, OneDArgs a) {
     __shared__ double bsum[MS];
     __shared__ double s_sc[MS];
     const int nx = c.nx;
+    const FastDiv dnx(nx);
     const int lp = padded_len(nx);
     const RowMap mp{lp};
     const cx<T>* tw = (const cx<T>*)c.twx;
     cx<T>* psi = (cx<T>*)a.psi;
     for (int idx = threadIdx.x; idx < MS * nx; idx += blockDim.x) {
-        const int x = idx % nx, m = idx / nx;
+        const int x = idx % dnx, m = idx / dnx;
         sm[m * lp + pad_idx(x)] = cscale(psi[(size_t)m * nx + x], (T)a.info[INFO_SC + m]);
     }
     __syncthreads();
@@ -588,7 +594,7 @@ k_1d(StepConst c, OneDArgs a) {
         __syncthreads();
         if (c.imag) {
             for (int idx = threadIdx.x; idx < MS * nx; idx += blockDim.x) {
-                const int x = idx % nx, m = idx / nx;
+                const int x = idx % dnx, m = idx / dnx;
                 sm[m * lp + pad_idx(x)] = cscale(sm[m * lp + pad_idx(x)], (T)s_sc[m]);
             }
             __syncthreads();
@@ -597,13 +603,13 @@ k_1d(StepConst c, OneDArgs a) {
             if (threadIdx.x < MS) a.info_prev[INFO_SC + threadIdx.x] = 1.0;
             cx<T>* sp = (cx<T>*)a.snap_prev;
             for (int idx = threadIdx.x; idx < MS * nx; idx += blockDim.x) {
-                const int x = idx % nx, m = idx / nx;
+                const int x = idx % dnx, m = idx / dnx;
                 sp[(size_t)m * nx + x] = sm[m * lp + pad_idx(x)];
             }
         }
     }
     for (int idx = threadIdx.x; idx < MS * nx; idx += blockDim.x) {
-        const int x = idx % nx, m = idx / nx;
+        const int x = idx % dnx, m = idx / dnx;
         psi[(size_t)m * nx + x] = sm[m * lp + pad_idx(x)];
     }
     if (threadIdx.x < MS) a.info[INFO_SC + threadIdx.x] = 1.0;
