@@ -183,6 +183,16 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
             rowC[tid] = oc;
         }
         const long long bofs = g.fold ? 0 : bq * g.sBb;
+        // rows past the end of a short tile (a weight gradient has 6 to 32 rows)
+        // are zeroed once per tile and not staged again with every K slice
+        const int mv = (int)(rows - m0 < TM ? (rows - m0 + 7) / 8 * 8 : TM);
+        if (mv < TM) {
+            for (int e = tid; e < (TM - mv) * (KC / 8); e += 128) {
+                const int off = a_off(mv + e % (TM - mv), e / (TM - mv) * 8);
+                *(uint4*)(sAh + off) = make_uint4(0u, 0u, 0u, 0u);
+                if (A_SPLIT) *(uint4*)(sAl + off) = make_uint4(0u, 0u, 0u, 0u);
+            }
+        }
         __syncthreads();
         for (int k0 = 0; k0 < g.K && ok; k0 += KC) {
             // K extent staged this round, a multiple of 16 (the products read
@@ -193,11 +203,11 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
                 // A rows as float4 along K: 16 consecutive threads read one
                 // row's 256-byte slice; 8 vectors in flight per thread
 #pragma unroll 1
-                for (int e0 = 0; e0 < TM * kx4; e0 += 128 * 8) {
+                for (int e0 = 0; e0 < mv * kx4; e0 += 128 * 8) {
                     float4 v[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const int e = min(e0 + tid + j * 128, TM * kx4 - 1);
+                        const int e = min(e0 + tid + j * 128, mv * kx4 - 1);
                         const int m = e / kx4, kq = (e % kx4) * 4;
                         const long long oa = rowA[m];
                         const float* src = (const float*)A + oa + k0 + kq;
@@ -213,7 +223,7 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
                         const int e = e0 + tid + j * 128;
-                        if (e < TM * kx4) {
+                        if (e < mv * kx4) {
                             const int m = e / kx4, kq = (e % kx4) * 4;
                             put4(sAh, sAl, a_off(m, kq), v[j]);
                         }
@@ -224,12 +234,13 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
                 // each thread issues LB independent loads before it converts and
                 // stores them (the loads' latency overlaps)
                 const bool akf = g.sAk == 1;
+                const int na = akf ? mv * kx : TM * kx;
 #pragma unroll 1
-                for (int e0 = 0; e0 < TM * kx; e0 += 128 * LB) {
+                for (int e0 = 0; e0 < na; e0 += 128 * LB) {
                     float v[LB];
 #pragma unroll
                     for (int j = 0; j < LB; ++j) {
-                        const int e = min(e0 + tid + j * 128, TM * kx - 1);   // TM*kx is a multiple of 128*LB
+                        const int e = min(e0 + tid + j * 128, na - 1);
                         const int m = akf ? e / kx : e % TM, k = akf ? e % kx : e / TM;
                         const long long oa = rowA[m];
                         v[j] = (oa >= 0 && k0 + k < g.K) ? ld_any(A + oa + (long long)(k0 + k) * g.sAk) : 0.f;
@@ -237,7 +248,7 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
 #pragma unroll
                     for (int j = 0; j < LB; ++j) {
                         const int e = e0 + tid + j * 128;
-                        if (e >= TM * kx) continue;
+                        if (e >= na) continue;
                         const int m = akf ? e / kx : e % TM, k = akf ? e % kx : e / TM;
                         const int off = a_off(m, k);
                         if (A_SPLIT) {

@@ -5,8 +5,10 @@
 // the network (pointwise channel mixing, the truncated DFT onto the retained
 // modes, the per-mode channel mixing) is expressed as this GEMM.
 #pragma once
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 namespace fno {
 
@@ -85,9 +87,24 @@ __device__ __forceinline__ float gelu_g(float x) {
     return 0.5f * (1.f + t) + 0.5f * x * (1.f - t * t) * c * (1.f + 3.f * 0.044715f * x * x);
 }
 
-// z[b,c,s] += bias[c]; h = act(z) (act 1: GELU, 0: identity)
-__global__ void k_bias_act(float* z, float* h, const float* bias, long long C, long long S, long long n, int act) {
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+// z[b,c,s] += bias[c]; h = act(z) (act 1: GELU, 0: identity).  vec: four
+// values per access (16-byte aligned rows, S a multiple of 4).
+__global__ void k_bias_act(float* z, float* h, const float* bias, long long C, long long S, long long n, int act, int vec) {
+    const long long step = (long long)gridDim.x * blockDim.x, t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (vec) {
+        for (long long t = t0; t < n / 4; t += step) {
+            const float b = bias ? bias[(4 * t / S) % C] : 0.f;
+            float4 v = ((const float4*)z)[t];
+            v.x += b; v.y += b; v.z += b; v.w += b;
+            ((float4*)z)[t] = v;
+            if (h) {
+                if (act) v = make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
+                ((float4*)h)[t] = v;
+            }
+        }
+        return;
+    }
+    for (long long t = t0; t < n; t += step) {
         const long long c = (t / S) % C;
         const float v = z[t] + (bias ? bias[c] : 0.f);
         z[t] = v;
@@ -95,47 +112,85 @@ __global__ void k_bias_act(float* z, float* h, const float* bias, long long C, l
     }
 }
 
-__global__ void k_act_bwd(float* dz, const float* dh, const float* z, long long n) {
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
-        dz[t] = dh[t] * gelu_g(z[t]);
+__global__ void k_act_bwd(float* dz, const float* dh, const float* z, long long n, int vec) {
+    const long long step = (long long)gridDim.x * blockDim.x, t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (vec) {
+        for (long long t = t0; t < n / 4; t += step) {
+            const float4 d = ((const float4*)dh)[t], v = ((const float4*)z)[t];
+            ((float4*)dz)[t] = make_float4(d.x * gelu_g(v.x), d.y * gelu_g(v.y), d.z * gelu_g(v.z), d.w * gelu_g(v.w));
+        }
+        return;
+    }
+    for (long long t = t0; t < n; t += step) dz[t] = dh[t] * gelu_g(z[t]);
 }
 
-// out[c] = beta*out[c] + sum_{b,s} x[b,c,s] in a fixed order.  S == 1 (the
-// per-chunk weight-gradient partials): one thread per channel walks b, the
-// reads coalesced across channels.  Otherwise one block per channel, each
-// thread with eight independent accumulators over its strided elements.
-__global__ void k_channel_sum_rows(float* out, const float* x, long long B, long long C, float beta) {
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
+// out[c] = beta*out[c] + sum_{b,s} x[b,c,s] in a fixed order, in FP64.
+//
+// S == 1 (the per-chunk weight-gradient partials): 32 channels per block,
+// eight threads each walk every eighth b with reads coalesced across channels
+// (1024 weights x 128 chunks: one thread per weight took 15 us, most of it one
+// load after the other).
+__global__ void __launch_bounds__(256) k_channel_sum_rows(float* out, const float* x, long long B, long long C, float beta) {
+    __shared__ double red[8][33];
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const long long c = (long long)blockIdx.x * 32 + lane;
     double acc = 0.0;
-    for (long long b = 0; b < B; ++b) acc += x[b * C + c];
-    out[c] = beta * out[c] + (float)acc;
+    if (c < C) {
+#pragma unroll 4
+        for (long long b = g; b < B; b += 8) acc += x[b * C + c];
+    }
+    red[g][lane] = acc;
+    __syncthreads();
+    if (g == 0 && c < C) {
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s += red[q][lane];
+        out[c] = beta * out[c] + (float)s;
+    }
 }
 
-__global__ void k_channel_sum(float* out, const float* x, long long B, long long C, long long S, float beta) {
-    const long long c = blockIdx.x;
-    const long long bd = blockDim.x;
-    double a[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) a[q] = 0.0;
+// Otherwise one cluster of eight blocks per channel, an eighth of s each: a
+// layer has 32 channels, and one block per channel left most of the GPU idle
+// (32 channels of 2^18 points: 33 -> 9 us).
+constexpr int kSumBlocks = 8;
+__global__ void __cluster_dims__(kSumBlocks, 1, 1) __launch_bounds__(256)
+k_channel_sum(float* out, const float* x, long long B, long long C, long long S, float beta) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    const int rank = (int)cl.block_rank();
+    const long long c = blockIdx.x / kSumBlocks;
+    const long long per = ((S + kSumBlocks - 1) / kSumBlocks + 3) / 4 * 4;
+    const long long s0 = per * rank < S ? per * rank : S, s1 = s0 + per < S ? s0 + per : S;
+    double a[4] = {0.0, 0.0, 0.0, 0.0};
     for (long long b = 0; b < B; ++b) {
         const float* row = x + (b * C + c) * S;
-        long long s = threadIdx.x;
-        for (; s + 7 * bd < S; s += 8 * bd) {
-#pragma unroll
-            for (int q = 0; q < 8; ++q) a[q] += row[s + q * bd];
+        if (((uintptr_t)row & 15) == 0) {          // s0 is a multiple of 4
+            const long long v1 = s0 + (s1 - s0) / 4 * 4;
+#pragma unroll 4
+            for (long long s = s0 + 4 * threadIdx.x; s < v1; s += 1024) {
+                const float4 v = *(const float4*)(row + s);
+                a[0] += v.x; a[1] += v.y; a[2] += v.z; a[3] += v.w;
+            }
+            for (long long s = v1 + threadIdx.x; s < s1; s += 256) a[0] += row[s];
+        } else {
+#pragma unroll 4
+            for (long long s = s0 + threadIdx.x; s < s1; s += 256) a[0] += row[s];
         }
-        for (; s < S; s += bd) a[0] += row[s];
     }
-    const double acc = ((a[0] + a[1]) + (a[2] + a[3])) + ((a[4] + a[5]) + (a[6] + a[7]));
     __shared__ double red[256];
-    red[threadIdx.x] = acc;
+    red[threadIdx.x] = (a[0] + a[1]) + (a[2] + a[3]);
     __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+    for (int o = 128; o > 0; o >>= 1) {
         if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[c] = beta * out[c] + (float)red[0];
+    cl.sync();
+    if (rank == 0 && threadIdx.x == 0) {
+        double s = 0.0;
+        for (int q = 0; q < kSumBlocks; ++q) s += *cl.map_shared_rank(red, q);
+        out[c] = beta * out[c] + (float)s;
+    }
+    cl.sync();          // no block leaves while its sum is read
 }
 
 __global__ void k_axpy(float* y, const float* x, float a, long long n) {
@@ -221,28 +276,28 @@ __global__ void k_rbig_fold(const float* drb, float* drr, float* dri, long long 
 }
 
 // ------------------------------------------------- tensor-core dense layer
-// z[m][n] = sum_k A(m,k) x[k][n] + bias[m],  h = GELU(z) or z,  for the
+// z[m][n] = sum_k W(m,k) x[k][n] + bias[m],  h = GELU(z) or z,  for the
 // pointwise channel mixes (M, K <= 128 channels, n over all B*N*N points).
-// A(m,k) = W[m*K+k] (or W[k*M+m] when transposed), BF16; x is FP32 and is
+// W(m,k) = W[m*K+k] (or W[k*M+m] when transposed), BF16; x is FP32 and is
 // rounded to BF16 on its way into shared memory; accumulation is FP32 in
-// tensor memory.  One CTA (4 warps) per 256 columns of n:
-//   - warp 0 allocates 256 TMEM columns (the 128 x 256 FP32 accumulator);
-//   - all threads stage A (K-major) and the x tile (N-major) in shared memory
-//     in the 8x8 core-matrix layout without swizzle;
-//   - thread 0 issues one tcgen05.mma (kind::f16, M=128, N=256, K=16) per 16
-//     channels and commits to an mbarrier;
-//   - each warp reads its 32 accumulator lanes with tcgen05.ld, adds the
-//     bias, applies GELU and stores rows of z and h.
-// The mbarrier wait is bounded; on expiry the CTA sets *err and skips its
-// stores (the accumulator is freed either way).
+// tensor memory.  The points are the tile's rows and the M output channels its
+// columns: a layer has 6 to 128 channels and 10^5 points, so every row of the
+// 128-row accumulator is a point, and a warp stores 32 adjacent points of
+// one channel at a time.  A CTA (4 warps) is persistent over tiles of 128
+// points; W and the tensor memory are set up once:
+//   - all threads stage the x tile (point-major 8x8 core matrices, no swizzle);
+//   - thread 0 issues one tcgen05.mma (kind::f16, M = 128, N = channels, K =
+//     16) per 16 channels and commits to an mbarrier;
+//   - each thread reads its point's accumulators with tcgen05.ld, adds the
+//     bias, applies GELU and stores.
+// Bound by reading x and writing z and h; several CTAs per SM overlap each
+// other's phases.  32 -> 32 channels of 2^18 points: 35 -> 20 us (3.4 TB/s) against
+// one CTA per 128 columns with the channels as rows, three quarters of which
+// were padding.
+// The mbarrier wait is bounded; on expiry the CTA sets *err, stores nothing
+// more and frees its tensor memory.
 namespace tc {
-// columns of n per CTA (accumulator width); the TMEM it takes (TN columns
-// of 512) bounds the CTAs resident per SM
-#ifndef FNO_DENSE_TN
-#define FNO_DENSE_TN 128
-#endif
-constexpr int TN = FNO_DENSE_TN;
-constexpr int TM = 128;      // accumulator rows (M padded)
+constexpr int TP = 128;      // points per tile (accumulator rows)
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -257,146 +312,150 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t 
     return d;
 }
 
-// Instruction descriptor: F32 accumulator, BF16 A and B, A K-major, B N-major,
-// N = TN, M = TM.
-__host__ __device__ constexpr uint32_t idesc_bf16() {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (0u << 15) | (1u << 16) | ((uint32_t)(TN >> 3) << 17) |
-           ((uint32_t)(TM >> 4) << 24);
+// Instruction descriptor: F32 accumulator, BF16 A and B, A point-major (bit
+// 15), B K-major, N = np, M = TP.
+__device__ __forceinline__ uint32_t idesc_bf16(int np) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | ((uint32_t)(np >> 3) << 17) | ((uint32_t)(TP >> 4) << 24);
+}
+// channels of a layer in tensor memory: accumulator columns, allocated columns
+__host__ __device__ __forceinline__ int dense_np(int M) { return (M + 15) / 16 * 16; }
+__host__ __device__ __forceinline__ int dense_cols(int M) { const int np = dense_np(M); return np <= 32 ? 32 : np <= 64 ? 64 : 128; }
+__host__ __device__ __forceinline__ size_t dense_smem(int M, int K) {
+    const int KP = (K + 15) / 16 * 16;
+    return 1024 + (size_t)KP * TP * 2 + (size_t)KP * dense_np(M) * 2;
 }
 }  // namespace tc
 
-__global__ void __launch_bounds__(128, 1)
+__global__ void __launch_bounds__(128)
 k_dense_tc(const __nv_bfloat16* __restrict__ W, int transw, const float* __restrict__ x, const float* __restrict__ bias,
            float* __restrict__ z, float* __restrict__ h, int M, int K, long long BS, int act, int* err) {
     using namespace tc;
     extern __shared__ __align__(1024) unsigned char smraw[];
-    const int KP = (K + 15) / 16 * 16;
+    const int KP = (K + 15) / 16 * 16, NP = dense_np(M), cols = dense_cols(M);
     // 1024-byte aligned operand tiles
     const uint32_t base = smem_u32(smraw);
     const uint32_t pad = (1024u - (base & 1023u)) & 1023u;
-    unsigned char* sA = smraw + pad;                          // TM x KP bf16, K-major cores
-    unsigned char* sB = sA + (size_t)TM * KP * 2;              // KP x TN bf16, N-major cores
+    unsigned char* sA = smraw + pad;                          // KP x TP bf16, point-major cores
+    unsigned char* sB = sA + (size_t)KP * TP * 2;             // NP x KP bf16, K-major cores
     __shared__ __align__(8) unsigned long long mbar;
     __shared__ uint32_t tmem_slot;
+    __shared__ float sbias[128];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const long long n0 = (long long)blockIdx.x * TN;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                     "r"(TN));
+                     "r"(cols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&mbar)), "r"(1));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // A: element (m, k) -> core (k/8, m/8), row m%8, column k%8
-    for (int e = tid; e < TM * KP; e += 128) {
+    sbias[tid] = (bias && tid < M) ? bias[tid] : 0.f;
+    // W: element (m, k) -> core (k/8, m/8), row m%8, column k%8
+    for (int e = tid; e < NP * KP; e += 128) {
         const int m = e / KP, k = e - (e / KP) * KP;
         __nv_bfloat16 v = __float2bfloat16(0.f);
         if (m < M && k < K) v = transw ? W[(size_t)k * M + m] : W[(size_t)m * K + k];
-        const int off = (((k >> 3) * (TM / 8) + (m >> 3)) << 7) + ((m & 7) << 4) + ((k & 7) << 1);
-        *(__nv_bfloat16*)(sA + off) = v;
+        const int off = (((k >> 3) * (NP / 8) + (m >> 3)) << 7) + ((m & 7) << 4) + ((k & 7) << 1);
+        *(__nv_bfloat16*)(sB + off) = v;
     }
-    // B: eight consecutive n of one k -> 16 bytes of core (k/8, n/8), row k%8
-    for (int e = tid; e < KP * (TN / 8); e += 128) {
-        const int k = e / (TN / 8), g = e - (e / (TN / 8)) * (TN / 8);
-        const long long n = n0 + g * 8;
-        float f[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] = 0.f;
-        if (k < K) {
-            const float* src = x + (size_t)k * BS + n;
-            if (n + 8 <= BS && ((((size_t)k * BS + n) & 3) == 0)) {
-                const float4 a = *(const float4*)src, b = *(const float4*)(src + 4);
-                f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) f[j] = (n + j < BS) ? src[j] : 0.f;
-            }
-        }
-        __nv_bfloat162 p[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) p[j] = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
-        const int off = (((k >> 3) * (TN / 8) + g) << 7) + ((k & 7) << 4);
-        *(uint4*)(sB + off) = *(uint4*)p;
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
-
-    if (tid == 0) {
-        const uint32_t idesc = idesc_bf16();
-        for (int s = 0; s < KP / 16; ++s) {
-            // K-major A: K chunks TM/8 cores apart, 8-row groups 128 B apart
-            const uint64_t da = sdesc(smem_u32(sA) + s * 2 * (TM / 8) * 128, (TM / 8) * 128, 128);
-            // N-major B: k groups TN/8 cores apart, 8-column groups 128 B apart
-            const uint64_t db = sdesc(smem_u32(sB) + s * 2 * (TN / 8) * 128, (TN / 8) * 128, 128);
-            const uint32_t acc = s > 0 ? 1u : 0u;
-            asm volatile(
-                "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
-                "l"(da), "l"(db), "r"(idesc), "r"(acc));
+    const bool rows16 = (BS & 3) == 0 && ((uintptr_t)x & 15) == 0;
+    const long long ntiles = (BS + TP - 1) / TP;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (long long tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        const long long n0 = tile * TP;
+        // x: eight consecutive points of one k -> 16 bytes of core (k/8, p/8), row k%8
+#pragma unroll 4
+        for (int e = tid; e < KP * (TP / 8); e += 128) {
+            const int k = e / (TP / 8), g = e % (TP / 8);
+            const long long n = n0 + g * 8;
+            float f[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) f[j] = 0.f;
+            if (k < K) {
+                const float* src = x + (size_t)k * BS + n;
+                if (rows16 && n + 8 <= BS) {
+                    const float4 a = *(const float4*)src, b = *(const float4*)(src + 4);
+                    f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) f[j] = (n + j < BS) ? src[j] : 0.f;
+                }
+            }
+            __nv_bfloat162 p[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) p[j] = __floats2bfloat162_rn(f[2 * j], f[2 * j + 1]);
+            *(uint4*)(sA + ((((k >> 3) * (TP / 8) + g) << 7) + ((k & 7) << 4))) = *(uint4*)p;
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-            smem_u32(&mbar)));
-    }
-    // bounded wait for the accumulator (phase 0)
-    uint32_t done = 0;
-    for (long long it = 0; it < (1LL << 22) && !done; ++it) {
-        asm volatile(
-            "{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
-            "selp.b32 %0, 1, 0, P1;\n\t}\n"
-            : "=r"(done)
-            : "r"(smem_u32(&mbar)), "r"(0));
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (!done) {
-        if (lane == 0) atomicExch(err, 1);
-    } else {
-        const int m = warp * 32 + lane;
-        const float bm = (bias && m < M) ? bias[m] : 0.f;
-        for (int cb = 0; cb < TN / 16; ++cb) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        if (tid == 0) {
+            const uint32_t idesc = idesc_bf16(NP);
+            for (int s = 0; s < KP / 16; ++s) {
+                // point-major A: k groups TP/8 cores apart, 8-point groups 128 B apart
+                const uint64_t da = sdesc(smem_u32(sA) + s * 2 * (TP / 8) * 128, (TP / 8) * 128, 128);
+                // K-major B: k groups NP/8 cores apart, 8-channel groups 128 B apart
+                const uint64_t db = sdesc(smem_u32(sB) + s * 2 * (NP / 8) * 128, (NP / 8) * 128, 128);
+                const uint32_t acc = s > 0 ? 1u : 0u;
+                asm volatile(
+                    "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
+                    "l"(da), "l"(db), "r"(idesc), "r"(acc));
+            }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+                smem_u32(&mbar)));
+        }
+        // bounded wait for the accumulator
+        uint32_t done = 0;
+        for (long long it = 0; it < (1LL << 22) && !done; ++it) {
+            asm volatile(
+                "{\n\t.reg .pred P1;\n\tmbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+                "selp.b32 %0, 1, 0, P1;\n\t}\n"
+                : "=r"(done)
+                : "r"(smem_u32(&mbar)), "r"(phase));
+        }
+        phase ^= 1u;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        ok = __syncthreads_and((int)done) != 0;
+        if (!ok) break;
+        const long long n = n0 + tid;            // this thread's point
+        for (int cb = 0; cb < NP; cb += 16) {
             uint32_t r[16];
-            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(cb * 16);
+            const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)cb;
             asm volatile(
                 "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                 : "r"(taddr));
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (m < M) {
-                float v[16], g[16];
+            if (n < BS) {
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    v[j] = __uint_as_float(r[j]) + bm;
-                    g[j] = act ? gelu_f(v[j]) : v[j];
-                }
-                const long long nb = n0 + cb * 16;
-                const size_t row = (size_t)m * BS + nb;
-                if (nb + 16 <= BS && (row & 3) == 0) {
-                    // each thread owns 64 contiguous bytes of its row
-#pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        if (z) *(float4*)(z + row + 4 * q) = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                        if (h) *(float4*)(h + row + 4 * q) = make_float4(g[4 * q], g[4 * q + 1], g[4 * q + 2], g[4 * q + 3]);
-                    }
-                } else {
-                    for (int j = 0; j < 16; ++j) {
-                        if (nb + j < BS) {
-                            if (z) z[row + j] = v[j];
-                            if (h) h[row + j] = g[j];
-                        }
+                    if (cb + j < M) {
+                        const float v = __uint_as_float(r[j]) + sbias[cb + j];
+                        const size_t at = (size_t)(cb + j) * BS + n;
+                        if (z) z[at] = v;
+                        if (h) h[at] = act ? gelu_f(v) : v;
                     }
                 }
             }
         }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }
+    if (!ok && tid == 0) atomicExch(err, 1);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TN));
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(cols));
 }
 
 }  // namespace fno

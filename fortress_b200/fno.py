@@ -217,8 +217,13 @@ class FNO:
         self.dh2 = z(W, B * S)
         self.dz = z(W, B * S)
         self.da = z(self.cin, B * S)
-        self.chunk = S                      # a divisor of B*S of at most ~2048 points
+        # points per weight-gradient product: a divisor of B*S of at most ~2048,
+        # and of 512 where the halves stay whole float4s, so that there are
+        # enough products to fill the GPU (64 x 64, batch 64: 512, not 128)
+        self.chunk = S
         while self.chunk > 2048 and self.chunk % 2 == 0:
+            self.chunk //= 2
+        while self.chunk > 512 and self.chunk % 8 == 0:
             self.chunk //= 2
         self.part = z((B * S // self.chunk) * max(self.hidden, W) * max(self.hidden, W, self.cin))
         self.dHm = z(NA * NM * 2 * W * B)
