@@ -42,37 +42,76 @@ int fno_gemm(int batch, int M, int N, int K, float alpha, const void* A, int a_b
 // tall GEMM; the tile width GN is the smallest of 16..256 that covers N.
 // CTAs per SM: as many as the shared memory (about 227 KB) and the 512 TMEM
 // columns hold, at most four; CTAs beyond those resident wait their turn.
-template <int GN> constexpr int gemm_tc_per_sm() {
-    const int by_smem = (int)((227 * 1024) / (fno::gtc::smem_bytes<GN>() + 3 * 1024));
-    const int by_tmem = 512 / fno::gtc::tmem_cols<GN>();
+template <int GN, int PAIR> constexpr int gemm_tc_per_sm() {
+    const int by_smem = (int)((227 * 1024) / (fno::gtc::smem_bytes<GN, PAIR>() + 3 * 1024));
+    const int by_tmem = 512 / fno::gtc::tmem_cols<GN, PAIR>();
     return std::min(4, std::min(by_smem, by_tmem));
 }
 
-template <typename TA, int GN> static int gemm_tc_launch(const fno::GemmTc& g, cudaStream_t st) {
+template <typename TA, int GN, int PAIR> static int gemm_tc_launch(const fno::GemmTc& g, cudaStream_t st) {
     static bool attr_set[64] = {false};
     int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return FGPE_E_ARG;
-    const size_t smem = fno::gtc::smem_bytes<GN>();
+    const size_t smem = fno::gtc::smem_bytes<GN, PAIR>();
     if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(fno::k_gemm_tc<TA, GN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(fno::k_gemm_tc<TA, GN, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return fno_ck(e);
         attr_set[dev] = true;
     }
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const long long rows = g.fold ? (long long)g.batch * g.M : (long long)g.M;
     const long long tiles = (rows + fno::gtc::TM - 1) / fno::gtc::TM * ((g.N + GN - 1) / GN) * (g.fold ? 1 : g.batch);
-    const long long grid = std::min<long long>(tiles, (long long)gemm_tc_per_sm<GN>() * nsm);
-    fno::k_gemm_tc<TA, GN><<<(unsigned)grid, 128, smem, st>>>(g);
+    const long long grid = std::min<long long>(tiles, (long long)gemm_tc_per_sm<GN, PAIR>() * nsm);
+    fno::k_gemm_tc<TA, GN, PAIR><<<(unsigned)grid, 128, smem, st>>>(g);
     return fno_ck(cudaGetLastError());
 }
 
 template <typename TA> static int gemm_tc_width(const fno::GemmTc& g, cudaStream_t st) {
-    if (g.N <= 16) return gemm_tc_launch<TA, 16>(g, st);
-    if (g.N <= 32) return gemm_tc_launch<TA, 32>(g, st);
-    if (g.N <= 64) return gemm_tc_launch<TA, 64>(g, st);
-    if (g.N <= 128) return gemm_tc_launch<TA, 128>(g, st);
-    return gemm_tc_launch<TA, 256>(g, st);
+    if (g.N <= 16) return gemm_tc_launch<TA, 16, fno::PAIR_NONE>(g, st);
+    if (g.N <= 32) return gemm_tc_launch<TA, 32, fno::PAIR_NONE>(g, st);
+    if (g.N <= 64) return gemm_tc_launch<TA, 64, fno::PAIR_NONE>(g, st);
+    if (g.N <= 128) return gemm_tc_launch<TA, 128, fno::PAIR_NONE>(g, st);
+    return gemm_tc_launch<TA, 256, fno::PAIR_NONE>(g, st);
+}
+// Pairs take tiles of up to 64 columns (two accumulators, 128 of the 512
+// tensor-memory columns, so that four CTAs fit an SM).
+template <int PAIR> static int gemm_tc_pair_width(const fno::GemmTc& g, cudaStream_t st) {
+    if (g.N <= 16) return gemm_tc_launch<float, 16, PAIR>(g, st);
+    if (g.N <= 32) return gemm_tc_launch<float, 32, PAIR>(g, st);
+    return gemm_tc_launch<float, 64, PAIR>(g, st);
+}
+
+// Checks, the transposed form for a shared left operand, and the float4
+// forms, for one product (A1 = B1 = C1 = null) or a pair.
+static int gemm_tc_args(int batch, int M, int N, int K, float alpha, const void* A, const void* A1, int a_bf16, long long sAb,
+                        long long sAi, long long sAk, const float* B, const float* B1, long long sBb, long long sBk,
+                        long long sBj, float beta, float* C, float* C1, long long sCb, long long sCi, long long sCj,
+                        int* err_dev, fno::GemmTc* out) {
+    if (!A || !B || !C || !err_dev) { fgpe::set_last_error("null argument"); return FGPE_E_ARG; }
+    if (batch <= 0 || M <= 0 || N <= 0 || K <= 0) { fgpe::set_last_error("empty GEMM"); return FGPE_E_ARG; }
+    if (sAb < 0 || sAi < 0 || sAk < 0 || sBb < 0 || sBk < 0 || sBj < 0 || sCb < 0 || sCi < 0 || sCj < 0) {
+        fgpe::set_last_error("negative stride");
+        return FGPE_E_ARG;
+    }
+    fno::GemmTc g{M, N, K, batch, 0, alpha, beta, A, sAb, sAi, sAk, B, sBb, sBk, sBj, C, sCb, sCi, sCj, err_dev, 0, 0, 0,
+                  A1, B1, C1};
+    if (batch > 1 && sAb == 0 && sBb != 0 && !a_bf16) {
+        // C^T = B^T A^T: the shared A becomes the B operand
+        g = fno::GemmTc{N, M, K, batch, 0, alpha, beta, B, sBb, sBj, sBk, (const float*)A, 0, sAk, sAi,
+                        C, sCb, sCj, sCi, err_dev, 0, 0, 0, B1, (const float*)A1, C1};
+    }
+    g.fold = batch > 1 && g.sBb == 0;
+    // float4 operand reads where the unit-stride runs start on 16-byte boundaries
+    const bool a16 = (((uintptr_t)g.A | (uintptr_t)g.A1) & 15) == 0, b16 = (((uintptr_t)g.B | (uintptr_t)g.B1) & 15) == 0;
+    g.avec = !a_bf16 && a16 && g.sAk == 1 && g.sAi % 4 == 0 && g.sAb % 4 == 0;
+    if (b16 && g.sBb % 4 == 0) {
+        if (g.sBj == 1 && g.sBk % 4 == 0) g.bvec = 1;
+        else if (g.sBk == 1 && g.sBj % 4 == 0) g.bvec = 2;
+    }
+    g.cvec = (((uintptr_t)g.C | (uintptr_t)g.C1) & 15) == 0 && g.sCj == 1 && g.sCi % 4 == 0 && g.sCb % 4 == 0;
+    *out = g;
+    return FGPE_OK;
 }
 
 extern "C" {
@@ -80,31 +119,28 @@ extern "C" {
 int fno_gemm_tc(int batch, int M, int N, int K, float alpha, const void* A, int a_bf16, long long sAb, long long sAi,
                 long long sAk, const float* B, long long sBb, long long sBk, long long sBj, float beta, float* C,
                 long long sCb, long long sCi, long long sCj, int* err_dev, void* stream) {
-    if (!A || !B || !C || !err_dev) { fgpe::set_last_error("null argument"); return FGPE_E_ARG; }
-    if (batch <= 0 || M <= 0 || N <= 0 || K <= 0) { fgpe::set_last_error("empty GEMM"); return FGPE_E_ARG; }
-    if (sAb < 0 || sAi < 0 || sAk < 0 || sBb < 0 || sBk < 0 || sBj < 0 || sCb < 0 || sCi < 0 || sCj < 0) {
-        fgpe::set_last_error("negative stride");
-        return FGPE_E_ARG;
-    }
-    fno::GemmTc g{M, N, K, batch, 0, alpha, beta, A, sAb, sAi, sAk, B, sBb, sBk, sBj, C, sCb, sCi, sCj, err_dev, 0, 0, 0};
-    if (batch > 1 && sAb == 0 && sBb != 0 && !a_bf16) {
-        // C^T = B^T A^T: the shared A becomes the B operand
-        g = fno::GemmTc{N, M, K, batch, 0, alpha, beta, B, sBb, sBj, sBk, (const float*)A, 0, sAk, sAi,
-                        C, sCb, sCj, sCi, err_dev, 0, 0, 0};
-    }
-    g.fold = batch > 1 && g.sBb == 0;
-    // float4 operand reads where the unit-stride runs start on 16-byte boundaries
-    const bool a16 = ((uintptr_t)g.A & 15) == 0, b16 = ((uintptr_t)g.B & 15) == 0;
-    g.avec = !a_bf16 && a16 && g.sAk == 1 && g.sAi % 4 == 0 && g.sAb % 4 == 0;
-    if (b16 && g.sBb % 4 == 0) {
-        if (g.sBj == 1 && g.sBk % 4 == 0) g.bvec = 1;
-        else if (g.sBk == 1 && g.sBj % 4 == 0) g.bvec = 2;
-    }
-    g.cvec = ((uintptr_t)g.C & 15) == 0 && g.sCj == 1 && g.sCi % 4 == 0 && g.sCb % 4 == 0;
+    fno::GemmTc g;
+    const int rc = gemm_tc_args(batch, M, N, K, alpha, A, nullptr, a_bf16, sAb, sAi, sAk, B, nullptr, sBb, sBk, sBj, beta, C,
+                                nullptr, sCb, sCi, sCj, err_dev, &g);
+    if (rc) return rc;
     const cudaStream_t st = (cudaStream_t)stream;
     return a_bf16 ? gemm_tc_width<__nv_bfloat16>(g, st) : gemm_tc_width<float>(g, st);
 }
 
+int fno_gemm_tc2(int batch, int M, int N, int K, float alpha, const float* A0, const float* A1, long long sAb, long long sAi,
+                 long long sAk, const float* B0, const float* B1, long long sBb, long long sBk, long long sBj, float beta,
+                 float* C0, float* C1, long long sCb, long long sCi, long long sCj, int* err_dev, void* stream) {
+    if (!A1 || !B1 || !C1) { fgpe::set_last_error("null argument"); return FGPE_E_ARG; }
+    fno::GemmTc g;
+    const int rc = gemm_tc_args(batch, M, N, K, alpha, A0, A1, 0, sAb, sAi, sAk, B0, B1, sBb, sBk, sBj, beta, C0, C1, sCb, sCi,
+                                sCj, err_dev, &g);
+    if (rc) return rc;
+    const cudaStream_t st = (cudaStream_t)stream;
+    if (C0 == C1) return gemm_tc_pair_width<fno::PAIR_SUM>(g, st);
+    if (g.A == g.A1) return gemm_tc_pair_width<fno::PAIR_SPLIT>(g, st);
+    fgpe::set_last_error("a pair of products shares its output, or its batched operand");
+    return FGPE_E_ARG;
+}
 int fno_bias_act(float* z, float* h, const float* bias, long long C, long long S, long long n, int act, void* stream) {
     const int vec = S % 4 == 0 && n % 4 == 0 && (((uintptr_t)z | (uintptr_t)h) & 15) == 0;
     fno::k_bias_act<<<fno_grid(vec ? n / 4 : n), 256, 0, (cudaStream_t)stream>>>(z, h, bias, C, S, n, act, vec);

@@ -37,7 +37,8 @@ import numpy as np
 from . import _abi
 
 FNO_EXPORTS = ("fno_gemm", "fno_bias_act", "fno_act_bwd", "fno_channel_sum", "fno_axpy", "fno_mse",
-               "fno_adam", "fno_to_bf16", "fno_rbig_build", "fno_rbig_fold", "fno_dense_tc", "fno_gemm_tc")
+               "fno_adam", "fno_to_bf16", "fno_rbig_build", "fno_rbig_fold", "fno_dense_tc", "fno_gemm_tc",
+               "fno_gemm_tc2")
 
 _L = None
 
@@ -60,6 +61,7 @@ def lib():
         "fno_rbig_build": [vp, vp, vp, ll, ip, ip, vp],
         "fno_rbig_fold": [vp, vp, vp, ll, ip, ip, vp],
         "fno_dense_tc": [vp, ip, vp, vp, vp, vp, ip, ip, ll, ip, vp, vp],
+        "fno_gemm_tc2": [ip, ip, ip, ip, fl, vp, vp, ll, ll, ll, vp, vp, ll, ll, ll, fl, vp, vp, ll, ll, ll, vp, vp],
         "fno_gemm_tc": [ip, ip, ip, ip, fl, vp, ip, ll, ll, ll, vp, ll, ll, ll, fl, vp, ll, ll, ll, vp, vp],
     }
     for name, args in sig.items():
@@ -258,6 +260,20 @@ class FNO:
         else:
             _ck(self.L.fno_gemm(*args, self._st()), "gemm")
 
+    def gemm2(self, batch, M, N, K, A, sA, B_, sB, C, sC, alpha=1.0, beta=0.0):
+        """The two products A[0] B_[0] and A[1] B_[1] of one shape; A, B_ and C
+        are pairs of (tensor, offset).  The same C twice: the first product
+        with beta, the second added; otherwise one product into each."""
+        if self.tensor_cores:
+            p = [ctypes.c_void_p(t.data_ptr() + 4 * o) for q in (A, B_, C) for t, o in q]
+            _ck(self.L.fno_gemm_tc2(batch, M, N, K, alpha, p[0], p[1], *sA, p[2], p[3], *sB, beta, p[4], p[5], *sC,
+                                    self._p(self.tc_err), self._st()), "gemm_tc2")
+            return
+        same = C[0] == C[1]
+        for q in range(2):
+            self.gemm(batch, M, N, K, A[q][0], sA, B_[q][0], sB, C[q][0], sC, alpha=alpha, beta=1.0 if same and q else beta,
+                      aoff=A[q][1], boff=B_[q][1], coff=C[q][1])
+
     def _use_tc(self, M, K):
         return self.tensor_cores and M <= 128 and K <= 128
 
@@ -290,32 +306,34 @@ class FNO:
         B, W, n, NM, NA = self.B, self.W, self.n, self.NM, self.NA
         CB, OB, nm = W * B, W * B, NA * NM
         T, Hm, Gm, U = self.T, self.Hm[l], self.Gm, self.U
-        for p in range(2):   # T[z1][p] = h_z1 Ey_p
-            self.gemm(CB, n, NM, n, h, (n * n, n, 1), self.Ey[p], (0, NM, 1), T, (2 * n * NM, NM, 1), coff=p * n * NM)
-        for p in range(2):   # Hm[a][k][p][c][b] = ExS_p Tstack_z1
-            self.gemm(CB, NA, NM, 2 * n, self.ExS[p], (0, 2 * n, 1), T, (2 * n * NM, NM, 1),
-                      Hm, (1, NM * 2 * CB, 2 * CB), coff=p * CB)
+        Ey, ExS, ExA, EywT = ([(t, 0) for t in q] for q in (self.Ey, self.ExS, self.ExA, self.EywT))
+        # T[z1][p] = h_z1 Ey_p
+        self.gemm2(CB, n, NM, n, [(h, 0)] * 2, (n * n, n, 1), Ey, (0, NM, 1), [(T, 0), (T, n * NM)], (2 * n * NM, NM, 1))
+        # Hm[a][k][p][c][b] = ExS_p Tstack_z1
+        self.gemm2(CB, NA, NM, 2 * n, ExS, (0, 2 * n, 1), [(T, 0)] * 2, (2 * n * NM, NM, 1),
+                   [(Hm, 0), (Hm, CB)], (1, NM * 2 * CB, 2 * CB))
         # Gm[mode][p][o][b] = Rbig[mode] Hm[mode]
         self.gemm(nm, 2 * W, B, 2 * W, self.pb[f"Rbig{l}"], (4 * W * W, 2 * W, 1), Hm, (2 * W * B, B, 1),
                   Gm, (2 * W * B, B, 1), a_bf16=True)
-        for q in range(2):   # U[z4][p][i][k] = sum_q ExA_q G_q
-            self.gemm(OB, 2 * n, NM, NA, self.ExA[q], (0, NA, 1), Gm, (1, NM * 2 * OB, 2 * OB),
-                      U, (2 * n * NM, NM, 1), beta=float(q), boff=q * OB)
-        for p in range(2):   # z_z4 += U_p EywT_p / n^2
-            self.gemm(OB, n, n, NM, U, (2 * n * NM, NM, 1), self.EywT[p], (0, n, 1), z, (n * n, n, 1),
-                      alpha=1.0 / (n * n), beta=1.0, aoff=p * n * NM)
+        # U[z4][p][i][k] = sum_q ExA_q G_q
+        self.gemm2(OB, 2 * n, NM, NA, ExA, (0, NA, 1), [(Gm, 0), (Gm, OB)], (1, NM * 2 * OB, 2 * OB),
+                   [(U, 0)] * 2, (2 * n * NM, NM, 1))
+        # z_z4 += sum_p U_p EywT_p / n^2
+        self.gemm2(OB, n, n, NM, [(U, 0), (U, n * NM)], (2 * n * NM, NM, 1), EywT, (0, n, 1), [(z, 0)] * 2, (n * n, n, 1),
+                   alpha=1.0 / (n * n), beta=1.0)
 
     def spectral_bwd(self, l, dz, dh):
         """dh += K_l^T dz; gradients of Rr_l, Ri_l."""
         B, W, n, NM, NA = self.B, self.W, self.n, self.NM, self.NA
         CB, OB, nm = W * B, W * B, NA * NM
         T, Hm, Gm, U = self.T, self.Hm[l], self.Gm, self.U     # reused as dT, -, dGm, dU
-        for p in range(2):   # dU_p = dz Eyw_p / n^2
-            self.gemm(OB, n, NM, n, dz, (n * n, n, 1), self.Eyw[p], (0, NM, 1), U, (2 * n * NM, NM, 1),
-                      alpha=1.0 / (n * n), coff=p * n * NM)
-        for q in range(2):   # dG_q = ExA_q^T dUstack
-            self.gemm(OB, NA, NM, 2 * n, self.ExA[q], (0, 1, NA), U, (2 * n * NM, NM, 1),
-                      Gm, (1, NM * 2 * OB, 2 * OB), coff=q * OB)
+        Ey, ExS, ExA, Eyw = ([(t, 0) for t in q] for q in (self.Ey, self.ExS, self.ExA, self.Eyw))
+        # dU_p = dz Eyw_p / n^2
+        self.gemm2(OB, n, NM, n, [(dz, 0)] * 2, (n * n, n, 1), Eyw, (0, NM, 1), [(U, 0), (U, n * NM)], (2 * n * NM, NM, 1),
+                   alpha=1.0 / (n * n))
+        # dG_q = ExA_q^T dUstack
+        self.gemm2(OB, NA, NM, 2 * n, ExA, (0, 1, NA), [(U, 0)] * 2, (2 * n * NM, NM, 1),
+                   [(Gm, 0), (Gm, OB)], (1, NM * 2 * OB, 2 * OB))
         # dRbig = dG Hm^T ; dHm = Rbig^T dG
         self.gemm(nm, 2 * W, 2 * W, B, Gm, (2 * W * B, B, 1), Hm, (2 * W * B, 1, B),
                   self.g_rbig, (4 * W * W, 2 * W, 1))
@@ -324,12 +342,12 @@ class FNO:
         dHm = self.dHm
         self.gemm(nm, 2 * W, B, 2 * W, self.pb[f"Rbig{l}"], (4 * W * W, 1, 2 * W), Gm, (2 * W * B, B, 1),
                   dHm, (2 * W * B, B, 1), a_bf16=True)
-        for p in range(2):   # dTstack = sum_p ExS_p^T dH_p
-            self.gemm(CB, 2 * n, NM, NA, self.ExS[p], (0, 1, 2 * n), dHm, (1, NM * 2 * CB, 2 * CB),
-                      T, (2 * n * NM, NM, 1), beta=float(p), boff=p * CB)
-        for p in range(2):   # dh += dT_p Ey_p^T
-            self.gemm(CB, n, n, NM, T, (2 * n * NM, NM, 1), self.Ey[p], (0, 1, NM), dh, (n * n, n, 1),
-                      beta=1.0, aoff=p * n * NM)
+        # dTstack = sum_p ExS_p^T dH_p
+        self.gemm2(CB, 2 * n, NM, NA, ExS, (0, 1, 2 * n), [(dHm, 0), (dHm, CB)], (1, NM * 2 * CB, 2 * CB),
+                   [(T, 0)] * 2, (2 * n * NM, NM, 1))
+        # dh += sum_p dT_p Ey_p^T
+        self.gemm2(CB, n, n, NM, [(T, 0), (T, n * NM)], (2 * n * NM, NM, 1), Ey, (0, 1, NM), [(dh, 0)] * 2, (n * n, n, 1),
+                   beta=1.0)
 
     # ------------------------------------------------------------ passes
     def forward(self, a_host=None):
