@@ -237,7 +237,7 @@ def run_cpu(w, phi, steps, warmup, budget_s):
 
 def capture(args):
     """The step kernels alone, for ncu launch lists and per-kernel captures
-    (-k regex:k_row_fast / k_col_fast / k_obs ...): warmup + steps split
+    (-k regex:k_regrow / k_regcol / k_row_fast / k_obs ...): warmup + steps split
     steps of the workload on its initial state, no timing and no other work.
     --workload 3d runs the 3D spin-1 case on --grid^3 points (default 192:
     the same kernel families as 256^3, wide column tiles included, with a

@@ -517,7 +517,6 @@ int fgpe_create(const fgpe_params* pin, fgpe_t** out) {
     c.tau0 = p.tau[0]; c.tau1 = p.tau[1]; c.tau2 = p.tau[2];
     c.gx = p.gamma[0]; c.gy = p.dim >= 2 ? p.gamma[1] : 0.0; c.gz = p.dim >= 3 ? p.gamma[2] : 0.0;
     c.se_half = (p.dim == 1 && p.spin == 2);
-    c.se_ge = (p.dim == 1);
     {
         // cgpe1d.f90:250, 443-444: projection in imaginary time when no SOC
         bool soc = fabs(p.gamma[0]) > 1e-40 || (p.dim >= 2 && fabs(p.gamma[1]) > 1e-40) || (p.dim >= 3 && fabs(p.gamma[2]) > 1e-40);

@@ -336,7 +336,6 @@ struct StepConst {
     double tau0, tau1, tau2;
     double gx, gy, gz;
     int se_half;              // 1D spin-2 predictor uses CDT/2 (cgpe1d.f90:1443)
-    int se_ge;                // 1D spin-1 uses |OMEGA| >= EPS (cgpe1d.f90:1413)
     int project;              // imaginary time without SOC: magnetisation projection
     double mag;               // MAG of the projection
     const double *kx, *ky, *kz;

@@ -26,6 +26,11 @@
 // leaves; every other block sees the code at its next ticket or wait and
 // leaves too, so a launch always ends and the host reports the error.
 //
+// What bounds it: the latency of an item (ticket, wait, loads, exchanges), not
+// a pipe or memory, so it runs three blocks of 256 threads per SM with three
+// components, with the column lines in registers (48 instances of 128^2 to
+// 512^2 spin 1: FP32 436 -> 366 us a step, FP64 610 -> 523 us).
+//
 // Coherence.  Data that one block writes and another reads in the same
 // launch (tiles of S, the scales and SIG in info, NORMC partials) is read
 // through L2 only (cp.async.cg, ld.global.cg): an SM's L1 is not coherent
@@ -36,13 +41,14 @@
 
 #include "fgpe_kernels.cuh"
 #include "fgpe_group.cuh"
+#include "fgpe_regcol.cuh"
 
 namespace fgpe {
 
 // One instance of a persistent batch.
 struct PInst {
     InstDesc d;          // constants, state buffers, info, NORMC partial slots
-    const int* fy;       // y position -> frequency map of the kernel's y plan
+    const int* fy;       // y position -> frequency map of the y plan (spin 2)
     int col_tiles;       // x positions / TX
     int row_tiles;       // y rows / R
     int chunk;           // row tiles per row item (divides row_tiles)
@@ -113,16 +119,151 @@ __device__ __forceinline__ void psignal(unsigned* ctr) {
     if (threadIdx.x == 0) atomicAdd(ctr, 1u);
 }
 
-// Radix passes of more than this many tasks per thread stay rolled: one
-// kernel holds the transforms of every line length, under one register cap.
-#ifndef FGPE_PERSIST_UNROLL
-#define FGPE_PERSIST_UNROLL 1
-#endif
-constexpr int kPUnroll = FGPE_PERSIST_UNROLL;
+// Radix plans of the column lines in registers: 0: radix 8 first and 4 last;
+// 1: radix 16 first; 3: other splits of the first two passes.  (Passes over
+// the tile take the plans of cplan.)
+template <int N, int PV> struct PColPlan : SmallPlan<N> {};
+template <int N> struct PColPlan<N, 1> { using P = LPlan<16, N / 64, 4>; };
+template <> struct PColPlan<128, 3> { using P = LPlan<8, 4, 4>; };
+template <> struct PColPlan<192, 3> { using P = LPlan<12, 4, 4>; };
+template <> struct PColPlan<256, 3> { using P = LPlan<4, 16, 4>; };
+template <> struct PColPlan<384, 3> { using P = LPlan<12, 8, 4>; };
+template <> struct PColPlan<512, 3> { using P = LPlan<16, 8, 4>; };
 
-// ------------------------------------------------------------ column tile
+// ------------------------------------------------------------ column tile, spin 1
 // F_y, pending scale + KE + SOC, F_y^-1 on TX adjacent x positions of one
-// instance (the arithmetic of k_col_group, with the y plan PV).
+// instance, in registers as the q2D pass of fgpe_regcol.cuh: five trips
+// through shared memory where passes over the tile take nine.  The tile comes
+// in by 16-byte copies past L1, as another block wrote it.  With five
+// components it is no faster (FP32) or 3 % slower (FP64, spills): pcol_tile.
+template <typename T, int MS, int N, int TX, int TH, class PL>
+__device__ __forceinline__ void pcol_regs(const PInst& P, const StepConst& c, int x0, cx<T>* sm) {
+    constexpr int R0 = PL::R0, R1 = PL::R1, RL = PL::RL;
+    static_assert(PL::N == N && PL::three, "plan length");
+    using TL = RegTile<T, TX, RL>;
+    constexpr int LINE = TL::rows(N) * TX, S0 = N / R0, S1 = S0 / R1, NQ = N / RL, NB = N / R1;
+    constexpr int EPC = 16 / (int)sizeof(cx<T>);
+    static_assert(TX % EPC == 0, "column tile narrower than a 16-byte chunk");
+    static_assert(TH % TX == 0, "threads per tile row");
+    constexpr int CPL = TX / EPC;
+    const long long np = c.npts;
+    const int st = c.nx;
+    cx<T>* S = (cx<T>*)P.d.S + x0;
+    #pragma unroll 1
+    for (int ch = threadIdx.x; ch < MS * N * CPL; ch += TH) {
+        const int tc = (ch % CPL) * EPC, q = ch / CPL, e = q % N, m = q / N;
+        cp16(sm + m * LINE + TL::at(e, tc), S + (size_t)m * np + (size_t)e * st + tc);
+    }
+    cp_commit();
+    // this step's pending scales, published by another block: read through L2
+    const double cfac = 1.0 / (double)c.npts;
+    T fac[MS];
+#pragma unroll
+    for (int m = 0; m < MS; ++m) fac[m] = (T)(__ldcg(P.d.info + INFO_SC + m) * cfac);
+    const cx<T>* tw = (const cx<T>*)c.twy;
+    const cx<T>* key = (const cx<T>*)c.key;
+    const int t = (int)threadIdx.x % TX, imag = c.imag;       // a thread keeps its line
+    const cx<T> kex = ((const cx<T>*)c.kex)[c.fx[x0 + t]];
+    const Soc4<T>* soc = c.soc ? (const Soc4<T>*)c.soc + x0 + t : nullptr;
+    cp_wait<0>();
+    __syncthreads();
+#pragma unroll 1
+    for (int b = threadIdx.x; b < MS * S0 * TX; b += TH) {
+        const int w = b / TX, q = w % S0;
+        cx<T>* d = sm + w / S0 * LINE;
+        Twiddles<T, R0> wq;
+        wq.load(tw, q, 1);
+        cx<T> v[1][R0];
+#pragma unroll
+        for (int r = 0; r < R0; ++r) v[0][r] = d[TL::at(q + r * S0, t)];
+        Dft<T, false, R0>::run(v[0]);
+        if (q) wq.template apply<false, 1>(v);
+#pragma unroll
+        for (int r = 0; r < R0; ++r) d[TL::at(q + r * S0, t)] = v[0][r];
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int b = threadIdx.x; b < MS * NB * TX; b += TH) {
+        const int w = b / TX, q = w % NB, n2 = q % S1, e0 = q / S1 * S0 + n2;
+        cx<T>* d = sm + w / NB * LINE;
+        Twiddles<T, R1> wq;
+        wq.load(tw, n2, R0);
+        cx<T> v[1][R1];
+#pragma unroll
+        for (int r = 0; r < R1; ++r) v[0][r] = d[TL::at(e0 + r * S1, t)];
+        Dft<T, false, R1>::run(v[0]);
+        if (n2) wq.template apply<false, 1>(v);
+#pragma unroll
+        for (int r = 0; r < R1; ++r) d[TL::at(e0 + r * S1, t)] = v[0][r];
+    }
+    __syncthreads();
+    // last forward pass, k-space operators, first inverse pass
+#pragma unroll 1
+    for (int b = threadIdx.x; b < NQ * TX; b += TH) {
+        const int q = b / TX, kq = PL::krev(q);
+        cx<T> v[MS][RL];
+#pragma unroll
+        for (int m = 0; m < MS; ++m) {
+#pragma unroll
+            for (int r = 0; r < RL; ++r) v[m][r] = sm[m * LINE + TL::at(q * RL + r, t)];
+            Dft<T, false, RL>::run(v[m]);
+        }
+#pragma unroll
+        for (int r = 0; r < RL; ++r) {
+            const int iy = kq + r * NQ;
+            const cx<T> f = fmul(imag, kex, key[iy]);
+            cx<T> u[MS];
+#pragma unroll
+            for (int m = 0; m < MS; ++m) u[m] = fmul(imag, f, cscale(v[m][r], fac[m]));
+            if (soc) soc_apply<T, MS>(imag, soc[(size_t)iy * st], u);
+#pragma unroll
+            for (int m = 0; m < MS; ++m) v[m][r] = u[m];
+        }
+#pragma unroll
+        for (int m = 0; m < MS; ++m) {
+            Dft<T, true, RL>::run(v[m]);
+#pragma unroll
+            for (int r = 0; r < RL; ++r) sm[m * LINE + TL::at(q * RL + r, t)] = v[m][r];
+        }
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int b = threadIdx.x; b < MS * NB * TX; b += TH) {
+        const int w = b / TX, q = w % NB, n2 = q % S1, e0 = q / S1 * S0 + n2;
+        cx<T>* d = sm + w / NB * LINE;
+        Twiddles<T, R1> wq;
+        wq.load(tw, n2, R0);
+        cx<T> v[1][R1];
+#pragma unroll
+        for (int r = 0; r < R1; ++r) v[0][r] = d[TL::at(e0 + r * S1, t)];
+        if (n2) wq.template apply<true, 1>(v);
+        Dft<T, true, R1>::run(v[0]);
+#pragma unroll
+        for (int r = 0; r < R1; ++r) d[TL::at(e0 + r * S1, t)] = v[0][r];
+    }
+    __syncthreads();
+    // last inverse pass, to global memory
+#pragma unroll 1
+    for (int b = threadIdx.x; b < MS * S0 * TX; b += TH) {
+        const int w = b / TX, q = w % S0, m = w / S0;
+        const cx<T>* d = sm + m * LINE;
+        Twiddles<T, R0> wq;
+        wq.load(tw, q, 1);
+        cx<T> v[1][R0];
+#pragma unroll
+        for (int r = 0; r < R0; ++r) v[0][r] = d[TL::at(q + r * S0, t)];
+        if (q) wq.template apply<true, 1>(v);
+        Dft<T, true, R0>::run(v[0]);
+        cx<T>* g = S + (size_t)m * np + (size_t)q * st + t;
+#pragma unroll
+        for (int r = 0; r < R0; ++r) g[(size_t)(r * S0) * st] = v[0][r];
+    }
+    __syncthreads();
+}
+
+// ------------------------------------------------------------ column tile, spin 2
+// F_y, pending scale + KE + SOC, F_y^-1 on TX adjacent x positions of one
+// instance by passes over the tile, with the y plan PV.
 template <typename T, int MS, int N, int TX, int TH, int PV>
 __device__ __forceinline__ void pcol_tile(const PInst& P, const StepConst& c, int x0, cx<T>* cur) {
     using CT = ColTile<N, TX>;
@@ -150,7 +291,7 @@ __device__ __forceinline__ void pcol_tile(const PInst& P, const StepConst& c, in
     cp_wait<0>();
     __syncthreads();
     const cx<T>* tw = (const cx<T>*)c.twy;
-    ct_fft<T, false, N, MS * TX, TH, CT, 0, 0, PV, kPUnroll>(cur, tw);
+    ct_fft<T, false, N, MS * TX, TH, CT, 0, 0, PV, 1>(cur, tw);
     #pragma unroll 1
     for (int p = threadIdx.x; p < N * TX; p += TH) {
         const int tt = p % TX, e = p / TX;
@@ -164,7 +305,7 @@ __device__ __forceinline__ void pcol_tile(const PInst& P, const StepConst& c, in
         for (int m = 0; m < MS; ++m) cur[(m * LPN + e + (e >> 3)) * TX + tt] = v[m];
     }
     __syncthreads();
-    ct_fft<T, true, N, MS * TX, TH, CT, 0, 0, PV, kPUnroll>(cur, tw);
+    ct_fft<T, true, N, MS * TX, TH, CT, 0, 0, PV, 1>(cur, tw);
     #pragma unroll 1
     for (int idx = threadIdx.x; idx < MS * N * TX; idx += TH) {
         const int tt = idx % TX, q = idx / TX, e = q % N, m = q / N;
@@ -209,7 +350,7 @@ __device__ __forceinline__ void prow_tile(const PInst& P, const StepConst& c, in
     __syncthreads();
     const cx<T>* twx = (const cx<T>*)c.twx;
     cx<T>* sn = snap == 1 ? (cx<T>*)P.d.psi : snap == 2 ? (cx<T>*)P.d.prev : nullptr;
-    ct_fft<T, true, N, MS * R, TH, RT, 0, 0, 0, kPUnroll>(cur, twx);
+    ct_fft<T, true, N, MS * R, TH, RT, 0, 0, 0, 1>(cur, twx);
     #pragma unroll 1
     for (int p = threadIdx.x; p < R * N; p += TH) {
         const int x = p % N, r = p / N;
@@ -233,7 +374,7 @@ __device__ __forceinline__ void prow_tile(const PInst& P, const StepConst& c, in
         }
     }
     __syncthreads();
-    ct_fft<T, false, N, MS * R, TH, RT, 0, 0, 0, kPUnroll>(cur, twx);
+    ct_fft<T, false, N, MS * R, TH, RT, 0, 0, 0, 1>(cur, twx);
     #pragma unroll 1
     for (int idx = threadIdx.x; idx < MS * R * N; idx += TH) {
         const int x = idx % N, q = idx / N, r = q % R, m = q / R;
@@ -302,12 +443,19 @@ __device__ void prow_item(const PersistArgs& a, const PInst& P, const StepConst&
 }
 
 // ---------------------------------------------------------------- kernel
+// Threads per SM that share the register file.  A block's item is a chain of
+// dependent loads, exchanges and barriers, so more blocks pay for the spills
+// of a smaller register share: 48 spin-1 instances of 128^2 to 512^2, 768
+// against 512 threads, FP32 433 -> 366 us a step, FP64 592 -> 523 us; with
+// five components the spills win (FP32 334 against 372, FP64 505 against 665).
+constexpr int persist_threads(int ms) { return ms == 3 ? 768 : 512; }
+
 // Variant <TH threads, RN values per row tile, TXB bytes per column tile
 // row, PV y plan>: the shape the autotuner picks per batch.
 #define FGPE_PSIZES(CALL) CALL(128) CALL(192) CALL(256) CALL(384) CALL(512)
 
 template <typename T, int MS, int TH, int RN, int TXB, int PV>
-__global__ void __launch_bounds__(TH, 2) k_persist(PersistArgs a) {
+__global__ void __launch_bounds__(TH, persist_threads(MS) / TH) k_persist(PersistArgs a) {
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T>* cur = (cx<T>*)smraw;
     __shared__ double red[32 * (MS + 1)];
@@ -351,7 +499,10 @@ __global__ void __launch_bounds__(TH, 2) k_persist(PersistArgs a) {
         if (col) {
             switch (c.ny) {
 #define PCOL(NN) \
-                case NN: pcol_tile<T, MS, NN, pcol_tx<T>(TXB), TH, PV>(P, c, idx * pcol_tx<T>(TXB), cur); break;
+                case NN: \
+                    if constexpr (MS == 3) pcol_regs<T, MS, NN, pcol_tx<T>(TXB), TH, typename PColPlan<NN, PV>::P>(P, c, idx * pcol_tx<T>(TXB), cur); \
+                    else pcol_tile<T, MS, NN, pcol_tx<T>(TXB), TH, PV>(P, c, idx * pcol_tx<T>(TXB), cur); \
+                    break;
                 FGPE_PSIZES(PCOL)
 #undef PCOL
                 default: break;
@@ -379,7 +530,7 @@ inline size_t persist_smem(int rn, int txb, int nmask) {
     for (int i = 0; i < 5; ++i) {
         if (!(nmask >> i & 1)) continue;
         const size_t row = (size_t)MS * prow_r(rn, ns[i]) * cpad(ns[i]) * sizeof(cx<T>);
-        const size_t col = (size_t)MS * cpad(ns[i]) * pcol_tx<T>(txb) * sizeof(cx<T>);
+        const size_t col = (size_t)MS * (MS == 3 ? ns[i] + ns[i] / 4 : cpad(ns[i])) * pcol_tx<T>(txb) * sizeof(cx<T>);
         s = std::max(s, std::max(row, col));
     }
     return s;

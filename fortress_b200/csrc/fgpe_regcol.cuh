@@ -38,15 +38,18 @@ template <int R0_, int R1_, int R2_ = 1> struct LPlan {
 
 // COLK_FWD / COLK_INV: one transform of one component's lines (3D y passes);
 // COLK_Y2D: F_y, pending scale + KE + SOC, F_y^-1 (the q2D pass);
-// COLK_Z3D: F_z, KE and SOC as one matrix per tile column, F_z^-1.
+// COLK_Z3D: F_z, KE and SOC, F_z^-1, with the SO-coupling numbers of a tile
+// column in registers.
 enum { COLK_FWD = 0, COLK_INV = 1, COLK_Y2D = 2, COLK_Z3D = 3 };
 
 template <typename T, int TX, int RL> struct RegTile {
-    // tile rows narrower than 128 bytes are padded by one row every RL, so
-    // that the strided butterflies of the last pass fall on distinct banks
+    // tile rows narrower than 128 bytes are padded by one row every RL (at
+    // least 4), so that the strided butterflies of the last pass fall on
+    // distinct banks
     static constexpr bool padded = TX * (int)sizeof(cx<T>) < 128;
-    static constexpr __host__ __device__ int rows(int n) { return padded ? n + n / RL : n; }
-    static __device__ __forceinline__ int at(int e, int t) { return (padded ? e + e / RL : e) * TX + t; }
+    static constexpr int PAD = RL < 4 ? 4 : RL;
+    static constexpr __host__ __device__ int rows(int n) { return padded ? n + n / PAD : n; }
+    static __device__ __forceinline__ int at(int e, int t) { return (padded ? e + e / PAD : e) * TX + t; }
 };
 
 template <typename T, int MS, int N, int TX, class PL, int KIND> constexpr size_t regcol_smem() {

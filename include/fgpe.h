@@ -61,7 +61,9 @@ enum { FGPE_KERNELS_AUTO = 0, FGPE_KERNELS_GENERIC = 1,
                                       shared memory, no block barriers in the
                                       transforms) where the MS lines of a row
                                       fit 16 KB, in either precision; AUTO
-                                      takes this row pass for FP64 */
+                                      takes it for FP64 spin 2, and for spin-1
+                                      lines without a register row pass, of
+                                      2048 or more rows */
        FGPE_KERNELS_BLOCK_ROW = 8  /* size-specialised kernels with the
                                       block-tiled row pass everywhere */ };
 
@@ -226,9 +228,11 @@ int fgpe_batch_mode(fgpe_batch_t *b, int mode);
  * variant >= 0 selects one, -1 keeps the current; *current (may be NULL)
  * receives the selection.  fgpe_batch_variant_shape writes the variant's
  * shape[4] = {threads per block, values per row tile, bytes of x per column
- * tile row, radix plan of the y lines (0: radix 8 first, then 4 or 2;
- * 1: 4*4 in place of a trailing 8*2; 2: plan 0 reversed; 3: a radix-16
- * pass first where it saves a pass, 128 = 16*8, 256 = 16*16, 384 = 16*8*3)}. */
+ * tile row, radix plan of the y lines}.  Plans, spin 1: 0: 8 * N/32 * 4
+ * (128 = 8*8*2); 1: 16 * N/64 * 4; 3: 128 = 8*4*4, 192 = 12*4*4, 256 =
+ * 4*16*4, 384 = 12*8*4, 512 = 16*8*4.  Spin 2: 0: radix 8 first, then 4 or 2;
+ * 1: 4*4 in place of a trailing 8*2; 3: a radix-16 pass first where it saves
+ * a pass, 128 = 16*8, 256 = 16*16, 384 = 16*8*3. */
 int fgpe_batch_variant(fgpe_batch_t *b, int variant, int *current);
 int fgpe_batch_variant_shape(int variant, int *shape);
 int fgpe_batch_variants(void);
