@@ -95,11 +95,11 @@ static int gemm_tc_args(int batch, int M, int N, int K, float alpha, const void*
         return FGPE_E_ARG;
     }
     fno::GemmTc g{M, N, K, batch, 0, alpha, beta, A, sAb, sAi, sAk, B, sBb, sBk, sBj, C, sCb, sCi, sCj, err_dev, 0, 0, 0,
-                  A1, B1, C1};
+                  A1, B1, C1, nullptr, nullptr, 1, 1, 0};
     if (batch > 1 && sAb == 0 && sBb != 0 && !a_bf16) {
         // C^T = B^T A^T: the shared A becomes the B operand
         g = fno::GemmTc{N, M, K, batch, 0, alpha, beta, B, sBb, sBj, sBk, (const float*)A, 0, sAk, sAi,
-                        C, sCb, sCj, sCi, err_dev, 0, 0, 0, B1, (const float*)A1, C1};
+                        C, sCb, sCj, sCi, err_dev, 0, 0, 0, B1, (const float*)A1, C1, nullptr, nullptr, 1, 1, 0};
     }
     g.fold = batch > 1 && g.sBb == 0;
     // float4 operand reads where the unit-stride runs start on 16-byte boundaries
@@ -141,6 +141,21 @@ int fno_gemm_tc2(int batch, int M, int N, int K, float alpha, const float* A0, c
     fgpe::set_last_error("a pair of products shares its output, or its batched operand");
     return FGPE_E_ARG;
 }
+int fno_gemm_tc2_act(int batch, int M, int N, int K, float alpha, const float* A0, const float* A1, long long sAb, long long sAi,
+                     long long sAk, const float* B0, const float* B1, long long sBb, long long sBk, long long sBj, float beta,
+                     float* C, long long sCb, long long sCi, long long sCj, const float* bias, long long nch, long long S,
+                     int act, float* H, int* err_dev, void* stream) {
+    if (!A1 || !B1 || !H) { fgpe::set_last_error("null argument"); return FGPE_E_ARG; }
+    if (nch <= 0 || S <= 0) { fgpe::set_last_error("empty channels"); return FGPE_E_ARG; }
+    fno::GemmTc g;
+    const int rc = gemm_tc_args(batch, M, N, K, alpha, A0, A1, 0, sAb, sAi, sAk, B0, B1, sBb, sBk, sBj, beta, C, C, sCb, sCi,
+                                sCj, err_dev, &g);
+    if (rc) return rc;
+    g.bias = bias; g.H = H; g.nch = nch; g.S = S; g.act = act;
+    g.cvec = g.cvec && ((uintptr_t)H & 15) == 0;
+    return gemm_tc_pair_width<fno::PAIR_SUM>(g, (cudaStream_t)stream);
+}
+
 int fno_bias_act(float* z, float* h, const float* bias, long long C, long long S, long long n, int act, void* stream) {
     const int vec = S % 4 == 0 && n % 4 == 0 && (((uintptr_t)z | (uintptr_t)h) & 15) == 0;
     fno::k_bias_act<<<fno_grid(vec ? n / 4 : n), 256, 0, (cudaStream_t)stream>>>(z, h, bias, C, S, n, act, vec);

@@ -32,6 +32,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fno_kernels.cuh"
+
 namespace fno {
 
 struct GemmTc {
@@ -52,6 +54,12 @@ struct GemmTc {
     const void* A1;
     const float* B1;
     float* C1;
+    // sums only, H not null: the result takes its channel's bias and its
+    // activation goes to H (offsets as C; channel: offset / S modulo nch)
+    const float* bias;
+    float* H;
+    long long nch, S;
+    int act;
 };
 
 // Pairs: the real and imaginary halves of a spectral stage as one launch, each
@@ -110,7 +118,8 @@ template <int GN> __device__ __forceinline__ int b_off(int k, int n) {
 }
 // element (k, n) of a K-major B slice (operands contiguous along K: four
 // consecutive k are one 8-byte store, where the N-major form took four stores
-// of one element: the 128 x 32 weight gradient of 2^18 points 102 -> 93 us)
+// of one element: the 128 x 32 weight gradient of 2^18 points 102 -> 93 us, then
+// 71 us with the rows' order of slot())
 template <int GN> __device__ __forceinline__ int bk_off(int k, int n) {
     return (((k >> 3) * (GN / 8) + (n >> 3)) << 7) + ((n & 7) << 4) + ((k & 7) << 1);
 }
@@ -155,8 +164,20 @@ __device__ __forceinline__ int wait_phase(uint32_t bar, uint32_t parity) {
 }
 }  // namespace gtc
 
+// Row and K position of vector e of a K-contiguous operand of `rows` rows (of
+// FULL in most tiles): four vectors of a row, then the next row, then the next
+// 16 of K.  With a row's vectors on consecutive threads, eight of them met in
+// one bank (weight gradients of 2^18 points: 128 x 32 93 -> 71 us, 6 x 128
+// 143 -> 118 us).
+template <int FULL> __device__ __forceinline__ void slot(int e, int rows, int& row, int& k) {
+    const int q = e >> 2;
+    const int kb = rows == FULL ? q / FULL : q / rows;
+    row = q - kb * rows;
+    k = (kb * 4 + (e & 3)) * 4;
+}
+
 template <typename TA, int GN, int PAIR>
-__global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
+__global__ void __launch_bounds__(128, 4) k_gemm_tc(GemmTc g) {
     using namespace gtc;
     using bf16 = __nv_bfloat16;
     constexpr bool A_SPLIT = sizeof(TA) == 4;
@@ -231,15 +252,17 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
             const int kx = min(KC, (g.K - k0 + 15) / 16 * 16);
             const int kx4 = kx / 4;
             if (A_SPLIT && g.avec) {
-                // A rows as float4 along K: 16 consecutive threads read one
-                // row's 256-byte slice; 8 vectors in flight per thread
+                // A rows as float4 along K, four consecutive threads in one row
+                // and eight rows per warp (slot): the cores' stores then fall
+                // on distinct banks but for pairs; 8 vectors in flight per
+                // thread
 #pragma unroll 1
                 for (int e0 = 0; e0 < mv * kx4; e0 += 128 * 8) {
                     float4 v[8];
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const int e = min(e0 + tid + j * 128, mv * kx4 - 1);
-                        const int m = e / kx4, kq = (e % kx4) * 4;
+                        int m, kq;
+                        slot<TM>(min(e0 + tid + j * 128, mv * kx4 - 1), mv, m, kq);
                         const long long oa = rowA[m];
                         const float* src = (const float*)A + oa + k0 + kq;
                         if (oa >= 0 && k0 + kq + 3 < g.K) {
@@ -255,7 +278,8 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
                     for (int j = 0; j < 8; ++j) {
                         const int e = e0 + tid + j * 128;
                         if (e < mv * kx4) {
-                            const int m = e / kx4, kq = (e % kx4) * 4;
+                            int m, kq;
+                            slot<TM>(e, mv, m, kq);
                             put4(sAh, sAl, a_off(m, kq), v[j]);
                         }
                     }
@@ -309,8 +333,8 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
                         const int e = e0 + tid + j * 128;
                         v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
                         if (e < NV) {
-                            const int k = nvec ? e / (GN / 4) : (e % kx4) * 4;
-                            const int n = nvec ? (e % (GN / 4)) * 4 : e / kx4;
+                            int k = e / (GN / 4), n = (e % (GN / 4)) * 4;
+                            if (!nvec) slot<GN>(e, GN, n, k);
                             const float* src = B + bofs + (long long)(k0 + k) * g.sBk + (long long)(n0 + n) * g.sBj;
                             const int lim = nvec ? (k0 + k < g.K ? g.N - (n0 + n) : 0) : (n0 + n < g.N ? g.K - (k0 + k) : 0);
                             // the vector runs along the unit-stride index
@@ -331,7 +355,8 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
                                 const int k = e / (GN / 4), nq = (e % (GN / 4)) * 4;
                                 put4(bh, bl, b_off<GN>(k, nq), v[j]);
                             } else {
-                                const int kq = (e % kx4) * 4, n = e / kx4;
+                                int kq, n;
+                                slot<GN>(e, GN, n, kq);
                                 put4(bh, bl, bk_off<GN>(kq, n), v[j]);
                             }
                         }
@@ -419,7 +444,10 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
                     : "r"(taddr + (uint32_t)GN));
             }
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            const bool onto = PAIR == PAIR_SUM && g.H != nullptr;
             if (oc >= 0) {
+                float* hrow = onto ? g.H + oc + (long long)nb * g.sCj : nullptr;
+                const float bias = onto && g.bias ? g.bias[oc / g.S % g.nch] : 0.f;
                 float* crow = (sp ? g.C1 : g.C) + oc + (long long)nb * g.sCj;
                 // the second product of a sum is added as a launch of its own
                 // with beta = 1 would add it
@@ -427,6 +455,10 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
                     if (PAIR == PAIR_SUM) {
 #pragma unroll
                         for (int j = 0; j < 16; ++j) out[j] = __fadd_rn(__fmul_rn(g.alpha, __uint_as_float(r1[j])), out[j]);
+                    }
+                    if (onto) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) out[j] = __fadd_rn(out[j], bias);
                     }
                 };
                 float out[16];
@@ -450,6 +482,14 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
                     add_pair(out);
 #pragma unroll
                     for (int q = 0; q < 4; ++q) c4[q] = make_float4(out[4 * q], out[4 * q + 1], out[4 * q + 2], out[4 * q + 3]);
+                    if (onto) {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            float4 v = make_float4(out[4 * q], out[4 * q + 1], out[4 * q + 2], out[4 * q + 3]);
+                            if (g.act) v = make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
+                            ((float4*)hrow)[q] = v;
+                        }
+                    }
                 } else {
                     // all reads of C before any write, so they overlap
                     if (g.beta != 0.f) {
@@ -463,6 +503,11 @@ __global__ void __launch_bounds__(128, 1) k_gemm_tc(GemmTc g) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j)
                         if (nb + j < g.N) crow[(long long)j * g.sCj] = out[j];
+                    if (onto) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            if (nb + j < g.N) hrow[(long long)j * g.sCj] = g.act ? gelu_f(out[j]) : out[j];
+                    }
                 }
             }
         }

@@ -38,7 +38,7 @@ from . import _abi
 
 FNO_EXPORTS = ("fno_gemm", "fno_bias_act", "fno_act_bwd", "fno_channel_sum", "fno_axpy", "fno_mse",
                "fno_adam", "fno_to_bf16", "fno_rbig_build", "fno_rbig_fold", "fno_dense_tc", "fno_gemm_tc",
-               "fno_gemm_tc2")
+               "fno_gemm_tc2", "fno_gemm_tc2_act")
 
 _L = None
 
@@ -61,6 +61,8 @@ def lib():
         "fno_rbig_build": [vp, vp, vp, ll, ip, ip, vp],
         "fno_rbig_fold": [vp, vp, vp, ll, ip, ip, vp],
         "fno_dense_tc": [vp, ip, vp, vp, vp, vp, ip, ip, ll, ip, vp, vp],
+        "fno_gemm_tc2_act": [ip, ip, ip, ip, fl, vp, vp, ll, ll, ll, vp, vp, ll, ll, ll, fl, vp, ll, ll, ll, vp, ll, ll, ip, vp,
+                             vp, vp],
         "fno_gemm_tc2": [ip, ip, ip, ip, fl, vp, vp, ll, ll, ll, vp, vp, ll, ll, ll, fl, vp, vp, ll, ll, ll, vp, vp],
         "fno_gemm_tc": [ip, ip, ip, ip, fl, vp, ip, ll, ll, ll, vp, ll, ll, ll, fl, vp, ll, ll, ll, vp, vp],
     }
@@ -301,8 +303,9 @@ class FNO:
             "bias_act")
 
     # ----------------------------------------------------------- spectral
-    def spectral(self, l, h, z):
-        """z[O][B][n][n] += K_l h (h [C][B][n][n])."""
+    def spectral(self, l, h, z, onto=None):
+        """z[O][B][n][n] += K_l h (h [C][B][n][n]).  onto = (hout, bias, act):
+        then z += bias and hout = act(z)."""
         B, W, n, NM, NA = self.B, self.W, self.n, self.NM, self.NA
         CB, OB, nm = W * B, W * B, NA * NM
         T, Hm, Gm, U = self.T, self.Hm[l], self.Gm, self.U
@@ -318,9 +321,18 @@ class FNO:
         # U[z4][p][i][k] = sum_q ExA_q G_q
         self.gemm2(OB, 2 * n, NM, NA, ExA, (0, NA, 1), [(Gm, 0), (Gm, OB)], (1, NM * 2 * OB, 2 * OB),
                    [(U, 0)] * 2, (2 * n * NM, NM, 1))
-        # z_z4 += sum_p U_p EywT_p / n^2
+        # z_z4 += sum_p U_p EywT_p / n^2, with the layer's bias and activation
+        if self.tensor_cores and onto is not None:
+            hout, bias, act = onto
+            _ck(self.L.fno_gemm_tc2_act(OB, n, n, NM, 1.0 / (n * n), self._p(U), self._p(U, n * NM), 2 * n * NM, NM, 1,
+                                        self._p(self.EywT[0]), self._p(self.EywT[1]), 0, n, 1, 1.0, self._p(z), n * n, n, 1,
+                                        self._p(bias), W, B * n * n, int(act), self._p(hout), self._p(self.tc_err),
+                                        self._st()), "gemm_tc2_act")
+            return
         self.gemm2(OB, n, n, NM, [(U, 0), (U, n * NM)], (2 * n * NM, NM, 1), EywT, (0, n, 1), [(z, 0)] * 2, (n * n, n, 1),
                    alpha=1.0 / (n * n), beta=1.0)
+        if onto is not None:
+            self.bias_act(z, onto[0], onto[1], W, onto[2])
 
     def spectral_bwd(self, l, dz, dh):
         """dh += K_l^T dz; gradients of Rr_l, Ri_l."""
@@ -359,9 +371,7 @@ class FNO:
         for l in range(self.layers):
             z = self.zs[l]
             self.pointwise(f"W{l}", self.h[l], z, W, W)
-            self.spectral(l, self.h[l], z)
-            last = l == self.layers - 1
-            self.bias_act(z, self.h[l + 1], self.p[f"b{l}"], W, not last)
+            self.spectral(l, self.h[l], z, onto=(self.h[l + 1], self.p[f"b{l}"], l < self.layers - 1))
         self.pointwise("Q1", self.h[-1], self.u, self.hidden, W, bias=self.p["c1"], act_out=self.q, act=True)
         self.pointwise("Q2", self.q, self.out, self.cout, self.hidden, bias=self.p["c2"])
         return self.out
@@ -406,15 +416,13 @@ class FNO:
         self._wgrad("Q1", self.dq, self.h[-1], hid, W)
         self._dinput("Q1", self.dq, self.dh, hid, W)
         for l in reversed(range(self.layers)):
+            dz = self.dz if l < self.layers - 1 else self.dh     # the last layer has no activation
             if l < self.layers - 1:
-                _ck(self.L.fno_act_bwd(self._p(self.dz), self._p(self.dh), self._p(self.zs[l]), n_all(self.dz),
-                                       self._st()), "act")
-            else:
-                self.dz.copy_(self.dh)
-            self._bgrad(f"b{l}", self.dz, W)
-            self._wgrad(f"W{l}", self.dz, self.h[l], W, W)
-            self._dinput(f"W{l}", self.dz, self.dh2, W, W)
-            self.spectral_bwd(l, self.dz, self.dh2)
+                _ck(self.L.fno_act_bwd(self._p(dz), self._p(self.dh), self._p(self.zs[l]), n_all(dz), self._st()), "act")
+            self._bgrad(f"b{l}", dz, W)
+            self._wgrad(f"W{l}", dz, self.h[l], W, W)
+            self._dinput(f"W{l}", dz, self.dh2, W, W)
+            self.spectral_bwd(l, dz, self.dh2)
             self.dh, self.dh2 = self.dh2, self.dh
         self._bgrad("bP", self.dh, W)
         self._wgrad("P", self.dh, self.a, W, self.cin)

@@ -41,6 +41,14 @@ int fno_gemm_tc2(int batch, int M, int N, int K, float alpha, const float *A0, c
                  long long sAi, long long sAk, const float *B0, const float *B1, long long sBb, long long sBk,
                  long long sBj, float beta, float *C0, float *C1, long long sCb, long long sCi, long long sCj,
                  int *err_dev, void *stream);
+/* The sum form of fno_gemm_tc2 followed by fno_bias_act on its result, in one
+ * launch: C = beta C + alpha (A0 B0 + A1 B1) + bias, H = act(C) at the offsets
+ * of C.  The channel of an element is its offset / S modulo nch; a row of C
+ * (of C^T where A is the shared operand) lies in one channel. */
+int fno_gemm_tc2_act(int batch, int M, int N, int K, float alpha, const float *A0, const float *A1, long long sAb,
+                     long long sAi, long long sAk, const float *B0, const float *B1, long long sBb, long long sBk,
+                     long long sBj, float beta, float *C, long long sCb, long long sCi, long long sCj,
+                     const float *bias, long long nch, long long S, int act, float *H, int *err_dev, void *stream);
 /* z[b,c,s] += bias[c] (bias may be NULL); h = GELU(z) if act else z (h may be NULL). */
 int fno_bias_act(float *z, float *h, const float *bias, long long C, long long S, long long n, int act, void *stream);
 /* dz = dh * GELU'(z) */

@@ -84,6 +84,33 @@ def test_a_pair_that_shares_nothing_is_refused():
     assert rc != 0
 
 
+# batch, planes per channel, n (M = N), K, beta, act, offset of H in elements
+@pytest.mark.parametrize("batch,per,n,K,beta,act,off", [(12, 4, 64, 16, 1.0, 1, 0), (6, 2, 37, 9, 1.0, 1, 0), (4, 4, 20, 16, 0.0, 0, 0),
+                                                        (6, 3, 32, 16, 1.0, 1, 1), (1, 1, 1, 1, 1.0, 1, 0)])
+def test_pair_with_bias_and_activation_is_the_two_passes(batch, per, n, K, beta, act, off):
+    from fortress_b200 import fno as FN
+    L = FN.lib()
+    gen = torch.Generator("cuda").manual_seed(n * 7 + K)
+    A = [torch.randn(batch * n * K, device="cuda", generator=gen) for _ in range(2)]
+    B = [torch.randn(K * n, device="cuda", generator=gen) for _ in range(2)]
+    C = torch.randn(batch * n * n, device="cuda", generator=gen)
+    bias = torch.randn(batch // per, device="cuda", generator=gen)
+    H, err = torch.zeros(C.numel() + off, device="cuda")[off:], torch.zeros(1, dtype=torch.int32, device="cuda")
+    want, wanth = C.clone(), torch.zeros_like(C)
+    sA, sB, sC, S = (n * K, K, 1), (0, n, 1), (n * n, n, 1), per * n * n
+    assert 0 == L.fno_gemm_tc2(batch, n, n, K, 0.25, _p(A[0]), _p(A[1]), *sA, _p(B[0]), _p(B[1]), *sB, beta, _p(want),
+                               _p(want), *sC, _p(err), None)
+    assert 0 == L.fno_bias_act(_p(want), _p(wanth), _p(bias), batch // per, S, want.numel(), act, None)
+    assert 0 == L.fno_gemm_tc2_act(batch, n, n, K, 0.25, _p(A[0]), _p(A[1]), *sA, _p(B[0]), _p(B[1]), *sB, beta, _p(C), *sC,
+                                   _p(bias), batch // per, S, act, _p(H), _p(err), None)
+    torch.cuda.synchronize()
+    assert err.item() == 0
+    # the same operations in the same order; the activation is compiled twice
+    # (products may fuse differently): a few units of 2^-24 of values up to 64
+    assert torch.equal(C, want)
+    assert (H - wanth).abs().max().item() <= (0.0 if act == 0 else 2.0 ** -24 * 64 * 8)
+
+
 @pytest.mark.parametrize("B,C,S,off", [
     (1, 1, 1, 0), (7, 33, 1, 0), (300, 1000, 1, 0),          # S = 1: channels past a block, batch not a multiple of 8
     (1, 3, 2, 0), (2, 32, 37, 0), (3, 5, 4096, 0),           # fewer points than blocks, ragged and full slices
