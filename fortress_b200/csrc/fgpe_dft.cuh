@@ -96,15 +96,18 @@ template <typename T, bool INV> struct Dft<T, INV, 24> : DftAB<T, INV, 3, 8> {};
 template <typename T, bool INV> struct Dft<T, INV, 32> : DftAB<T, INV, 4, 8> {};
 
 // The twiddles w^1..w^(R-1) a thread applies, w = tw[j * step].  FP32 loads
-// every power (the rounding of products would show up there); FP64 loads w
-// and forms the powers by products, as w^(r mod 8) w^(8 (r div 8)), so that
-// few of them are live at a time.
+// every power (the rounding of products would show up there).  FP64 up to
+// radix 8 loads w and forms the powers by products; above, it loads w, w^4
+// and w^16 and forms w^(r mod 4) w^(4 (r div 4)), so that few powers are live
+// at a time and none is far from the table: powers of w alone doubled the rms
+// error of a 512-point transform (32 * 16: 6.1 units of 2^-53 against 3.1
+// with radix 8; this way 2.2).
 template <typename T, int R> struct Twiddles {
-    static constexpr int NW = sizeof(T) == 4 ? R : 2;
-    cx<T> w[NW];
+    static constexpr int NW = sizeof(T) == 4 ? R : R <= 8 ? 2 : R <= 16 ? 3 : 4;
+    cx<T> w[NW];        // FP64: w, w^4, w^16
     __device__ __forceinline__ void load(const cx<T>* __restrict__ tw, int j, int step) {
 #pragma unroll
-        for (int r = 1; r < NW; ++r) w[r] = tw[j * step * r];
+        for (int r = 1; r < NW; ++r) w[r] = tw[j * step * (sizeof(T) == 4 ? r : r == 1 ? 1 : r == 2 ? 4 : 16)];
     }
     // v[m][r] *= w^r (conjugate for the inverse)
     template <bool INV, int CNT> __device__ __forceinline__ void apply(cx<T> (&v)[CNT][R]) const {
@@ -115,7 +118,7 @@ template <typename T, int R> struct Twiddles {
 #pragma unroll
                 for (int m = 0; m < CNT; ++m) v[m][r] = mul(v[m][r], w[r]);
         } else {
-            constexpr int LOW = R < 8 ? R : 8;
+            constexpr int LOW = R <= 8 ? R : 4;
             cx<T> b[LOW];
             b[1] = w[1];
 #pragma unroll
@@ -125,13 +128,13 @@ template <typename T, int R> struct Twiddles {
 #pragma unroll
                 for (int m = 0; m < CNT; ++m) v[m][r] = mul(v[m][r], b[r]);
             if constexpr (R > 8) {
-                const cx<T> w8 = cmul(b[4], b[4]);
-                cx<T> g = w8;
+                cx<T> g = w[2];
 #pragma unroll
-                for (int h = 8; h < R; h += 8) {
-                    if (h > 8) g = cmul(g, w8);
+                for (int h = 4; h < R; h += 4) {
+                    if (h == 16) g = w[NW - 1];
+                    else if (h > 4) g = cmul(g, w[2]);
 #pragma unroll
-                    for (int r = h; r < h + 8 && r < R; ++r) {
+                    for (int r = h; r < h + 4 && r < R; ++r) {
                         const cx<T> x = r == h ? g : cmul(g, b[r - h]);
 #pragma unroll
                         for (int m = 0; m < CNT; ++m) v[m][r] = mul(v[m][r], x);
@@ -141,5 +144,50 @@ template <typename T, int R> struct Twiddles {
         }
     }
 };
+
+// -------------------------------------------- radix plans of column lines
+// Radix plan of a column line: two passes (R2 = 1) or three.
+template <int R0_, int R1_, int R2_ = 1> struct LPlan {
+    static constexpr int R0 = R0_, R1 = R1_, R2 = R2_;
+    static constexpr int N = R0 * R1 * R2;
+    static constexpr bool three = R2 > 1;
+    static constexpr int RL = three ? R2 : R1;      // radix of the last pass (contiguous positions)
+    // frequency of position q*RL is krev(q); position q*RL + r adds r*N/RL
+    static __host__ __device__ __forceinline__ int krev(int q) { return three ? q / R1 + R0 * (q % R1) : q; }
+};
+
+// COLK_FWD / COLK_INV: one transform of one component's lines (3D y passes);
+// COLK_Y2D: F_y, pending scale + KE + SOC, F_y^-1 (the q2D pass);
+// COLK_Z3D: F_z, KE and SOC, F_z^-1, with the SO-coupling numbers of a tile
+// column in registers.
+enum { COLK_FWD = 0, COLK_INV = 1, COLK_Y2D = 2, COLK_Z3D = 3 };
+
+// Radix plans.  Single-component passes take (N/16, 16): one exchange.  The z
+// pass of a grid that fills the GPU holds MS * RL complex values per thread
+// between its transforms, so RL = 16 with three components and 8 with five.
+// The q2D pass, and the z pass of a small grid, have few tiles and are bound
+// by one tile's latency: short last radices and more threads per tile
+// (512^2 spin-1 FP32: 16 us with (8, 16, 4) and 256 threads, 27 us with
+// (32, 16) and 128).
+template <int MS, int N, int KIND, bool BIG> struct ColPlan { using P = LPlan<N / 16, 16>; };
+template <int N> struct ColPlan<5, N, COLK_Z3D, true> { using P = LPlan<N / 8, 8>; };
+template <> struct ColPlan<5, 384, COLK_Z3D, true> { using P = LPlan<8, 6, 8>; };
+template <> struct ColPlan<5, 512, COLK_Z3D, true> { using P = LPlan<8, 8, 8>; };
+template <int N> struct SmallPlan { using P = LPlan<8, N / 32, 4>; };
+template <> struct SmallPlan<128> { using P = LPlan<8, 8, 2>; };
+template <int MS, int N> struct ColPlan<MS, N, COLK_Z3D, false> : SmallPlan<N> {};
+template <int N> struct ColPlan<5, N, COLK_Z3D, false> : SmallPlan<N> {};
+template <int MS, int N, bool BIG> struct ColPlan<MS, N, COLK_Y2D, BIG> : SmallPlan<N> {};
+
+// Plans of the persistent kernel's variants: 0: radix 8 first and 4 last;
+// 1: radix 16 first; 3: other splits of the first two passes.  (Passes over
+// the tile take the plans of cplan.)
+template <int N, int PV> struct PColPlan : SmallPlan<N> {};
+template <int N> struct PColPlan<N, 1> { using P = LPlan<16, N / 64, 4>; };
+template <> struct PColPlan<128, 3> { using P = LPlan<8, 4, 4>; };
+template <> struct PColPlan<192, 3> { using P = LPlan<12, 4, 4>; };
+template <> struct PColPlan<256, 3> { using P = LPlan<4, 16, 4>; };
+template <> struct PColPlan<384, 3> { using P = LPlan<12, 8, 4>; };
+template <> struct PColPlan<512, 3> { using P = LPlan<16, 8, 4>; };
 
 }  // namespace fgpe

@@ -119,17 +119,6 @@ __device__ __forceinline__ void psignal(unsigned* ctr) {
     if (threadIdx.x == 0) atomicAdd(ctr, 1u);
 }
 
-// Radix plans of the column lines in registers: 0: radix 8 first and 4 last;
-// 1: radix 16 first; 3: other splits of the first two passes.  (Passes over
-// the tile take the plans of cplan.)
-template <int N, int PV> struct PColPlan : SmallPlan<N> {};
-template <int N> struct PColPlan<N, 1> { using P = LPlan<16, N / 64, 4>; };
-template <> struct PColPlan<128, 3> { using P = LPlan<8, 4, 4>; };
-template <> struct PColPlan<192, 3> { using P = LPlan<12, 4, 4>; };
-template <> struct PColPlan<256, 3> { using P = LPlan<4, 16, 4>; };
-template <> struct PColPlan<384, 3> { using P = LPlan<12, 8, 4>; };
-template <> struct PColPlan<512, 3> { using P = LPlan<16, 8, 4>; };
-
 // ------------------------------------------------------------ column tile, spin 1
 // F_y, pending scale + KE + SOC, F_y^-1 on TX adjacent x positions of one
 // instance, in registers as the q2D pass of fgpe_regcol.cuh: five trips

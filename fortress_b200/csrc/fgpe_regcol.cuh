@@ -26,22 +26,6 @@
 
 namespace fgpe {
 
-// Radix plan of a column line: two passes (R2 = 1) or three.
-template <int R0_, int R1_, int R2_ = 1> struct LPlan {
-    static constexpr int R0 = R0_, R1 = R1_, R2 = R2_;
-    static constexpr int N = R0 * R1 * R2;
-    static constexpr bool three = R2 > 1;
-    static constexpr int RL = three ? R2 : R1;      // radix of the last pass (contiguous positions)
-    // frequency of position q*RL is krev(q); position q*RL + r adds r*N/RL
-    static __host__ __device__ __forceinline__ int krev(int q) { return three ? q / R1 + R0 * (q % R1) : q; }
-};
-
-// COLK_FWD / COLK_INV: one transform of one component's lines (3D y passes);
-// COLK_Y2D: F_y, pending scale + KE + SOC, F_y^-1 (the q2D pass);
-// COLK_Z3D: F_z, KE and SOC, F_z^-1, with the SO-coupling numbers of a tile
-// column in registers.
-enum { COLK_FWD = 0, COLK_INV = 1, COLK_Y2D = 2, COLK_Z3D = 3 };
-
 template <typename T, int TX, int RL> struct RegTile {
     // tile rows narrower than 128 bytes are padded by one row every RL (at
     // least 4), so that the strided butterflies of the last pass fall on
@@ -379,23 +363,6 @@ __global__ void __launch_bounds__(TH, MINB) k_regcol_group(const __grid_constant
 }
 
 // ------------------------------------------------------- launch shapes
-// Radix plans.  Single-component passes take (N/16, 16): one exchange.  The z
-// pass of a grid that fills the GPU holds MS * RL complex values per thread
-// between its transforms, so RL = 16 with three components and 8 with five.
-// The q2D pass, and the z pass of a small grid, have few tiles and are bound
-// by one tile's latency: short last radices and more threads per tile
-// (512^2 spin-1 FP32: 16 us with (8, 16, 4) and 256 threads, 27 us with
-// (32, 16) and 128).
-template <int MS, int N, int KIND, bool BIG> struct ColPlan { using P = LPlan<N / 16, 16>; };
-template <int N> struct ColPlan<5, N, COLK_Z3D, true> { using P = LPlan<N / 8, 8>; };
-template <> struct ColPlan<5, 384, COLK_Z3D, true> { using P = LPlan<8, 6, 8>; };
-template <> struct ColPlan<5, 512, COLK_Z3D, true> { using P = LPlan<8, 8, 8>; };
-template <int N> struct SmallPlan { using P = LPlan<8, N / 32, 4>; };
-template <> struct SmallPlan<128> { using P = LPlan<8, 8, 2>; };
-template <int MS, int N> struct ColPlan<MS, N, COLK_Z3D, false> : SmallPlan<N> {};
-template <int N> struct ColPlan<5, N, COLK_Z3D, false> : SmallPlan<N> {};
-template <int MS, int N, bool BIG> struct ColPlan<MS, N, COLK_Y2D, BIG> : SmallPlan<N> {};
-
 template <typename T, int MS, int N, int KIND, bool BIG> struct ColShape {
     using P = typename ColPlan<MS, N, KIND, BIG>::P;
     static constexpr bool KOP = KIND >= COLK_Y2D, F64 = sizeof(T) == 8;
