@@ -387,34 +387,31 @@ template <> struct A0<5> {
     }
 };
 
-// exp(-i CDT x) for |dt x| <= 1/16 by the Taylor series of sin/cos (real
+// exp(-i CDT x) - 1 for |dt x| <= 1/16 by the Taylor series of sin/cos (real
 // time) or exp (imaginary time) truncated after the x^10 term: the first
 // omitted term is below (1/16)^11/11! ~ 8e-22, under FP64 rounding.
-template <typename T> __device__ __forceinline__ cx<T> small_phase(int imag, T th) {
+template <typename T> __device__ __forceinline__ cx<T> small_phase_m1(int imag, T th) {
     const T t2 = th * th;
     if constexpr (sizeof(T) == 4) {
         // FP32: terms to th^5; the first omitted one is below
         // (1/16)^6/6! ~ 8e-11, under FP32 rounding (6e-8)
-        if (imag) {
-            const T e = (T)1 - th * ((T)1 - th * ((T)(1.0 / 2) - th * ((T)(1.0 / 6) - th * ((T)(1.0 / 24)
-                        - th * (T)(1.0 / 120)))));
-            return mk<T>(e, (T)0);
-        }
-        const T cs = (T)1 - t2 * ((T)(1.0 / 2) - t2 * (T)(1.0 / 24));
-        const T sn = th * ((T)1 - t2 * ((T)(1.0 / 6) - t2 * (T)(1.0 / 120)));
-        return mk<T>(cs, -sn);
+        if (imag)
+            return mk<T>(-th * ((T)1 - th * ((T)(1.0 / 2) - th * ((T)(1.0 / 6) - th * ((T)(1.0 / 24) - th * (T)(1.0 / 120))))),
+                         (T)0);
+        return mk<T>(-t2 * ((T)(1.0 / 2) - t2 * (T)(1.0 / 24)), -th * ((T)1 - t2 * ((T)(1.0 / 6) - t2 * (T)(1.0 / 120))));
     }
-    if (imag) {
+    if (imag)
         // exp(-th) = sum (-th)^k/k!
-        const T e = (T)1 - th * ((T)1 - th * ((T)(1.0 / 2) - th * ((T)(1.0 / 6) - th * ((T)(1.0 / 24) - th * ((T)(1.0 / 120)
-                    - th * ((T)(1.0 / 720) - th * ((T)(1.0 / 5040) - th * ((T)(1.0 / 40320) - th * ((T)(1.0 / 362880)
-                    - th * (T)(1.0 / 3628800))))))))));
-        return mk<T>(e, (T)0);
-    }
-    const T cs = (T)1 - t2 * ((T)(1.0 / 2) - t2 * ((T)(1.0 / 24) - t2 * ((T)(1.0 / 720) - t2 * ((T)(1.0 / 40320)
-                 - t2 * (T)(1.0 / 3628800)))));
-    const T sn = th * ((T)1 - t2 * ((T)(1.0 / 6) - t2 * ((T)(1.0 / 120) - t2 * ((T)(1.0 / 5040) - t2 * (T)(1.0 / 362880)))));
-    return mk<T>(cs, -sn);
+        return mk<T>(-th * ((T)1 - th * ((T)(1.0 / 2) - th * ((T)(1.0 / 6) - th * ((T)(1.0 / 24) - th * ((T)(1.0 / 120)
+                     - th * ((T)(1.0 / 720) - th * ((T)(1.0 / 5040) - th * ((T)(1.0 / 40320) - th * ((T)(1.0 / 362880)
+                     - th * (T)(1.0 / 3628800)))))))))), (T)0);
+    return mk<T>(-t2 * ((T)(1.0 / 2) - t2 * ((T)(1.0 / 24) - t2 * ((T)(1.0 / 720) - t2 * ((T)(1.0 / 40320)
+                 - t2 * (T)(1.0 / 3628800))))),
+                 -th * ((T)1 - t2 * ((T)(1.0 / 6) - t2 * ((T)(1.0 / 120) - t2 * ((T)(1.0 / 5040) - t2 * (T)(1.0 / 362880))))));
+}
+template <typename T> __device__ __forceinline__ cx<T> small_phase(int imag, T th) {
+    const cx<T> f = small_phase_m1<T>(imag, th);
+    return mk<T>((T)1 + f.x, f.y);
 }
 
 // v <- exp(-i CDT H_SO(k)) v with H_SO = A(beta) diag(L alpha) A(beta)^H,
@@ -786,20 +783,29 @@ __device__ __forceinline__ void apply_sp(const StepConst& c, cx<T> eV, cx<T>* v)
     if constexpr (MS == 3) {
         const T th0 = dt * d0;
         if (c.dim > 1 && fabs(th0) <= (T)0.0625 && dt * fabs(t1) * rho <= (T)(1.0 / 1024)) {
-            const cx<T> e0 = fmul(c.imag, eV, small_phase<T>(c.imag, th0));
+            // a factor a becomes a (1 + f) as a + a f: f is small, so the sum
+            // rounds once where a product with the rounded 1 + f would round
+            // twice, with an error that is the same on every step
+            const cx<T> f0 = small_phase_m1<T>(c.imag, th0);
+            if (c.imag) {
+                const T e0 = fma(eV.x, f0.x, eV.x);
 #pragma unroll
-            for (int m = 0; m < MS; ++m) {
-                const T th = dt * B[m];
-                if (c.imag) {
-                    T e = sizeof(T) == 4 ? (T)1 - th * ((T)1 - th * (T)0.5)
-                                         : (T)1 - th * ((T)1 - th * ((T)0.5 - th * ((T)(1.0 / 6) - th * (T)(1.0 / 24))));
-                    e *= e0.x;
-                    v[m] = mk<T>(v[m].x * e, v[m].y * e);
-                } else {
-                    const T s2 = th * th;
-                    const T cs = sizeof(T) == 4 ? (T)1 - (T)0.5 * s2 : (T)1 - s2 * ((T)0.5 - s2 * (T)(1.0 / 24));
-                    const T sn = th * ((T)1 - s2 * (T)(1.0 / 6));
-                    v[m] = cmul(cmul(e0, mk<T>(cs, -sn)), v[m]);
+                for (int m = 0; m < MS; ++m) {
+                    const T th = dt * B[m];
+                    const T f = sizeof(T) == 4 ? th * (th * (T)0.5 - (T)1)
+                                               : th * (th * ((T)0.5 - th * ((T)(1.0 / 6) - th * (T)(1.0 / 24))) - (T)1);
+                    v[m] = cscale(v[m], fma(e0, f, e0));
+                }
+            } else {
+                auto turn = [](cx<T> a, cx<T> f) {
+                    return mk<T>(a.x + fma(a.x, f.x, -a.y * f.y), a.y + fma(a.y, f.x, a.x * f.y));
+                };
+                const cx<T> e0 = turn(eV, f0);
+#pragma unroll
+                for (int m = 0; m < MS; ++m) {
+                    const T th = dt * B[m], s2 = th * th;
+                    const T fx = sizeof(T) == 4 ? (T)-0.5 * s2 : s2 * (s2 * (T)(1.0 / 24) - (T)0.5);
+                    v[m] = cmul(turn(e0, mk<T>(fx, th * (s2 * (T)(1.0 / 6) - (T)1))), v[m]);
                 }
             }
             return;
