@@ -228,35 +228,40 @@ void choose_row_pass(fgpe_t* h, int kernels) {
 }
 
 // ---------------------------------------------------------------- launches
+// Status of a launch: what its launcher returned, else what the runtime has
+// pending (kernels launched here).
+cudaError_t launched(cudaError_t e = cudaSuccess) {
+    const cudaError_t pending = cudaGetLastError();
+    return e != cudaSuccess ? e : pending;
+}
+
 template <typename T, int MS>
-void launch_row(fgpe_t* h, int mode, void* snap) {
+cudaError_t launch_row(fgpe_t* h, int mode, void* snap) {
     RowArgs a;
     a.S = h->S; a.psi = h->psi; a.snap = snap; a.part = h->part; a.counter = h->counters;
     a.info = h->info; a.rows = h->row.tile; a.mode = mode;
     ProfScope ps(h, 0);
     if constexpr (MS == 3) {
         if (h->reg_row && mode == ROW_FULL) {
-            regrow_launch<T>(h->p.nx, h->reg_row_grid, h->sc, a, h->st, use_pdl(h));
             h->launches++;
-            return;
+            return launched(regrow_launch<T>(h->p.nx, h->reg_row_grid, h->sc, a, h->st, use_pdl(h)));
         }
     }
     if (h->warp_row && mode == ROW_FULL) {
-        row_launch<T, MS>(h->p.nx, true, h->warp_row_grid, h->sc, a, h->st, use_pdl(h));
         h->launches++;
-        return;
+        return launched(row_launch<T, MS>(h->p.nx, true, h->warp_row_grid, h->sc, a, h->st, use_pdl(h)));
     }
     if (h->fast_row) {
-        row_launch<T, MS>(h->p.nx, false, h->fast_row_grid, h->sc, a, h->st, use_pdl(h));
         h->launches++;
-        return;
+        return launched(row_launch<T, MS>(h->p.nx, false, h->fast_row_grid, h->sc, a, h->st, use_pdl(h)));
     }
     k_row<T, MS><<<h->row.grid, h->row.T, h->row.smem, h->st>>>(h->sc, a);
     h->launches++;
+    return launched();
 }
 
 template <typename T, int MS>
-void launch_col(fgpe_t* h, int axis, int flags) {
+cudaError_t launch_col(fgpe_t* h, int axis, int flags) {
     ColArgs a;
     a.S = h->S;
     a.tw = axis == 1 ? h->sc.twy : h->sc.twz;
@@ -277,16 +282,16 @@ void launch_col(fgpe_t* h, int axis, int flags) {
     ProfScope ps(h, axis);
     if (step && h->fast_col[axis]) {
         const int kind = h->p.dim == 2 ? 2 : axis == 2 ? 3 : (flags & COL_FWD) ? 0 : 1;
-        regcol_launch<T, MS>(a.n, kind, h->reg_wide[kind], h->reg_grid[kind], h->sc, a, h->st, use_pdl(h));
         h->launches++;
-        return;
+        return launched(regcol_launch<T, MS>(a.n, kind, h->reg_wide[kind], h->reg_grid[kind], h->sc, a, h->st, use_pdl(h)));
     }
     k_col<T, MS><<<h->col[axis].grid, h->col[axis].T, h->col[axis].smem, h->st>>>(h->sc, a);
     h->launches++;
+    return launched();
 }
 
 template <typename T, int MS>
-void launch_obs(fgpe_t* h, int mode, bool with_prev) {
+cudaError_t launch_obs(fgpe_t* h, int mode, bool with_prev) {
     ObsArgs a;
     a.psi = h->psi; a.prev = with_prev ? h->prev : nullptr;
     a.info = h->info; a.info_prev = h->info_prev;
@@ -294,24 +299,27 @@ void launch_obs(fgpe_t* h, int mode, bool with_prev) {
     a.dx = h->p.dx; a.dy = h->p.dy; a.dz = h->p.dz; a.mode = mode;
     k_obs<T, MS><<<h->obsl.grid, 256, 0, h->st>>>(h->sc, a);
     h->launches++;
+    return launched();
 }
 
 template <typename T, int MS>
-void launch_point(fgpe_t* h, int op, double factor) {
+cudaError_t launch_point(fgpe_t* h, int op, double factor) {
     PointArgs a; a.psi = h->psi; a.op = op; a.factor = factor;
     const long long blocks = std::min<long long>((h->npts + 255) / 256, 148LL * 16);
     k_pointwise_op<T, MS><<<(unsigned)blocks, 256, 0, h->st>>>(h->sc, a);
     h->launches++;
+    return launched();
 }
 
 template <typename T, int MS>
-void launch_1d(fgpe_t* h, int nsteps, void* snap_prev) {
+cudaError_t launch_1d(fgpe_t* h, int nsteps, void* snap_prev) {
     OneDArgs a;
     a.psi = h->psi; a.snap_prev = snap_prev; a.info = h->info; a.info_prev = h->info_prev;
     a.nsteps = nsteps;
     ProfScope ps(h, 3);
     k_1d<T, MS><<<1, h->k1.T, h->k1.smem, h->st>>>(h->sc, a);
     h->launches++;
+    return launched();
 }
 
 template <typename T, int MS>
@@ -325,21 +333,23 @@ Split1dArgs split_args(fgpe_t* h, int mode, void* snap) {
 }
 
 template <typename T, int MS>
-void launch_r1d(fgpe_t* h) {
+cudaError_t launch_r1d(fgpe_t* h) {
     Split1dArgs a = split_args<T, MS>(h, C1D_FULL, nullptr);
     a.tile = h->r1d.tile;
     ProfScope ps(h, 0);
     k_r1d<T, MS><<<h->r1d.grid, h->r1d.T, h->r1d.smem, h->st>>>(h->sc, a);
     h->launches++;
+    return launched();
 }
 
 template <typename T, int MS>
-void launch_c1d(fgpe_t* h, int mode, void* snap) {
+cudaError_t launch_c1d(fgpe_t* h, int mode, void* snap) {
     Split1dArgs a = split_args<T, MS>(h, mode, snap);
     a.tile = h->c1d.tile;
     ProfScope ps(h, 1);
     k_c1d<T, MS><<<h->c1d.grid, h->c1d.T, h->c1d.smem, h->st>>>(h->sc, a);
     h->launches++;
+    return launched();
 }
 
 // The cluster form of the 1D split when n1 and n2 divide over the cluster,
@@ -367,7 +377,7 @@ void setup_cl1d(fgpe_t* h) {
 
 // All nsteps of a call in one launch of the cluster kernel.
 template <typename T, int MS>
-void launch_cl1d(fgpe_t* h, int nsteps, void* snap_last, void* snap_prev) {
+cudaError_t launch_cl1d(fgpe_t* h, int nsteps, void* snap_last, void* snap_prev) {
     Cluster1dArgs a;
     a.S = h->S; a.snap_last = snap_last; a.snap_prev = snap_prev;
     a.twn = h->twn; a.tw1 = h->tw1; a.tw2 = h->tw2;
@@ -376,6 +386,7 @@ void launch_cl1d(fgpe_t* h, int nsteps, void* snap_last, void* snap_prev) {
     ProfScope ps(h, 3);
     k_cl1d<T, MS><<<CL1D, 256, h->cl1d_smem, h->st>>>(h->sc, a);
     h->launches++;
+    return launched();
 }
 
 // Kernel launches of one step call of k whole steps on h.
@@ -384,15 +395,10 @@ static long long step_launches(const fgpe_t* h, int k) {
     return (long long)k * (h->p.dim == 1 ? (h->split1d ? 2 : 1) : (h->p.dim == 2 ? 2 : 4));
 }
 
-// dispatch on (precision, spin)
-#define DISPATCH(h, FN, ...)                                                  \
-    do {                                                                      \
-        if ((h)->fp32) {                                                      \
-            if ((h)->ms == 3) FN<float, 3>(__VA_ARGS__); else FN<float, 5>(__VA_ARGS__);   \
-        } else {                                                              \
-            if ((h)->ms == 3) FN<double, 3>(__VA_ARGS__); else FN<double, 5>(__VA_ARGS__); \
-        }                                                                     \
-    } while (0)
+// FN of the handle's (precision, spin); of a launch_*, the status
+#define DISPATCH(h, FN, ...)                                                                    \
+    ((h)->fp32 ? ((h)->ms == 3 ? FN<float, 3>(__VA_ARGS__) : FN<float, 5>(__VA_ARGS__))          \
+               : ((h)->ms == 3 ? FN<double, 3>(__VA_ARGS__) : FN<double, 5>(__VA_ARGS__)))
 
 template <typename T>
 __global__ void k_export(const T* psi, double* out, long long n2, long long per2, const double* info) {
@@ -447,18 +453,17 @@ __global__ void k_permute(StepConst c, const cx<T>* src, cx<T>* dst, int to_natu
 }
 
 template <typename T, int MS>
-void launch_permute(fgpe_t* h, int to_natural) {
+cudaError_t launch_permute(fgpe_t* h, int to_natural) {
     k_permute<T, MS><<<148 * 8, 256, 0, h->st>>>(h->sc, (const cx<T>*)h->psi, (cx<T>*)h->S, to_natural);
     h->launches++;
     std::swap(h->psi, h->S);
+    return launched();
 }
 
 int materialize(fgpe_t* h) {
     if (h->psi_valid) return FGPE_OK;
     if (!h->S_valid) return fail(h, FGPE_E_STATE, "no state set");
-    if (h->split1d) DISPATCH(h, launch_c1d, h, C1D_INV, nullptr);
-    else DISPATCH(h, launch_row, h, ROW_INV, nullptr);
-    CK(cudaGetLastError());
+    CK(h->split1d ? DISPATCH(h, launch_c1d, h, C1D_INV, nullptr) : DISPATCH(h, launch_row, h, ROW_INV, nullptr));
     h->psi_valid = true;
     return FGPE_OK;
 }
@@ -955,8 +960,7 @@ int fgpe_step_ex(fgpe_t* h, int nsteps, int flags) {
                     sp = h->prev;
                 }
             }
-            DISPATCH(h, launch_1d, h, chunk, sp);
-            CK(cudaGetLastError());
+            CK(DISPATCH(h, launch_1d, h, chunk, sp));
             done += chunk;
         }
         h->prev_valid = true; h->psi_valid = true; h->norms_valid = true;
@@ -964,9 +968,7 @@ int fgpe_step_ex(fgpe_t* h, int nsteps, int flags) {
     }
     if (!h->S_valid) {
         if (!h->psi_valid) return fail(h, FGPE_E_STATE, "no state set");
-        if (h->split1d) DISPATCH(h, launch_c1d, h, C1D_FWD, nullptr);
-        else DISPATCH(h, launch_row, h, ROW_FWD, nullptr);
-        CK(cudaGetLastError());
+        CK(h->split1d ? DISPATCH(h, launch_c1d, h, C1D_FWD, nullptr) : DISPATCH(h, launch_row, h, ROW_FWD, nullptr));
         h->S_valid = true;
     }
     h->prev_valid = false;
@@ -983,8 +985,7 @@ int fgpe_step_ex(fgpe_t* h, int nsteps, int flags) {
         // the whole call on one cluster: one launch, no graph
         void* sl = snap ? h->psi : nullptr;
         void* sp = (snap && nsteps >= 2) ? h->prev : nullptr;
-        DISPATCH(h, launch_cl1d, h, nsteps, sl, sp);
-        CK(cudaGetLastError());
+        CK(DISPATCH(h, launch_cl1d, h, nsteps, sl, sp));
         if (sp) h->prev_valid = true;
         h->psi_valid = snap;
         h->norms_valid = true;
@@ -992,19 +993,22 @@ int fgpe_step_ex(fgpe_t* h, int nsteps, int flags) {
     }
     // the passes of one step; sn: real-space snapshot target of the step
     auto launch_step = [&](void* sn) {
+        cudaError_t e = cudaSuccess;
+        auto pass = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
         if (h->split1d) {
-            DISPATCH(h, launch_r1d, h);
-            DISPATCH(h, launch_c1d, h, C1D_FULL, sn);
-            return;
+            pass(DISPATCH(h, launch_r1d, h));
+            pass(DISPATCH(h, launch_c1d, h, C1D_FULL, sn));
+            return e;
         }
         if (h->p.dim == 2) {
-            DISPATCH(h, launch_col, h, 1, COL_SCALE | COL_FWD | COL_KOP | COL_INV | COL_STEP);
+            pass(DISPATCH(h, launch_col, h, 1, COL_SCALE | COL_FWD | COL_KOP | COL_INV | COL_STEP));
         } else {
-            DISPATCH(h, launch_col, h, 1, COL_SCALE | COL_FWD | COL_STEP);
-            DISPATCH(h, launch_col, h, 2, COL_FWD | COL_KOP | COL_INV | COL_STEP);
-            DISPATCH(h, launch_col, h, 1, COL_INV | COL_STEP);
+            pass(DISPATCH(h, launch_col, h, 1, COL_SCALE | COL_FWD | COL_STEP));
+            pass(DISPATCH(h, launch_col, h, 2, COL_FWD | COL_KOP | COL_INV | COL_STEP));
+            pass(DISPATCH(h, launch_col, h, 1, COL_INV | COL_STEP));
         }
-        DISPATCH(h, launch_row, h, ROW_FULL, sn);
+        pass(DISPATCH(h, launch_row, h, ROW_FULL, sn));
+        return e;
     };
     // bulk steps (no snapshot: all but the last two of a snapshotting call)
     // as replays of a captured graph, unless profiling or already capturing
@@ -1019,8 +1023,9 @@ int fgpe_step_ex(fgpe_t* h, int nsteps, int flags) {
                 cudaGraph_t g = nullptr;
                 cudaError_t e = cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal);
                 if (e == cudaSuccess) {
-                    for (int k = 0; k < kBulkSteps; ++k) launch_step(nullptr);
-                    e = cudaStreamEndCapture(h->st, &g);
+                    for (int k = 0; k < kBulkSteps && e == cudaSuccess; ++k) e = launch_step(nullptr);
+                    const cudaError_t end = cudaStreamEndCapture(h->st, &g);
+                    if (e == cudaSuccess) e = end;
                 }
                 if (e == cudaSuccess) e = cudaGraphInstantiate(&h->bulk, g, 0);
                 if (g) cudaGraphDestroy(g);
@@ -1045,7 +1050,7 @@ int fgpe_step_ex(fgpe_t* h, int nsteps, int flags) {
         void* sn = nullptr;
         if (snap && s == nsteps - 1) sn = h->psi;
         if (snap && s == nsteps - 2) sn = h->prev;
-        launch_step(sn);
+        CK(launch_step(sn));
         if (snap && s == nsteps - 2) {
             CK(cudaMemcpyAsync(h->info_prev, h->info, INFO_LEN * sizeof(double), cudaMemcpyDeviceToDevice, h->st));
             h->prev_valid = true;
@@ -1063,8 +1068,7 @@ int fgpe_normalize(fgpe_t* h, double* tnorm) {
     if (!h) return fail(h, FGPE_E_ARG, "null handle");
     if (!h->has_state) return fail(h, FGPE_E_STATE, "no state set");
     int r = materialize(h); if (r) return r;
-    DISPATCH(h, launch_obs, h, OBS_NORMALIZE, false);
-    CK(cudaGetLastError());
+    CK(DISPATCH(h, launch_obs, h, OBS_NORMALIZE, false));
     CK(cudaMemcpyAsync(h->h_small, h->obs, OBS_LEN * sizeof(double), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     const double tot = h->h_small[OBS_TOTAL];
@@ -1085,8 +1089,7 @@ int fgpe_norms(fgpe_t* h, double* norm) {
         return check_err(h);
     }
     int r = materialize(h); if (r) return r;
-    DISPATCH(h, launch_obs, h, OBS_NORMS, false);
-    CK(cudaGetLastError());
+    CK(DISPATCH(h, launch_obs, h, OBS_NORMS, false));
     CK(cudaMemcpyAsync(h->h_small, h->obs, OBS_LEN * sizeof(double), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     for (int m = 0; m < h->ms; ++m) norm[m] = h->h_small[OBS_NORM + m];
@@ -1097,8 +1100,7 @@ int fgpe_observables(fgpe_t* h, double* en, double* mu, double* mz, double* rms)
     if (!h) return fail(h, FGPE_E_ARG, "null handle");
     if (!h->has_state) return fail(h, FGPE_E_STATE, "no state set");
     int r = materialize(h); if (r) return r;
-    DISPATCH(h, launch_obs, h, OBS_FULL, false);
-    CK(cudaGetLastError());
+    CK(DISPATCH(h, launch_obs, h, OBS_FULL, false));
     CK(cudaMemcpyAsync(h->h_small, h->obs, OBS_LEN * sizeof(double), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     const double* o = h->h_small;
@@ -1116,8 +1118,7 @@ int fgpe_conv(fgpe_t* h, double* max_dphi) {
     if (!h || !max_dphi) return fail(h, FGPE_E_ARG, "null argument");
     if (!h->prev_valid) return fail(h, FGPE_E_STATE, "no previous-step snapshot (step with snapshots first)");
     int r = materialize(h); if (r) return r;
-    DISPATCH(h, launch_obs, h, OBS_NORMS, true);
-    CK(cudaGetLastError());
+    CK(DISPATCH(h, launch_obs, h, OBS_NORMS, true));
     CK(cudaMemcpyAsync(h->h_small, h->obs, OBS_LEN * sizeof(double), cudaMemcpyDeviceToHost, h->st));
     CK(cudaStreamSynchronize(h->st));
     *max_dphi = h->h_small[OBS_CONV];
@@ -1155,33 +1156,35 @@ int fgpe_apply_op(fgpe_t* h, int op) {
     CK(cudaMemcpyAsync(h->info + INFO_SC, ones, sizeof(ones), cudaMemcpyHostToDevice, h->st));
     if (h->split1d && (op == FGPE_OP_FFT || op == FGPE_OP_BFT))
         return fail(h, FGPE_E_ARG, "the unfused FFT/BFT need the whole 1D line in one block (this line is split)");
+    cudaError_t e = cudaSuccess;
+    auto run = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
     switch (op) {
         case FGPE_OP_FFT: {
             void* keep = h->S;
             h->S = h->psi;                                    // in place
-            DISPATCH(h, launch_row, h, ROW_FWD, nullptr);
-            if (h->p.dim >= 2) DISPATCH(h, launch_col, h, 1, COL_FWD);
-            if (h->p.dim >= 3) DISPATCH(h, launch_col, h, 2, COL_FWD);
+            run(DISPATCH(h, launch_row, h, ROW_FWD, nullptr));
+            if (h->p.dim >= 2) run(DISPATCH(h, launch_col, h, 1, COL_FWD));
+            if (h->p.dim >= 3) run(DISPATCH(h, launch_col, h, 2, COL_FWD));
             h->S = keep;
-            DISPATCH(h, launch_permute, h, 1);                // digit-reversed -> natural
+            run(DISPATCH(h, launch_permute, h, 1));                // digit-reversed -> natural
         } break;
         case FGPE_OP_BFT: {
-            DISPATCH(h, launch_permute, h, 0);                // natural -> digit-reversed
+            run(DISPATCH(h, launch_permute, h, 0));                // natural -> digit-reversed
             void* keep = h->S;
             h->S = h->psi;
-            if (h->p.dim >= 3) DISPATCH(h, launch_col, h, 2, COL_INV);
-            if (h->p.dim >= 2) DISPATCH(h, launch_col, h, 1, COL_INV);
-            DISPATCH(h, launch_row, h, ROW_INV, nullptr);     // psi <- F_x^-1[psi]/NX
+            if (h->p.dim >= 3) run(DISPATCH(h, launch_col, h, 2, COL_INV));
+            if (h->p.dim >= 2) run(DISPATCH(h, launch_col, h, 1, COL_INV));
+            run(DISPATCH(h, launch_row, h, ROW_INV, nullptr));     // psi <- F_x^-1[psi]/NX
             h->S = keep;
-            if (h->p.dim >= 2) DISPATCH(h, launch_point, h, OP_SCALE, 1.0 / ((double)h->p.ny * h->p.nz));
+            if (h->p.dim >= 2) run(DISPATCH(h, launch_point, h, OP_SCALE, 1.0 / ((double)h->p.ny * h->p.nz)));
         } break;
-        case FGPE_OP_KE: DISPATCH(h, launch_point, h, OP_KE, 0.0); break;
-        case FGPE_OP_SOC: DISPATCH(h, launch_point, h, OP_SOC, 0.0); break;
-        case FGPE_OP_SE: DISPATCH(h, launch_point, h, OP_SE, 0.0); break;
-        case FGPE_OP_SP: DISPATCH(h, launch_point, h, OP_SP, 0.0); break;
+        case FGPE_OP_KE: run(DISPATCH(h, launch_point, h, OP_KE, 0.0)); break;
+        case FGPE_OP_SOC: run(DISPATCH(h, launch_point, h, OP_SOC, 0.0)); break;
+        case FGPE_OP_SE: run(DISPATCH(h, launch_point, h, OP_SE, 0.0)); break;
+        case FGPE_OP_SP: run(DISPATCH(h, launch_point, h, OP_SP, 0.0)); break;
         default: return fail(h, FGPE_E_ARG, "unknown operator");
     }
-    CK(cudaGetLastError());
+    CK(e);
     h->psi_valid = true; h->S_valid = false; h->prev_valid = false; h->norms_valid = false;
     return FGPE_OK;
 }
@@ -1382,8 +1385,7 @@ int capture(fgpe_batch_t* b, int nsteps) {
     for (fgpe_t* h : b->inst) {
         if (!h->has_state) return bfail(b, FGPE_E_STATE, "batch instance without a state");
         if (h->p.dim >= 2 && !h->S_valid) {
-            DISPATCH(h, launch_row, h, ROW_FWD, nullptr);
-            BCK(cudaGetLastError());
+            BCK(DISPATCH(h, launch_row, h, ROW_FWD, nullptr));
             h->S_valid = true;
         }
         BCK(cudaStreamSynchronize(h->st));
@@ -1421,15 +1423,21 @@ bool group_setup(BatchGroup& g) {
     return g.ms == 3 ? group_shape<double, 3>(g.nx, g.ny, n, &g.shape) : group_shape<double, 5>(g.nx, g.ny, n, &g.shape);
 }
 // One whole step of every instance of g: the column pass, then the row pass.
-void group_step(const BatchGroup& g, int snap, cudaStream_t st) {
+cudaError_t group_step(const BatchGroup& g, int snap, cudaStream_t st) {
     const int n = (int)g.members.size();
-    if (g.fp32) {
-        if (g.ms == 3) group_launch<float, 3>(g.nx, g.ny, g.shape, g.d_desc, n, snap, st);
-        else group_launch<float, 5>(g.nx, g.ny, g.shape, g.d_desc, n, snap, st);
-    } else {
-        if (g.ms == 3) group_launch<double, 3>(g.nx, g.ny, g.shape, g.d_desc, n, snap, st);
-        else group_launch<double, 5>(g.nx, g.ny, g.shape, g.d_desc, n, snap, st);
-    }
+    return g.fp32 ? (g.ms == 3 ? group_launch<float, 3>(g.nx, g.ny, g.shape, g.d_desc, n, snap, st)
+                               : group_launch<float, 5>(g.nx, g.ny, g.shape, g.d_desc, n, snap, st))
+                  : (g.ms == 3 ? group_launch<double, 3>(g.nx, g.ny, g.shape, g.d_desc, n, snap, st)
+                               : group_launch<double, 5>(g.nx, g.ny, g.shape, g.d_desc, n, snap, st));
+}
+
+// Ends the capture on the batch's launch stream and drops what it holds.
+int drop_capture(fgpe_batch_t* b, int code, const std::string& m) {
+    cudaGraph_t junk = nullptr;
+    cudaStreamEndCapture(b->origin, &junk);
+    if (junk) cudaGraphDestroy(junk);
+    cudaGetLastError();
+    return bfail(b, code, m);
 }
 
 void free_groups(fgpe_batch_t* b) {
@@ -1506,8 +1514,7 @@ int capture_grouped(fgpe_batch_t* b, int nsteps) {
     for (fgpe_t* h : b->inst) {
         if (!h->has_state) return bfail(b, FGPE_E_STATE, "batch instance without a state");
         if (h->p.dim >= 2 && !h->S_valid) {
-            DISPATCH(h, launch_row, h, ROW_FWD, nullptr);
-            BCK(cudaGetLastError());
+            BCK(DISPATCH(h, launch_row, h, ROW_FWD, nullptr));
             h->S_valid = true;
         }
         BCK(cudaStreamSynchronize(h->st));
@@ -1525,7 +1532,11 @@ int capture_grouped(fgpe_batch_t* b, int nsteps) {
     int lane = 0;
     for (const BatchGroup& g : b->groups) {
         cudaStream_t st = b->lanes[lane++ % b->width];
-        for (int s = 0; s < nsteps; ++s) group_step(g, s == nsteps - 1 ? 1 : (s == nsteps - 2 ? 2 : 0), st);
+        for (int s = 0; s < nsteps; ++s) {
+            const cudaError_t e = group_step(g, s == nsteps - 1 ? 1 : (s == nsteps - 2 ? 2 : 0), st);
+            if (e != cudaSuccess)
+                return drop_capture(b, FGPE_E_CUDA, std::string("grouped batch launch: ") + cudaGetErrorString(e));
+        }
         for (int i : g.members) {
             fgpe_t* h = b->inst[i];
             h->S_valid = true; h->psi_valid = true; h->prev_valid = true; h->norms_valid = true;
@@ -1700,8 +1711,7 @@ int capture_persistent(fgpe_batch_t* b, int nsteps) {
     for (fgpe_t* h : b->inst) {
         if (!h->has_state) return bfail(b, FGPE_E_STATE, "batch instance without a state");
         if (h->p.dim >= 2 && !h->S_valid) {
-            DISPATCH(h, launch_row, h, ROW_FWD, nullptr);
-            BCK(cudaGetLastError());
+            BCK(DISPATCH(h, launch_row, h, ROW_FWD, nullptr));
             h->S_valid = true;
         }
         BCK(cudaStreamSynchronize(h->st));

@@ -223,7 +223,10 @@ cudaError_t group_launch(int nx, int ny, const GroupShape& g, const InstDesc* d,
     } break;
         FGPE_STEP_SIZES(C)
 #undef C
+        default: return cudaErrorInvalidValue;
     }
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
     switch (nx) {
 #define R(NN)                                                                                                     \
     case NN: {                                                                                                    \
@@ -238,6 +241,7 @@ cudaError_t group_launch(int nx, int ny, const GroupShape& g, const InstDesc* d,
     } break;
         FGPE_STEP_SIZES(R)
 #undef R
+        default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }

@@ -1,6 +1,7 @@
 """Compiles device code of the library for the host: the headers' functions
 with CUDA's qualifiers defined away."""
 import os
+import shutil
 import subprocess
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "fortress_b200", "csrc")
@@ -33,9 +34,12 @@ static inline float rsqrt(float x) { return 1.0f / sqrtf(x); }
 """
 
 
-def cuda_include():
-    home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    return os.path.join(home, "include")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+def nvcc():
+    path = shutil.which("nvcc") or os.path.join(CUDA, "bin", "nvcc")
+    return path if os.path.exists(path) else None
 
 
 def compile_probe(folder, source):
@@ -43,6 +47,6 @@ def compile_probe(folder, source):
     contraction: products and sums round one by one, on every host alike."""
     src, exe = folder / "probe.cpp", folder / "probe"
     src.write_text(PRELUDE + source)
-    subprocess.run(["g++", "-std=c++17", "-O2", "-w", "-ffp-contract=off", "-I", cuda_include(), "-I", CSRC, "-o", str(exe),
+    subprocess.run(["g++", "-std=c++17", "-O2", "-w", "-ffp-contract=off", "-I", os.path.join(CUDA, "include"), "-I", CSRC, "-o", str(exe),
                     str(src)], check=True, capture_output=True)
     return exe
