@@ -77,10 +77,14 @@ struct fgpe_s {
     bool has_fast_row = false, has_fast_col[3] = {false, false, false};
     int fast_row_grid = 0;
     // column passes with register-resident transforms, by kind (fgpe_step.h);
-    // 3D y passes leave their spectra in the order of ymap (position ->
-    // frequency), which the z pass of the step reads
+    // single transforms leave their spectra in the order of regmap[axis]
+    // (position -> frequency): the 3D y passes, for the z pass of the step, and
+    // the column passes of the unfused FFT and BFT (plain: their grids, forward
+    // and inverse, from the first such call on)
     int reg_grid[4] = {0, 0, 0, 0}, reg_wide[4] = {0, 0, 0, 0};
-    int* ymap = nullptr;
+    const int* regmap[3] = {nullptr, nullptr, nullptr};
+    int plain_grid[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+    bool plain_known = false, plain[3] = {false, false, false};
     // row pass with one warp per x row (k_row_warp), where a row fits 16 KB
     bool has_warp_row = false, warp_row = false;
     int warp_row_grid = 0;
@@ -267,7 +271,8 @@ cudaError_t launch_col(fgpe_t* h, int axis, int flags) {
     a.tw = axis == 1 ? h->sc.twy : h->sc.twz;
     a.plan = axis == 1 ? h->sc.py : h->sc.pz;
     a.info = h->info;
-    a.cfac = 1.0 / (double)h->npts;
+    const bool step = (flags & COL_STEP) != 0;
+    a.cfac = step ? 1.0 / (double)h->npts : 1.0;
     a.n = axis == 1 ? h->p.ny : h->p.nz;
     a.axis_stride = axis == 1 ? h->p.nx : (long long)h->p.nx * h->p.ny;
     a.other_stride = h->p.dim == 2 ? 0 : (axis == 1 ? (long long)h->p.nx * h->p.ny : h->p.nx);
@@ -277,13 +282,19 @@ cudaError_t launch_col(fgpe_t* h, int axis, int flags) {
     a.axis = axis;
     // the y spectra of a 3D step live only between its two y passes, so those
     // may take a radix plan of their own; the z pass reads ky through fother
-    const bool step = (flags & COL_STEP) != 0;
-    a.fother = step && h->p.dim == 3 && h->fast_col[1] ? h->ymap : h->sc.fy;
+    a.fother = step && h->p.dim == 3 && h->fast_col[1] ? h->regmap[1] : h->sc.fy;
     ProfScope ps(h, axis);
+    const int single = (flags & COL_FWD) ? 0 : 1;
     if (step && h->fast_col[axis]) {
-        const int kind = h->p.dim == 2 ? 2 : axis == 2 ? 3 : (flags & COL_FWD) ? 0 : 1;
+        const int kind = h->p.dim == 2 ? 2 : axis == 2 ? 3 : single;
         h->launches++;
         return launched(regcol_launch<T, MS>(a.n, kind, h->reg_wide[kind], h->reg_grid[kind], h->sc, a, h->st, use_pdl(h)));
+    }
+    // one transform of every line; its scale is 1 (the unfused operators fold
+    // the pending one first)
+    if (!step && h->plain[axis]) {
+        h->launches++;
+        return launched(regcol_launch<T, MS>(a.n, single, 1, h->plain_grid[axis][single], h->sc, a, h->st, use_pdl(h)));
     }
     k_col<T, MS><<<h->col[axis].grid, h->col[axis].T, h->col[axis].smem, h->st>>>(h->sc, a);
     h->launches++;
@@ -454,10 +465,33 @@ __global__ void k_permute(StepConst c, const cx<T>* src, cx<T>* dst, int to_natu
 
 template <typename T, int MS>
 cudaError_t launch_permute(fgpe_t* h, int to_natural) {
-    k_permute<T, MS><<<148 * 8, 256, 0, h->st>>>(h->sc, (const cx<T>*)h->psi, (cx<T>*)h->S, to_natural);
+    StepConst c = h->sc;
+    if (h->plain[1]) c.fy = h->regmap[1];
+    if (h->plain[2]) c.fz = h->regmap[2];
+    k_permute<T, MS><<<148 * 8, 256, 0, h->st>>>(c, (const cx<T>*)h->psi, (cx<T>*)h->S, to_natural);
     h->launches++;
     std::swap(h->psi, h->S);
     return launched();
+}
+
+// Which column axes of the unfused FFT and BFT take the register-resident
+// single transforms: compiled lengths, unless the kernel family says otherwise
+// (256^3 spin-1 FP64 FFT with the generic pass 2.85 ms, this way 1.92).
+void choose_plain_cols(fgpe_t* h) {
+    for (int a = 1; a < h->p.dim; ++a) {
+        const int n = a == 1 ? h->p.ny : h->p.nz, other = h->p.dim == 2 ? 1 : (a == 1 ? h->p.nz : h->p.ny);
+        if (!h->plain_known && h->has_fast_col[a])
+            for (int inv = 0; inv < 2; ++inv) {
+                int wide = 0;
+                h->plain_grid[a][inv] =
+                    h->fp32 ? (h->ms == 3 ? regcol_grid<float, 3>(n, inv, h->p.nx, other, &wide)
+                                          : regcol_grid<float, 5>(n, inv, h->p.nx, other, &wide))
+                            : (h->ms == 3 ? regcol_grid<double, 3>(n, inv, h->p.nx, other, &wide)
+                                          : regcol_grid<double, 5>(n, inv, h->p.nx, other, &wide));
+            }
+        h->plain[a] = h->fast_col[a] && h->plain_grid[a][0] > 0 && h->plain_grid[a][1] > 0;
+    }
+    h->plain_known = true;
 }
 
 int materialize(fgpe_t* h) {
@@ -649,9 +683,20 @@ int fgpe_create(const fgpe_params* pin, fgpe_t** out) {
             offp[a] = pm.size();
             pm.insert(pm.end(), f.begin(), f.end());
         }
+        size_t offr[3] = {0, 0, 0};
+        for (int a = 1; a < p.dim; ++a) {
+            if (!fast_size(ns[a])) continue;
+            FftPlan pl;
+            pl.n = ns[a];
+            pl.nf = regcol_radices(ns[a], pl.r);
+            const std::vector<int> f = position_map(pl);
+            offr[a] = pm.size();
+            pm.insert(pm.end(), f.begin(), f.end());
+        }
         CK(cudaMalloc(&h->pmap, pm.size() * sizeof(int)));
         CK(cudaMemcpy(h->pmap, pm.data(), pm.size() * sizeof(int), cudaMemcpyHostToDevice));
         c.fx = h->pmap + offp[0]; c.fy = h->pmap + offp[1]; c.fz = h->pmap + offp[2];
+        for (int a = 1; a < 3; ++a) if (offr[a]) h->regmap[a] = h->pmap + offr[a];
     }
     const size_t bytes = (size_t)h->npts * h->ms * h->cs;
     CK(cudaMalloc(&h->S, bytes));
@@ -793,14 +838,6 @@ int fgpe_create(const fgpe_params* pin, fgpe_t** out) {
         else if (a == 2) setup(3);
         else { setup(0); setup(1); }
         h->fast_col[a] = h->has_fast_col[a] = ok;
-        if (ok && p.dim == 3 && a == 1) {
-            FftPlan pl;
-            pl.n = p.ny;
-            pl.nf = regcol_radices(p.ny, pl.r);
-            const std::vector<int> f = position_map(pl);
-            CK(cudaMalloc(&h->ymap, f.size() * sizeof(int)));
-            CK(cudaMemcpy(h->ymap, f.data(), f.size() * sizeof(int), cudaMemcpyHostToDevice));
-        }
     }
     cudaGetLastError();   // clear any attribute/occupancy probe error
     h->obsl.grid = dim3((unsigned)((h->npts + 255) / 256));
@@ -850,7 +887,7 @@ int fgpe_destroy(fgpe_t* h) {
     if (h->bulk) cudaGraphExecDestroy(h->bulk);
     cudaFree(h->S); cudaFree(h->psi); cudaFree(h->prev); cudaFree(h->stage);
     cudaFree(h->dtab); cudaFree(h->ctab); cudaFree(h->part); cudaFree(h->info);
-    cudaFree(h->counters); cudaFree(h->pmap); cudaFree(h->ymap);
+    cudaFree(h->counters); cudaFree(h->pmap);
     if (h->h_small) cudaFreeHost(h->h_small);
     for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
     if (h->own_stream && h->st) cudaStreamDestroy(h->st);
@@ -1158,6 +1195,7 @@ int fgpe_apply_op(fgpe_t* h, int op) {
         return fail(h, FGPE_E_ARG, "the unfused FFT/BFT need the whole 1D line in one block (this line is split)");
     cudaError_t e = cudaSuccess;
     auto run = [&](cudaError_t r) { if (e == cudaSuccess) e = r; };
+    if (op == FGPE_OP_FFT || op == FGPE_OP_BFT) choose_plain_cols(h);
     switch (op) {
         case FGPE_OP_FFT: {
             void* keep = h->S;

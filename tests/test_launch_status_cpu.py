@@ -4,7 +4,8 @@ The launchers of the size-specialised passes refuse lengths without a kernel
 by their return value alone, and a failed grouped pass is known only from its
 launcher.  The library's host code is compiled with a program that asks for
 such passes (no GPU is used) and has to get the refusal back from launch_row,
-launch_col and group_step."""
+launch_col and group_step.  Where the unfused FFT and BFT may take the
+size-specialised column passes, they have to ask for them as well."""
 import os
 import subprocess
 
@@ -31,6 +32,11 @@ template <typename T, int MS> int refused() {
     if (launch_row<T, MS>(&h, ROW_FULL, nullptr) == cudaSuccess) bad |= 4;
     if (launch_col<T, MS>(&h, 1, COL_SCALE | COL_FWD | COL_STEP) == cudaSuccess) bad |= 8;
     if (launch_col<T, MS>(&h, 2, COL_FWD | COL_KOP | COL_INV | COL_STEP) == cudaSuccess) bad |= 16;
+    // single transforms outside a step go to the same launchers, not to the
+    // pass of any length
+    h.plain[1] = h.plain[2] = true;
+    if (launch_col<T, MS>(&h, 1, COL_FWD) != cudaErrorInvalidValue) bad |= 128;
+    if (launch_col<T, MS>(&h, 2, COL_INV) != cudaErrorInvalidValue) bad |= 256;
     BatchGroup g;
     g.nx = 128; g.ny = 100; g.ms = MS; g.fp32 = h.fp32;
     g.members.push_back(0);
