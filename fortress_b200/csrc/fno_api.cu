@@ -138,6 +138,14 @@ int fno_gemm_tc2(int batch, int M, int N, int K, float alpha, const float* A0, c
     const cudaStream_t st = (cudaStream_t)stream;
     if (C0 == C1) return gemm_tc_pair_width<fno::PAIR_SUM>(g, st);
     if (g.A == g.A1) return gemm_tc_pair_width<fno::PAIR_SPLIT>(g, st);
+    // a shared B that is the batched operand of a batch of one: not folded, so
+    // one launch a product
+    if (batch == 1 && sAb == 0 && sBb != 0 && B0 == B1) {
+        const int rc0 = fno_gemm_tc(batch, M, N, K, alpha, A0, 0, sAb, sAi, sAk, B0, sBb, sBk, sBj, beta, C0, sCb, sCi, sCj,
+                                    err_dev, stream);
+        return rc0 ? rc0 : fno_gemm_tc(batch, M, N, K, alpha, A1, 0, sAb, sAi, sAk, B1, sBb, sBk, sBj, beta, C1, sCb, sCi, sCj,
+                                       err_dev, stream);
+    }
     fgpe::set_last_error("a pair of products shares its output, or its batched operand");
     return FGPE_E_ARG;
 }
