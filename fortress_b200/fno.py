@@ -103,6 +103,25 @@ def input_channels(params_norm, n):
     return a
 
 
+# products that occupy the GPU: four CTAs on each of 148 SMs
+GRADIENT_PRODUCTS = 592
+
+
+def gradient_chunk(batch, points):
+    """Points per weight-gradient product: a divisor of the sample's of at most
+    about 2048, halved towards 512, where the halves stay whole float4s, while
+    the products do not fill the GPU (64 samples of 64^2: 512 products, not
+    128).  Larger problems fill it at 2048 with a quarter of the partial sums
+    (the 128 x 32 gradient of 32 samples of 256^2: 666 us with 512 points a
+    product, 602 with 2048)."""
+    chunk = points
+    while chunk > 2048 and chunk % 2 == 0:
+        chunk //= 2
+    while chunk > 512 and chunk % 8 == 0 and batch * points // chunk < GRADIENT_PRODUCTS:
+        chunk //= 2
+    return chunk
+
+
 class FNO:
     """Forward, backward and Adam on the device for one grid size n and
     batch size B.  The parameters do not depend on n (the truncated DFT
@@ -221,15 +240,9 @@ class FNO:
         self.dh2 = z(W, B * S)
         self.dz = z(W, B * S)
         self.da = z(self.cin, B * S)
-        # points per weight-gradient product: a divisor of B*S of at most ~2048,
-        # and of 512 where the halves stay whole float4s, so that there are
-        # enough products to fill the GPU (64 x 64, batch 64: 512, not 128)
-        self.chunk = S
-        while self.chunk > 2048 and self.chunk % 2 == 0:
-            self.chunk //= 2
-        while self.chunk > 512 and self.chunk % 8 == 0:
-            self.chunk //= 2
-        self.part = z((B * S // self.chunk) * max(self.hidden, W) * max(self.hidden, W, self.cin))
+        self.chunk = gradient_chunk(B, S)
+        pairs = (W * self.cin, W * W, self.hidden * W, self.cout * self.hidden)     # the weights of P, W, Q1, Q2
+        self.part = z((B * S // self.chunk) * max(pairs))
         self.dHm = z(NA * NM * 2 * W * B)
 
     def refresh_bf16(self):

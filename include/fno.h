@@ -34,9 +34,9 @@ int fno_gemm_tc(int batch, int M, int N, int K, float alpha, const void *A, int 
 /* Two products of fno_gemm_tc (FP32 operands) of one shape and one set of
  * strides in one launch (two for a shared B of a batch of one), with the
  * results of the two calls one after the other.  C0 == C1: C = alpha A0 B0 +
- * beta C, then C += alpha A1 B1.  Otherwise C0 = alpha A0 B0 + beta C0 and C1 = alpha A1 B1 + beta C1, where
- * the operand that is not shared by the batch entries (A, or B when sAb == 0
- * and sBb != 0) is the same for both. */
+ * beta C, then C += alpha A1 B1.  Otherwise C0 = alpha A0 B0 + beta C0 and
+ * C1 = alpha A1 B1 + beta C1, where the operand that is not shared by the
+ * batch entries (A, or B when sAb == 0 and sBb != 0) is the same for both. */
 int fno_gemm_tc2(int batch, int M, int N, int K, float alpha, const float *A0, const float *A1, long long sAb,
                  long long sAi, long long sAk, const float *B0, const float *B1, long long sBb, long long sBk,
                  long long sBj, float beta, float *C0, float *C1, long long sCb, long long sCi, long long sCj,
