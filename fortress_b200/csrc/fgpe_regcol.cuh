@@ -36,8 +36,9 @@ template <typename T, int TX, int RL> struct RegTile {
     static __device__ __forceinline__ int at(int e, int t) { return (padded ? e + e / PAD : e) * TX + t; }
 };
 
-template <typename T, int MS, int N, int TX, class PL, int KIND> constexpr size_t regcol_smem() {
-    return ((size_t)(KIND >= COLK_Y2D ? MS : 1) * RegTile<T, TX, PL::RL>::rows(N) * TX + (KIND == COLK_Z3D ? MS * N : 0)) * sizeof(cx<T>);
+// KEZ: the kz part of KE beside the tile (z pass)
+template <typename T, int MS, int N, int TX, class PL, int KIND, bool KEZ> constexpr size_t regcol_smem() {
+    return ((size_t)(KIND >= COLK_Y2D ? MS : 1) * RegTile<T, TX, PL::RL>::rows(N) * TX + (KEZ ? MS * N : 0)) * sizeof(cx<T>);
 }
 
 template <typename T> __device__ __forceinline__ cx<T> ld_stream(const cx<T>* p) { return __ldcg(p); }
@@ -86,7 +87,7 @@ template <typename T, int TX> struct ManyGrids {
     }
 };
 
-template <typename T, int MS, int N, int TX, int TH, class PL, int KIND, class Src>
+template <typename T, int MS, int N, int TX, int TH, class PL, int KIND, bool KEZ, class Src>
 __device__ __forceinline__ void regcol_tiles(const Src& src) {
     static_assert(PL::N == N, "plan length");
     constexpr bool KOP = KIND >= COLK_Y2D;
@@ -100,8 +101,9 @@ __device__ __forceinline__ void regcol_tiles(const Src& src) {
     constexpr int TOT0 = KOP ? MS / CNT * T0 : T0;
     extern __shared__ __align__(16) unsigned char smraw[];
     cx<T>* sm = (cx<T>*)smraw;
-    cx<T>* kez = sm + MS * LINE;                     // z pass: exp(-i CDT (kz^2 - 2 L GAMMAZ kz)) per component
     const StepConst& c0 = src.c(0);
+    // z pass: exp(-i CDT (kz^2 - 2 L GAMMAZ kz)) per component
+    const cx<T>* kez = KEZ ? sm + MS * LINE : (const cx<T>*)c0.kez;
     const long long np = c0.npts;
     const int nx = c0.nx;
     const cx<T>* tw = (const cx<T>*)src.tw();
@@ -117,8 +119,8 @@ __device__ __forceinline__ void regcol_tiles(const Src& src) {
     constexpr bool KEEPW = T0 == TH;
     Twiddles<T, R0> wq;
     if constexpr (KEEPW) wq.load(tw, (threadIdx.x / TX) % S0, 1);
-    if constexpr (KIND == COLK_Z3D) {
-        for (int i = threadIdx.x; i < MS * N; i += TH) kez[i] = ((const cx<T>*)c0.kez)[i];
+    if constexpr (KEZ) {
+        for (int i = threadIdx.x; i < MS * N; i += TH) sm[MS * LINE + i] = ((const cx<T>*)c0.kez)[i];
     }
     // passes with the operators: a butterfly's slots of the first forward and
     // of the last inverse pass belong to one thread, which refills them with
@@ -347,11 +349,11 @@ __device__ __forceinline__ void regcol_tiles(const Src& src) {
     }
 }
 
-template <typename T, int MS, int N, int TX, int TH, int MINB, class PL, int KIND>
+template <typename T, int MS, int N, int TX, int TH, int MINB, class PL, int KIND, bool KEZ>
 __global__ void __launch_bounds__(TH, MINB) k_regcol(const __grid_constant__ StepConst c, const __grid_constant__ ColArgs a) {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     const OneGrid<T, MS, TX, KIND> src(c, a);
-    regcol_tiles<T, MS, N, TX, TH, PL, KIND>(src);
+    regcol_tiles<T, MS, N, TX, TH, PL, KIND, KEZ>(src);
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
@@ -359,7 +361,7 @@ __global__ void __launch_bounds__(TH, MINB) k_regcol(const __grid_constant__ Ste
 template <typename T, int MS, int N, int TX, int TH, int MINB, class PL>
 __global__ void __launch_bounds__(TH, MINB) k_regcol_group(const __grid_constant__ GroupArgs g) {
     const ManyGrids<T, TX> src(g);
-    regcol_tiles<T, MS, N, TX, TH, PL, COLK_Y2D>(src);
+    regcol_tiles<T, MS, N, TX, TH, PL, COLK_Y2D, false>(src);
 }
 
 // ------------------------------------------------------- launch shapes
@@ -381,11 +383,19 @@ template <typename T, int MS, int N, int KIND, bool BIG> struct ColShape {
     static constexpr int PER_SM = SMALL ? (F64 || MS == 5 ? 256 : 512)
                                   : KOP ? (F64 ? 256 : 384)
                                         : (F64 ? (P::R0 > 16 ? 256 : 512) : (P::R0 > 16 ? 512 : 768));
-    static constexpr size_t SMEM = regcol_smem<T, MS, N, TX, P, KIND>();
-    static constexpr int FIT = (int)((226 * 1024) / (SMEM + 1024));
     static constexpr int MINB0 = PER_SM / TH < 1 ? 1 : PER_SM / TH;
-    static constexpr int MINB = MINB0 < FIT ? MINB0 : (FIT < 1 ? 1 : FIT);
-    static constexpr auto kernel() { return k_regcol<T, MS, N, TX, TH, MINB, P, KIND>; }
+    static constexpr int fit(size_t smem) {
+        const int f = (int)((226 * 1024) / (smem + 1024));
+        return f < 1 ? 1 : f < MINB0 ? f : MINB0;
+    }
+    // the z pass keeps the kz part of KE in shared memory, except where that
+    // costs a resident block (512-point FP64 lines: one block of 128 threads
+    // per SM, spin-2 z pass of 3072 lines 162 us against 121)
+    static constexpr bool KEZ = KIND == COLK_Z3D && fit(regcol_smem<T, MS, N, TX, P, KIND, true>()) ==
+                                                        fit(regcol_smem<T, MS, N, TX, P, KIND, false>());
+    static constexpr size_t SMEM = regcol_smem<T, MS, N, TX, P, KIND, KEZ>();
+    static constexpr int MINB = fit(SMEM);
+    static constexpr auto kernel() { return k_regcol<T, MS, N, TX, TH, MINB, P, KIND, KEZ>; }
 };
 
 }  // namespace fgpe

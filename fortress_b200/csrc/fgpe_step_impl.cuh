@@ -160,7 +160,7 @@ template <typename T, int MS, int N> struct GroupCol {
     using B = ColShape<T, MS, N, COLK_Z3D, true>;
     using P = typename B::P;
     static constexpr int TX = B::TX, TH = B::TH;
-    static constexpr size_t SMEM = regcol_smem<T, MS, N, TX, P, COLK_Y2D>();
+    static constexpr size_t SMEM = regcol_smem<T, MS, N, TX, P, COLK_Y2D, false>();
     static constexpr auto kernel() { return k_regcol_group<T, MS, N, TX, TH, B::MINB, P>; }
 };
 // Rows: k_regrow_group where k_regrow is available, else the block pass.
