@@ -374,11 +374,17 @@ template <typename T, int MS, int N, int KIND, bool BIG> struct ColShape {
     // blocks per SM.  Small tiles: 2 positions, 4 where FP32 lines are long.
     static constexpr int ROOM = F64 ? 108 * 1024 : 74 * 1024;
     static constexpr int TXB = !KOP || MS * N * 128 <= ROOM ? 128 : MS * N * 64 <= ROOM ? 64 : 32;
-    static constexpr int TX = SMALL ? (!F64 && N >= 384 ? 4 : 2) : TXB / (int)sizeof(cx<T>);
+    // q2D, five components, 192 and 256 points: one block of 256 threads takes
+    // an SM's registers, so grids of more than two x positions per SM (BIG)
+    // would run a second, nearly empty wave.  They take half the threads and
+    // two blocks (FP64), or four positions a tile (FP32): 512 x 256, us a step,
+    // one form / this one: FP64 36.6 / 33.0, FP32 30.8 / 24.7
+    static constexpr bool MANY = KIND == COLK_Y2D && BIG && MS == 5 && (N == 192 || N == 256);
+    static constexpr int TX = SMALL ? (!F64 && (N >= 384 || MANY) ? 4 : 2) : TXB / (int)sizeof(cx<T>);
     // threads: one butterfly of the operator pass (or of the wider pass of a
     // single-component kernel) each
     static constexpr int TASKS = TX * (KOP ? N / P::RL : 16);
-    static constexpr int TH = SMALL ? (N == 128 || (F64 && N >= 384) ? 128 : 256) : TASKS < 64 ? 64 : (TASKS + 31) / 32 * 32;
+    static constexpr int TH = SMALL ? (N == 128 || (F64 && (N >= 384 || MANY)) ? 128 : 256) : TASKS < 64 ? 64 : (TASKS + 31) / 32 * 32;
     // threads per SM that share the register file
     static constexpr int PER_SM = SMALL ? (F64 || MS == 5 ? 256 : 512)
                                   : KOP ? (F64 ? 256 : 384)

@@ -17,8 +17,16 @@ template <typename T, int MS, int N, int KIND> int regcol_grid_n(int nx, int n_o
     const long long tw = (long long)((nx + W::TX - 1) / W::TX) * n_other * ncomp;
     const int gw = resident_grid(W::kernel(), W::TH, W::SMEM, tw);
     *wide = 1;
-    if constexpr (KIND != COLK_Z3D) {
+    if constexpr (KIND < COLK_Y2D) {
         return gw;
+    } else if constexpr (KIND == COLK_Y2D) {
+        // the form for many tiles once the other one's take more than one wave
+        // (up to there it has more threads on each tile: 256 x 256 FP64 24.4 us)
+        const long long ts = (long long)((nx + S::TX - 1) / S::TX) * n_other;
+        const int gs = resident_grid(S::kernel(), S::TH, S::SMEM, ts);
+        if (gw > 0 && ts > gs) return gw;
+        *wide = 0;
+        return gs;
     } else {
         // the big tiles once there is one for every SM
         if (gw > 0 && tw >= 148) return gw;
@@ -46,7 +54,7 @@ template <typename T, int MS, int N, int KIND>
 cudaError_t regcol_launch_n(int wide, int grid, const StepConst& c, const ColArgs& a, cudaStream_t st, bool pdl) {
     using W = ColShape<T, MS, N, KIND, true>;
     using S = ColShape<T, MS, N, KIND, false>;
-    if constexpr (KIND != COLK_Z3D) {
+    if constexpr (KIND < COLK_Y2D) {
         return launch_step_kernel(W::kernel(), grid, W::TH, W::SMEM, c, a, st, pdl);
     } else {
         if (wide) return launch_step_kernel(W::kernel(), grid, W::TH, W::SMEM, c, a, st, pdl);
