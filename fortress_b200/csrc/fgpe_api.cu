@@ -194,9 +194,16 @@ bool use_pdl(fgpe_t* h) {
     return cs == cudaStreamCaptureStatusNone;
 }
 // Rows from which AUTO takes the one-warp-per-row passes.  Below, a warp per
-// row leaves schedulers empty and the block pass is faster (us, warp / block,
-// 256-point spin-1 rows: FP64 512 rows 19.7 / 16.8, 2048 31.1 / 35.3, 16384
-// 156 / 195; FP32 512 rows 16.8 / 15.4, 1024 18.9 / 20.9, 16384 95 / 149).
+// row leaves schedulers empty and the block pass is faster.  Us, warp / block
+// (waves of rows move single sizes by up to 7 % either way):
+//   FP64 spin 1, 256 points: 512 rows 20.8 / 16.8, 1024 22.9 / 22.9, 2048 31.3 /
+//     35.2, 8192 85 / 103; 128: 1024 20.8 / 17.7, 2048 22.9 / 22.8, 4096 31.1 /
+//     35.9; 384: 512 31.0 / 24.9, 2048 61.7 / 59.4, 8192 183 / 205
+//   FP64 spin 2 (128 points, k_row_warp): 512 rows 27.0 / 20.8, 1536 37.3 / 33.2,
+//     2048 37.3 / 41.3, 4096 62.1 / 67.9
+//   FP32 spin 1, 256 points: 512 rows 17.2 / 16.7, 1024 18.7 / 20.4, 8192 54 / 79;
+//     128: 1024 16.8 / 14.9, 2048 18.8 / 19.5; 512: 1024 31.0 / 30.6, 8192 143 /
+//     149
 constexpr long long many_rows(bool fp32) { return fp32 ? 1024 : 2048; }
 
 bool fast_size(int n) {

@@ -177,8 +177,11 @@ k_row(StepConst c, RowArgs a) {
 // A tile of TX adjacent x positions, full lines of length n along the
 // transformed axis (stride a.axis_stride), all MS components.
 // Three blocks per SM (FP32 four): the pass waits on its loads and barriers,
-// and left alone would take registers for one block fewer (96 x 80 x 120
-// spin-2 FP64: y pass 131 against 100 us).
+// and left alone would take registers for one block fewer.  Us, left alone /
+// bounded: 96 x 80 x 120 FP64 y pass spin 2 112 / 94, spin 1 77 / 66; 160^3 FP64
+// z pass spin 2 688 / 543, spin 1 464 / 373; grids with fewer tiles than blocks
+// lose a little (320 x 240 FP64 spin 2 27.5 / 29.2, spin 1 21.1 / 21.6); FP32
+// takes four either way (within 2 %).
 template <typename T, int MS>
 __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 3 : 4)
 k_col(StepConst c, ColArgs a) {

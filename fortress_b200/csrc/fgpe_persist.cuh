@@ -29,7 +29,7 @@
 // What bounds it: the latency of an item (ticket, wait, loads, exchanges), not
 // a pipe or memory, so it runs three blocks of 256 threads per SM with three
 // components, with the column lines in registers (48 instances of 128^2 to
-// 512^2 spin 1: FP32 436 -> 366 us a step, FP64 610 -> 523 us).
+// 512^2 spin 1, best variant: FP32 430 -> 351 us a step, FP64 609 -> 507 us).
 //
 // Coherence.  Data that one block writes and another reads in the same
 // launch (tiles of S, the scales and SIG in info, NORMC partials) is read
@@ -434,8 +434,8 @@ __device__ void prow_item(const PersistArgs& a, const PInst& P, const StepConst&
 // ---------------------------------------------------------------- kernel
 // Threads per SM that share the register file.  A block's item is a chain of
 // dependent loads, exchanges and barriers, so more blocks pay for the spills
-// of a smaller register share: 48 spin-1 instances of 128^2 to 512^2, 768
-// against 512 threads, FP32 433 -> 366 us a step, FP64 592 -> 523 us; with
+// of a smaller register share: 48 spin-1 instances of 128^2 to 512^2, 512
+// against 768 threads, FP32 423 -> 363 us a step, FP64 592 -> 523 us; with
 // five components the spills win (FP32 334 against 372, FP64 505 against 665).
 constexpr int persist_threads(int ms) { return ms == 3 ? 768 : 512; }
 

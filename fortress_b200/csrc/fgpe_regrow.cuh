@@ -13,10 +13,10 @@
 // of its next ones and transforms and stores the old ones meanwhile.  Nothing
 // but __syncwarp orders these steps.
 //
-// Bound by FP64 issue (256^3 spin-1: 306 FP64 operations a point, that pipe
-// 52 % busy) or, in FP32, by issue and latency (51 %).  One B200, 65536 rows of
+// Bound by FP64 issue (256^3 spin-1: about 300 FP64 operations a point, that
+// pipe half busy) or, in FP32, by issue and latency.  One B200, 65536 rows of
 // 256 spin-1 points: FP64 0.72 (k_row_warp) -> 0.56 ms, of which the shorter
-// SE and SP are 0.09; FP32 0.57 (k_row_fast) -> 0.33 ms.  Unrolling the point
+// SE and SP are 0.1; FP32 0.57 (k_row_fast) -> 0.32 ms.  Unrolling the point
 // loop (two or more points in flight, or all eight in registers) spilled and
 // was slower.
 #pragma once
@@ -164,6 +164,8 @@ __device__ __forceinline__ void regrow_rows(const Src& src, double (&acc)[MS]) {
         for (int q = 0; q < RW * MS; ++q) {
             const int rr = q / MS, m = q - rr * MS;
             const int row = src.row0(batch, RW) + rr;
+            // (axes are even, so batches of two rows are whole: the checks on
+            // nrows hold for any RW)
             if (RW > 1 && row >= nrows) break;
             const cx<T>* g = src.S(batch) + (size_t)m * np + (size_t)row * N;
 #pragma unroll

@@ -63,14 +63,19 @@ inline cudaError_t launch_step_kernel(K kern, int grid, int threads, size_t smem
     return cudaLaunchKernelEx(&cfg, kern, c, a);
 }
 
-// Resident blocks of kern over the device for ntiles tiles (0: it does not fit).
-template <class K> inline int resident_grid(K kern, int th, size_t smem, long long ntiles) {
-    int dev = 0, nsm = 0, per = 0;
+inline int sm_count() {
+    int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return nsm;
+}
+
+// Resident blocks of kern over the device for ntiles tiles (0: it does not fit).
+template <class K> inline int resident_grid(K kern, int th, size_t smem, long long ntiles) {
+    int per = 0;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, th, smem) != cudaSuccess || per < 1) return 0;
-    const long long g = (long long)per * nsm;
+    const long long g = (long long)per * sm_count();
     return (int)(ntiles < g ? ntiles : g);
 }
 

@@ -28,8 +28,12 @@ template <typename T, int MS, int N, int KIND> int regcol_grid_n(int nx, int n_o
         *wide = 0;
         return gs;
     } else {
-        // the big tiles once there is one for every SM
-        if (gw > 0 && tw >= 148) return gw;
+        // the big tiles once there is one for every SM; fewer leave SMs idle,
+        // where the small ones occupy them (us by lines, small / big: 256-point
+        // FP64 spin 1: 512 lines, 64 big tiles, 14.6 / 18.7; 1024, 128, 20.9 /
+        // 18.8; 2048 31.1 / 22.9; 128-point FP32 spin 1: 1024 12.6 / 14.6, 1536,
+        // 96, 14.7 / 14.7, 2048 16.8 / 14.7)
+        if (gw > 0 && tw >= sm_count()) return gw;
         *wide = 0;
         return resident_grid(S::kernel(), S::TH, S::SMEM, (long long)((nx + S::TX - 1) / S::TX) * n_other);
     }

@@ -218,8 +218,9 @@ int fno_dense_tc(const void* w_bf16, int transpose_w, const float* x, const floa
     }
     const size_t smem = fno::tc::dense_smem(M, K);
     static bool attr_set[64] = {false};
-    int dev = 0;
+    int dev = 0, nsm = 0;
     cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     if (dev >= 0 && dev < 64 && !attr_set[dev]) {
         cudaError_t e = cudaFuncSetAttribute(fno::k_dense_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)fno::tc::dense_smem(128, 128));
@@ -229,7 +230,7 @@ int fno_dense_tc(const void* w_bf16, int transpose_w, const float* x, const floa
     // CTAs per SM: the tensor memory's 512 columns, shared memory, eight at most
     const int fit = (int)std::min<size_t>(std::min(8, 512 / fno::tc::dense_cols(M)), (220 * 1024) / (smem + 2048));
     const long long tiles = (n + fno::tc::TP - 1) / fno::tc::TP;
-    const unsigned grid = (unsigned)std::min<long long>(tiles, 148LL * fit);
+    const unsigned grid = (unsigned)std::min<long long>(tiles, (long long)nsm * fit);
     fno::k_dense_tc<<<grid, 128, smem, (cudaStream_t)stream>>>(
         (const __nv_bfloat16*)w_bf16, transpose_w, x, bias, z, h, M, K, n, act, err_dev);
     return fno_ck(cudaGetLastError());

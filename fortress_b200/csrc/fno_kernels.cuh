@@ -340,7 +340,7 @@ k_dense_tc(const __nv_bfloat16* __restrict__ W, int transw, const float* __restr
     __shared__ __align__(8) unsigned long long mbar;
     __shared__ uint32_t tmem_slot;
     __shared__ float sbias[128];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = tid >> 5;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),

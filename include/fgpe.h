@@ -61,9 +61,10 @@ enum { FGPE_KERNELS_AUTO = 0, FGPE_KERNELS_GENERIC = 1,
                                       shared memory, no block barriers in the
                                       transforms) where the MS lines of a row
                                       fit 16 KB, in either precision; AUTO
-                                      takes it for FP64 spin 2, and for spin-1
-                                      lines without a register row pass, of
-                                      2048 or more rows */
+                                      takes it for FP64 spin 2 of 2048 or
+                                      more rows (spin 1: the register row pass,
+                                      or the block pass for FP64 512-point rows
+                                      and few rows) */
        FGPE_KERNELS_BLOCK_ROW = 8  /* size-specialised kernels with the
                                       block-tiled row pass everywhere */ };
 
