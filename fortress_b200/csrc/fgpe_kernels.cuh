@@ -883,10 +883,20 @@ __global__ void k_soc_table(StepConst c, Soc4<T>* soc) {
         const double kx = c.kx[c.fx[x]], ky = c.ky[iy];
         const double ax = c.gx * kx, ay = c.gy * ky, r2 = ax * ax + ay * ay;
         const double r = sqrt(r2), alpha = 2.0 * r;
-        Soc4<double> e = {1.0, 0.0, 1.0, c.imag ? 1.0 : 0.0};
+        const double th = c.dt * alpha;
+        Soc4<double> e = {1.0, 0.0, 1.0, 0.0};
         if (alpha > 1.0e-40) { e.cb = ax / r; e.sb = ay / r; }
-        if (c.imag) { e.p = exp(-c.dt * alpha); e.q = exp(c.dt * alpha); }
-        else { sincos(c.dt * alpha, &e.q, &e.p); e.q = -e.q; }
+        if (!c.imag) {
+            sincos(th, &e.q, &e.p);
+            e.q = -e.q;
+        } else if (c.ms == 3) {
+            const double h = sinh(0.5 * th);
+            e.p = 2.0 * h * h;               // cosh t - 1
+            e.q = -1.41421356237309504880 * sinh(th);
+        } else {
+            e.p = expm1(-th);
+            e.q = expm1(th);
+        }
         soc[t] = {(T)e.cb, (T)e.sb, (T)e.p, (T)e.q};
     }
 }

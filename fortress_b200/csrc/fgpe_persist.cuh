@@ -187,6 +187,8 @@ __device__ __forceinline__ void pcol_regs(const PInst& P, const StepConst& c, in
     }
     __syncthreads();
     // last forward pass, k-space operators, first inverse pass
+    auto operators = [&](auto time) {
+    const int im = time;
 #pragma unroll 1
     for (int b = threadIdx.x; b < NQ * TX; b += TH) {
         const int q = b / TX, kq = PL::krev(q);
@@ -200,11 +202,11 @@ __device__ __forceinline__ void pcol_regs(const PInst& P, const StepConst& c, in
 #pragma unroll
         for (int r = 0; r < RL; ++r) {
             const int iy = kq + r * NQ;
-            const cx<T> f = fmul(imag, kex, key[iy]);
+            const cx<T> f = fmul(im, kex, key[iy]);
             cx<T> u[MS];
 #pragma unroll
-            for (int m = 0; m < MS; ++m) u[m] = fmul(imag, f, cscale(v[m][r], fac[m]));
-            if (soc) soc_apply<T, MS>(imag, soc[(size_t)iy * st], u);
+            for (int m = 0; m < MS; ++m) u[m] = fmul(im, f, cscale(v[m][r], fac[m]));
+            if (soc) soc_apply<T, MS>(im, soc[(size_t)iy * st], u);
 #pragma unroll
             for (int m = 0; m < MS; ++m) v[m][r] = u[m];
         }
@@ -215,6 +217,9 @@ __device__ __forceinline__ void pcol_regs(const PInst& P, const StepConst& c, in
             for (int r = 0; r < RL; ++r) sm[m * LINE + TL::at(q * RL + r, t)] = v[m][r];
         }
     }
+    };
+    if (imag) operators(std::integral_constant<int, 1>{});
+    else operators(std::integral_constant<int, 0>{});
     __syncthreads();
 #pragma unroll 1
     for (int b = threadIdx.x; b < MS * NB * TX; b += TH) {

@@ -221,6 +221,8 @@ __device__ __forceinline__ void regcol_tiles(const Src& src) {
         }
         if constexpr (KOP) {
             // last forward pass, k-space operators, first inverse pass
+            auto operators = [&](auto time) {
+            const int im = time;
 #pragma unroll 1
             for (int b = threadIdx.x; b < TF; b += TH) {
                 const int t = b % TX, q = b / TX;
@@ -237,8 +239,8 @@ __device__ __forceinline__ void regcol_tiles(const Src& src) {
                     for (int r = 0; r < RL; ++r) {
                         cx<T> u[MS];
 #pragma unroll
-                        for (int m = 0; m < MS; ++m) u[m] = fmul(imag, fmul(imag, ke, kez[m * N + kq + r * NQ]), v[m][r]);
-                        if (soc) soc_apply<T, MS>(imag, so, u);
+                        for (int m = 0; m < MS; ++m) u[m] = fmul(im, fmul(im, ke, kez[m * N + kq + r * NQ]), v[m][r]);
+                        if (soc) soc_apply<T, MS>(im, so, u);
 #pragma unroll
                         for (int m = 0; m < MS; ++m) v[m][r] = u[m];
                     }
@@ -247,11 +249,11 @@ __device__ __forceinline__ void regcol_tiles(const Src& src) {
 #pragma unroll
                     for (int r = 0; r < RL; ++r) {
                         const int iy = kq + r * NQ;
-                        const cx<T> f = fmul(imag, ke, key[iy]);
+                        const cx<T> f = fmul(im, ke, key[iy]);
                         cx<T> u[MS];
 #pragma unroll
-                        for (int m = 0; m < MS; ++m) u[m] = fmul(imag, f, cscale(v[m][r], fac[m]));
-                        if (soc) soc_apply<T, MS>(imag, soc[(size_t)iy * nx + xt], u);
+                        for (int m = 0; m < MS; ++m) u[m] = fmul(im, f, cscale(v[m][r], fac[m]));
+                        if (soc) soc_apply<T, MS>(im, soc[(size_t)iy * nx + xt], u);
 #pragma unroll
                         for (int m = 0; m < MS; ++m) v[m][r] = u[m];
                     }
@@ -263,6 +265,14 @@ __device__ __forceinline__ void regcol_tiles(const Src& src) {
                     for (int r = 0; r < RL; ++r) sm[m * LINE + TL::at(q * RL + r, t)] = v[m][r];
                 }
             }
+            };
+            // one body per time direction (the factors of imaginary time are
+            // real), except where two spill: 256^3 FP64 spin-1 z pass in real
+            // time 447 us with one, 529 with two; elsewhere two are faster (FP32
+            // 260 -> 248, q2D 512^2 FP64 20.7 -> 18.9)
+            if constexpr (sizeof(T) == 8 && MS == 3 && KIND == COLK_Z3D) operators(imag);
+            else if (imag) operators(std::integral_constant<int, 1>{});
+            else operators(std::integral_constant<int, 0>{});
             __syncthreads();
         } else if constexpr (KIND == COLK_FWD) {
             // last forward pass, to global memory in position order
