@@ -29,7 +29,7 @@
 // What bounds it: the latency of an item (ticket, wait, loads, exchanges), not
 // a pipe or memory, so it runs three blocks of 256 threads per SM with three
 // components, with the column lines in registers (48 instances of 128^2 to
-// 512^2 spin 1, best variant: FP32 430 -> 351 us a step, FP64 609 -> 507 us).
+// 512^2 spin 1, best variant: FP32 430 -> 349 us a step, FP64 609 -> 499 us).
 //
 // Coherence.  Data that one block writes and another reads in the same
 // launch (tiles of S, the scales and SIG in info, NORMC partials) is read

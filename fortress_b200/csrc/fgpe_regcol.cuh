@@ -13,8 +13,8 @@
 //
 // Measured on one B200, 256^3 spin-1, against the shared-tile passes:
 //   y pass   FP64 0.33 -> 0.30 ms (5.3 TB/s, 0.81 of the measured copy
-//            rate), FP32 0.19 -> 0.14 ms (5.7 TB/s): bound by HBM;
-//   z pass   FP64 0.65 -> 0.42 ms, FP32 0.37 -> 0.26 ms: bound by latency at
+//            rate), FP32 0.19 -> 0.14 ms (5.8 TB/s): bound by HBM;
+//   z pass   FP64 0.65 -> 0.42 ms, FP32 0.37 -> 0.25 ms: bound by latency at
 //            8 or 12 warps per SM, the FP64 pipe about half busy.  A thread
 //            holds 48 complex values there; (8,4,8) and (32,8) lines with
 //            twice the warps took 10 to 40 % longer.

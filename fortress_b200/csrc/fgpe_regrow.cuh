@@ -15,7 +15,7 @@
 //
 // Bound by FP64 issue (256^3 spin-1: about 300 FP64 operations a point, that
 // pipe half busy) or, in FP32, by issue and latency.  One B200, 65536 rows of
-// 256 spin-1 points: FP64 0.72 (k_row_warp) -> 0.56 ms, of which the shorter
+// 256 spin-1 points: FP64 0.72 (k_row_warp) -> 0.55 ms, of which the shorter
 // SE and SP are 0.1; FP32 0.57 (k_row_fast) -> 0.32 ms.  Unrolling the point
 // loop (two or more points in flight, or all eight in registers) spilled and
 // was slower.
